@@ -154,7 +154,8 @@ extern "C" bbw_status bbw_set_c2q(bbw_ctx *c, const float *c2q) {
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess)
     e = cudaMemcpy(c->c2q, c2q, (size_t)c->K * c->Nq * sizeof(float), cudaMemcpyHostToDevice);
-  return set_cuda_error(e, "bbw_set_c2q");
+  if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_c2q");
+  return c->c2p ? warp_medium(c->K, c->Nq, c->c2q, c->c2max, c->c2p, c->stream) : BBW_OK;
 }
 
 extern "C" bbw_status bbw_tape_free(bbw_tape *t) {
@@ -233,7 +234,7 @@ extern "C" bbw_status bbw_forward_ex(bbw_ctx *c, float dt, int nsteps, int check
         return set_cuda_error(e, "bbw_forward: checkpoint");
       }
     }
-    if ((s = bbw_steps(c, dt, 1)) != BBW_OK) {
+    if ((s = run_steps(c, dt, 1, true)) != BBW_OK) {
       bbw_tape_free(t);
       return s;
     }
@@ -280,23 +281,12 @@ extern "C" bbw_status bbw_backward(bbw_ctx *c, bbw_tape *t, const float *dL_dtra
     e = cudaMemcpy(g, dL_dtraces, (size_t)S * R * nsteps * sizeof(float), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return set_cuda_error(e, "bbw_backward: upload");
 
-  FusedPlan pl = c->plan;
-  pl.time = tdev;
-  TcPlan tpl = c->tc;
-  tpl.time = tdev;
-  // one forward stage of the recomputation in the context's own form (FP32
-  // fused or tensor-core stage, bit-identical to the forward pass),
-  // optionally storing Vq S(Q)_p at the cubature points
+  // one forward stage of the recomputation, bit-identical to the forward pass
+  // (one stage form for both), optionally storing Vq S(Q)_p at the
+  // cubature points
   auto launch = [&](int i, const float *in, float *outq, float *vqo) {
-    const float cs = c->src_stage_times ? (float)kRK4C[i] : 0.f;
-    if (c->precision != BBW_PREC_FP32) {
-      TcPlan tp = tpl;
-      tp.vq_out = vqo;
-      return tc_launch(tp, in, outq, res, (float)kRK4A[i], (float)kRK4B[i], dt, cs, st);
-    }
-    FusedPlan p = pl;
-    p.vq_out = vqo;
-    return fused_launch(p, in, outq, res, (float)kRK4A[i], (float)kRK4B[i], dt, cs, st);
+    return launch_tape_stage(c, in, outq, res, (float)kRK4A[i], (float)kRK4B[i], dt,
+                             c->src_stage_times ? (float)kRK4C[i] : 0.f, st, vqo, tdev);
   };
   // step-start times exactly as the device clock accumulated them
   std::vector<double> tn(nsteps + 1);
@@ -383,7 +373,7 @@ extern "C" bbw_status bbw_backward(bbw_ctx *c, bbw_tape *t, const float *dL_dtra
       }
       for (int i = 4; i >= 0; --i) {
         const float ai = (float)kRK4A[i], bi = (float)kRK4B[i];
-        if ((s = adj_wadg(N, S, K, Nq, a.PqT, a.VqT, pl.c2q, lamQ, lamR, ai, bi, dt,
+        if ((s = adj_wadg(N, S, K, Nq, a.PqT, a.VqT, c->c2q, lamQ, lamR, ai, bi, dt,
                           vqs + (size_t)i * vqn, z, grad, st)) != BBW_OK ||
             (s = adj_volume(N, S, K, c->vgeo, a.DTp, z, rhs, st)) != BBW_OK ||
             (s = adj_sigma(N, S, K, c->fgeo, a.LTp, z, sigma, st)) != BBW_OK ||

@@ -54,7 +54,7 @@ void release(bbw_ctx *c) {
     delete c->gs;
     c->gs = nullptr;
   }
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < 4; ++i)
     if (c->step_graph[i]) cudaGraphExecDestroy(c->step_graph[i]);
   cudaFree(c->Q[0]);
   cudaFree(c->Q[1]);
@@ -76,6 +76,9 @@ void release(bbw_ctx *c) {
   cudaFree(c->traces);
   cudaFree(c->geo_tc);
   cudaFree(c->ops_tc);
+  cudaFree(c->ops_wp);
+  cudaFree(c->c2max);
+  cudaFree(c->c2p);
   cudaFree(c->err);
   adj_release(c);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -192,6 +195,17 @@ void dense_operators(int N, int Nq, const bbw_ops_desc *o, bool bb, bbw_ctx *c) 
       }
     }
   for (size_t i = 0; i < lift.size(); ++i) c->hLIFT[i] = (float)lift[i];
+}
+
+// one record per element: fgeo 16 | vgeo 9 | pad 3, and a tile's worth of
+// zero records after the last one
+std::vector<float> geometry_records(int K, const float *fgeo, const float *vgeo) {
+  std::vector<float> geo((size_t)(K + 16) * TC_GEO, 0.f);
+  for (int k = 0; k < K; ++k) {
+    std::memcpy(&geo[(size_t)k * TC_GEO], fgeo + (size_t)k * 16, 16 * sizeof(float));
+    std::memcpy(&geo[(size_t)k * TC_GEO + 16], vgeo + (size_t)k * 9, 9 * sizeof(float));
+  }
+  return geo;
 }
 
 // vmapP -> per face (neighbour << 8 | permutation id), permutation table
@@ -408,6 +422,34 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
       return s;
     }
   }
+  if (!gemm && precision != BBW_PREC_BF16X3 && warp_supported(N)) {
+    // FP32 contexts take four products per split pair, split FP16 three; BB
+    // contexts the dense equivalents of their sparse operators
+    WarpPlan &wp = c->wp;
+    wp.N = N, wp.K = K, wp.Nq = Nq, wp.bc = bc, wp.products = precision == BBW_PREC_FP32 ? 4 : 3;
+    wp.pat_off = pat_off, wp.table_ints = bb_off;  // Fmask and the face permutations
+    std::vector<uint32_t> wops;
+    const std::vector<float> geo = geometry_records(K, m->fgeo, m->vgeo);
+    warp_pack(wp, c->hD, c->hLIFT, c->hVq, c->hPq, wops);
+    if ((s = upload(&c->ops_wp, reinterpret_cast<const uint4 *>(wops.data()), wops.size() / 4,
+                    "bbw_create: split operators")) != BBW_OK ||
+        (s = upload(&c->geo_tc, geo.data(), geo.size(), "bbw_create: geometry")) != BBW_OK ||
+        (s = upload<float>(&c->c2max, nullptr, K, "bbw_create: medium bound")) != BBW_OK ||
+        (s = upload<float>(&c->c2p, nullptr, (size_t)K * ((Nq + 15) / 16 * 16),
+                           "bbw_create: medium")) != BBW_OK ||
+        (s = warp_medium(K, Nq, c->c2q, c->c2max, c->c2p, c->stream)) != BBW_OK) {
+      release(c);
+      return s;
+    }
+    wp.geo = c->geo_tc, wp.c2p = c->c2p, wp.c2max = c->c2max;
+    wp.nbr = c->nbr, wp.tables = c->tables, wp.ops = c->ops_wp, wp.time = c->d_time;
+    s = warp_prepare(wp);
+    if (s != BBW_OK && s != BBW_ERR_UNSUPPORTED) {
+      release(c);
+      return s;
+    }
+    wp.on = s == BBW_OK;
+  }
   if (tcp) {
     // geometry records, split-FP16 / split-BF16 operators in the canonical
     // K-major layout
@@ -418,11 +460,7 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
     tp.table_ints = bb_off, tp.pat_off = pat_off;
     tp.L = tc_layout(N, Nq, tp.table_ints);
     const TcLayout &TL = tp.L;
-    std::vector<float> geo((size_t)K * TC_GEO, 0.f);
-    for (int k = 0; k < K; ++k) {
-      std::memcpy(&geo[(size_t)k * TC_GEO], m->fgeo + (size_t)k * 16, 16 * sizeof(float));
-      std::memcpy(&geo[(size_t)k * TC_GEO + 16], m->vgeo + (size_t)k * 9, 9 * sizeof(float));
-    }
+    const std::vector<float> geo = geometry_records(K, m->fgeo, m->vgeo);
     // operator planes with MR (MRQ) stored rows, see tc_layout.  The dense
     // operators of the context's basis: for BB the dense equivalents of the
     // sparse derivative and of the L0 + degree-elevation lift
@@ -442,7 +480,8 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
     tc_pack_operator(c->hVq.data(), Nq, Np, 1, Nq, MRQ, TL.KV, &h[TL.oVq],
                      &h[TL.oVq + MRQ * TL.KV], tp.bf);
     uint16_t *dops = nullptr;
-    if ((s = upload(&c->geo_tc, geo.data(), geo.size(), "bbw_create: geometry")) != BBW_OK ||
+    if ((!c->geo_tc &&
+         (s = upload(&c->geo_tc, geo.data(), geo.size(), "bbw_create: geometry")) != BBW_OK) ||
         (s = upload(&dops, h.data(), h.size(), "bbw_create: tensor-core operators")) != BBW_OK ||
         (s = upload<int>(&c->err, nullptr, 1, "bbw_create: status")) != BBW_OK) {
       c->ops_tc = dops;
@@ -514,10 +553,42 @@ extern "C" bbw_status bbw_get_residual(bbw_ctx *c, float *r) {
 }
 
 static void drop_graphs(bbw_ctx *c) {
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < 4; ++i) {
     if (c->step_graph[i]) cudaGraphExecDestroy(c->step_graph[i]);
     c->step_graph[i] = nullptr;
   }
+}
+
+bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
+                        float fdt, float cstage, cudaStream_t st, int K0, int Kc) {
+  if (c->wp.on && (c->wp.pinned || warp_preferred(c->N, (long long)c->S * c->K))) {
+    WarpPlan p = c->wp;
+    p.S = c->S, p.K0 = K0, p.Kc = Kc > 0 ? Kc : c->plan.Kc, p.max_ctas = c->plan.max_ctas;
+    p.src_tile = c->src_tile, p.src_elem = c->src_elem, p.src_vec = c->src_vec;
+    p.f0 = c->plan.f0, p.tR = c->plan.tR, p.samp = c->plan.samp;
+    return warp_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
+  }
+  if (c->precision != BBW_PREC_FP32)
+    return tc_launch(c->tc, Qin, Qout, res, fa, fb, fdt, cstage, st);
+  FusedPlan p = c->plan;
+  p.K0 = K0;
+  if (Kc > 0) p.Kc = Kc;
+  return fused_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
+}
+
+bbw_status launch_tape_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa,
+                             float fb, float fdt, float cstage, cudaStream_t st, float *vq_out,
+                             const double *time) {
+  if (c->precision != BBW_PREC_FP32) {
+    TcPlan p = c->tc;
+    p.vq_out = vq_out;
+    if (time) p.time = time;
+    return tc_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
+  }
+  FusedPlan p = c->plan;
+  p.vq_out = vq_out;
+  if (time) p.time = time;
+  return fused_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
 }
 
 extern "C" bbw_status bbw_stage_ex(bbw_ctx *c, float fa, float fb, float fdt, float cstage) {
@@ -529,11 +600,7 @@ extern "C" bbw_status bbw_stage_ex(bbw_ctx *c, float fa, float fb, float fdt, fl
     s = gemm_stage_launch(*c->gs, in, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt,
                           c->stream);
   } else {
-    s = c->precision != BBW_PREC_FP32
-            ? tc_launch(c->tc, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, cstage,
-                        c->stream)
-            : fused_launch(c->plan, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, cstage,
-                           c->stream);
+    s = launch_stage(c, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, cstage, c->stream);
   }
   if (s == BBW_OK) c->cur ^= 1;
   return s;
@@ -544,62 +611,65 @@ extern "C" bbw_status bbw_stage(bbw_ctx *c, float fa, float fb, float fdt) {
   return bbw_stage_ex(c, fa, fb, fdt, 0.f);
 }
 
-// one LSRK45 step: five fused stages at times t + rk4c[s] dt, then the
-// receivers and the clock
-static bbw_status one_step(bbw_ctx *c, float dt) {
-  bbw_status s = BBW_OK;
-  for (int i = 0; i < 5 && s == BBW_OK; ++i)
-    s = bbw_stage_ex(c, (float)kRK4A[i], (float)kRK4B[i], dt,
-                     c->src_stage_times ? (float)kRK4C[i] : 0.f);
-  if (s != BBW_OK) return s;
+// one LSRK45 step: five stages at times t + rk4c[s] dt, then the receivers
+// and the clock; vq: also store each stage's pre-c^2 cubature values at vq + i *
+// vqn (tape passes)
+static bbw_status one_step(bbw_ctx *c, float dt, bool tape, float *vq, size_t vqn) {
+  for (int i = 0; i < 5; ++i) {
+    const float fa = (float)kRK4A[i], fb = (float)kRK4B[i];
+    const float cs = c->src_stage_times ? (float)kRK4C[i] : 0.f;
+    bbw_status s = BBW_OK;
+    if (tape) {
+      s = launch_tape_stage(c, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, dt, cs, c->stream,
+                            vq ? vq + (size_t)i * vqn : nullptr);
+      if (s == BBW_OK) c->cur ^= 1;
+    } else {
+      s = bbw_stage_ex(c, fa, fb, dt, cs);
+    }
+    if (s != BBW_OK) return s;
+  }
   return record_and_advance(c->N, c->K, c->S, c->Q[c->cur], c->R, c->rec_elem, c->rec_w,
                             c->traces, c->max_steps, c->d_time, c->d_step, dt, c->stream);
 }
 
-// one LSRK45 step launched stage by stage (no graph), as one_step, storing
-// each stage's pre-c^2 cubature values at vq + i * vqn (the adjoint tape)
+// one LSRK45 step of the adjoint's forward pass launched stage by stage (no
+// graph), storing the cubature values
 bbw_status step_storing_cubature(bbw_ctx *c, float dt, float *vq, size_t vqn) {
-  float *keep_f = c->plan.vq_out, *keep_t = c->tc.vq_out;
-  bbw_status s = BBW_OK;
-  for (int i = 0; i < 5 && s == BBW_OK; ++i) {
-    c->plan.vq_out = c->tc.vq_out = vq + (size_t)i * vqn;
-    s = bbw_stage_ex(c, (float)kRK4A[i], (float)kRK4B[i], dt,
-                     c->src_stage_times ? (float)kRK4C[i] : 0.f);
+  return one_step(c, dt, true, vq, vqn);
+}
+
+bbw_status run_steps(bbw_ctx *c, float dt, int nsteps, bool tape) {
+  uint32_t bits;
+  std::memcpy(&bits, &dt, 4);
+  for (int step = 0; step < nsteps; ++step) {
+    const int par = c->cur, slot = par + (tape ? 2 : 0);
+    if (!c->step_graph[slot] || c->graph_dt_bits[slot] != bits) {
+      if (c->step_graph[slot]) cudaGraphExecDestroy(c->step_graph[slot]);
+      c->step_graph[slot] = nullptr;
+      cudaGraph_t g;
+      cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+      if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: capture");
+      bbw_status s = one_step(c, dt, tape, nullptr, 0);
+      e = cudaStreamEndCapture(c->stream, &g);
+      c->cur = par;  // capture recorded the launches without running them
+      if (s != BBW_OK) return s;
+      if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: end capture");
+      e = cudaGraphInstantiate(&c->step_graph[slot], g, 0);
+      cudaGraphDestroy(g);
+      if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: instantiate");
+      c->graph_dt_bits[slot] = bits;
+    }
+    cudaError_t e = cudaGraphLaunch(c->step_graph[slot], c->stream);
+    if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: launch");
+    c->cur ^= 1;  // five stages swap the buffers an odd number of times
   }
-  c->plan.vq_out = keep_f, c->tc.vq_out = keep_t;
-  if (s != BBW_OK) return s;
-  return record_and_advance(c->N, c->K, c->S, c->Q[c->cur], c->R, c->rec_elem, c->rec_w,
-                            c->traces, c->max_steps, c->d_time, c->d_step, dt, c->stream);
+  return BBW_OK;
 }
 
 extern "C" bbw_status bbw_steps(bbw_ctx *c, float dt, int nsteps) {
   DeviceGuard dg(c ? c->device : -1);
   if (!c || nsteps < 0) return set_error(BBW_ERR_ARG, "bbw_steps: bad argument");
-  uint32_t bits;
-  std::memcpy(&bits, &dt, 4);
-  for (int step = 0; step < nsteps; ++step) {
-    const int par = c->cur;
-    if (!c->step_graph[par] || c->graph_dt_bits[par] != bits) {
-      if (c->step_graph[par]) cudaGraphExecDestroy(c->step_graph[par]);
-      c->step_graph[par] = nullptr;
-      cudaGraph_t g;
-      cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
-      if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: capture");
-      bbw_status s = one_step(c, dt);
-      e = cudaStreamEndCapture(c->stream, &g);
-      c->cur = par;  // capture recorded the launches without running them
-      if (s != BBW_OK) return s;
-      if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: end capture");
-      e = cudaGraphInstantiate(&c->step_graph[par], g, 0);
-      cudaGraphDestroy(g);
-      if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: instantiate");
-      c->graph_dt_bits[par] = bits;
-    }
-    cudaError_t e = cudaGraphLaunch(c->step_graph[par], c->stream);
-    if (e != cudaSuccess) return set_cuda_error(e, "bbw_steps: launch");
-    c->cur ^= 1;  // five stages swap the buffers an odd number of times
-  }
-  return BBW_OK;
+  return run_steps(c, dt, nsteps, false);
 }
 
 // plan of the fused stage with W warps, E-element tiles and the requested
@@ -629,11 +699,20 @@ extern "C" bbw_status bbw_set_config(bbw_ctx *c, int config) {
   DeviceGuard dg(c ? c->device : -1);
   if (!c) return set_error(BBW_ERR_ARG, "bbw_set_config: ctx is NULL");
   const int W = config & 255;
-  if ((W != 8 && W != 16) || (config >> 11) != 0)
+  if ((W != 8 && W != 16) || ((config >> 11) != 0 && config != kWarpConfig))
     return set_error(BBW_ERR_ARG, "bbw_set_config: W must be 8 or 16, flags bits 8-10");
   if (c->precision != BBW_PREC_FP32) return BBW_OK;
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_config");
+  if (config == kWarpConfig) {
+    if (!c->ops_wp)
+      return set_error(BBW_ERR_UNSUPPORTED, "bbw_set_config: no warp-matrix stage at this size");
+    const bbw_status s = warp_prepare(c->wp);
+    if (s != BBW_OK) return s;
+    c->wp.on = c->wp.pinned = true;
+    drop_graphs(c);
+    return BBW_OK;
+  }
   FusedPlan p;
   float *buf = nullptr;
   bbw_status s = make_variant(c, W, (config >> 10 & 1) ? 16 : 32, config >> 8 & 1, config >> 9 & 1, p,
@@ -645,6 +724,7 @@ extern "C" bbw_status bbw_set_config(bbw_ctx *c, int config) {
   cudaFree(c->ops);
   c->ops = buf;
   c->plan = p;
+  c->wp.on = false;
   drop_graphs(c);
   return BBW_OK;
 }
@@ -679,38 +759,50 @@ extern "C" bbw_status bbw_autotune(bbw_ctx *c, float dt, int stages, int *config
   const int Ws[2] = {8, 16}, Es[2] = {32, 16};
   float best_ms = 0.f;
   int best = -1;
-  for (int ei = 0; ei < 2; ++ei)
-  for (int wi = 0; wi < 2; ++wi)
-    for (int v = 0; v < 4; ++v) {
+  // times one form over `stages` launches; launch(in, out, a, b) is one stage
+  auto time_form = [&](int code, auto &&launch) {
+    int cur = 0;
+    for (int i = 0; i < 2; ++i, cur ^= 1)  // warm-up
+      launch(q[cur], q[cur ^ 1], 0.f, (float)kRK4B[0]);
+    cudaEventRecord(e0, c->stream);
+    for (int i = 0; i < stages; ++i, cur ^= 1)
+      launch(q[cur], q[cur ^ 1], (float)kRK4A[i % 5], (float)kRK4B[i % 5]);
+    cudaEventRecord(e1, c->stream);
+    e = cudaEventSynchronize(e1);
+    float ms = 0.f;
+    if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+    if (e == cudaSuccess && (best < 0 || ms < best_ms)) best = code, best_ms = ms;
+  };
+  if (c->ops_wp && warp_prepare(c->wp) == BBW_OK) {
+    WarpPlan p = c->wp;
+    p.S = c->S, p.Kc = c->plan.Kc, p.max_ctas = c->plan.max_ctas;
+    time_form(kWarpConfig, [&](const float *in, float *out, float fa, float fb) {
+      warp_launch(p, in, out, r, fa, fb, dt, 0.f, c->stream);
+    });
+  }
+  for (int ei = 0; ei < 2 && e == cudaSuccess; ++ei)
+  for (int wi = 0; wi < 2 && e == cudaSuccess; ++wi)
+    for (int v = 0; v < 4 && e == cudaSuccess; ++v) {
       FusedPlan p;
       float *buf = nullptr;
       if (make_variant(c, Ws[wi], Es[ei], v < 2 ? 1 : 0, v % 2 == 0 ? 1 : 0, p, &buf) != BBW_OK) {
         cudaFree(buf);  // does not fit
         continue;
       }
-      int cur = 0;
-      for (int i = 0; i < 2; ++i, cur ^= 1)  // warm-up
-        fused_launch(p, q[cur], q[cur ^ 1], r, 0.f, (float)kRK4B[0], dt, 0.f, c->stream);
-      cudaEventRecord(e0, c->stream);
-      for (int i = 0; i < stages; ++i, cur ^= 1)
-        fused_launch(p, q[cur], q[cur ^ 1], r, (float)kRK4A[i % 5], (float)kRK4B[i % 5], dt, 0.f,
-                     c->stream);
-      cudaEventRecord(e1, c->stream);
-      e = cudaEventSynchronize(e1);
+      time_form(config_code(p), [&](const float *in, float *out, float fa, float fb) {
+        fused_launch(p, in, out, r, fa, fb, dt, 0.f, c->stream);
+      });
       cudaFree(buf);
-      if (e != cudaSuccess) {
-        cleanup();
-        return set_cuda_error(e, "bbw_autotune: timing");
-      }
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (best < 0 || ms < best_ms) best = config_code(p), best_ms = ms;
     }
+  if (e != cudaSuccess) {
+    cleanup();
+    return set_cuda_error(e, "bbw_autotune: timing");
+  }
   cleanup();
   if (best < 0) return set_error(BBW_ERR_UNSUPPORTED, "bbw_autotune: no variant fits");
   bbw_status s2 = bbw_set_config(c, best);
   if (s2 != BBW_OK) return s2;
-  if (config) *config = config_code(c->plan);
+  if (config) *config = c->wp.on ? kWarpConfig : config_code(c->plan);
   return BBW_OK;
 }
 
@@ -756,9 +848,8 @@ extern "C" bbw_status bbw_stage_part(bbw_ctx *c, float fa, float fb, float fdt, 
     return set_error(BBW_ERR_ARG, "bbw_stage_part: need 0 <= K0 < K1 <= K");
   if (c->precision != BBW_PREC_FP32)
     return set_error(BBW_ERR_UNSUPPORTED, "bbw_stage_part: FP32 stage only");
-  FusedPlan p = c->plan;
-  p.K0 = K0, p.Kc = K1;
-  return fused_launch(p, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, 0.f, c->stream);
+  return launch_stage(c, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, 0.f, c->stream,
+                      K0, K1);
 }
 
 extern "C" bbw_status bbw_stage_commit(bbw_ctx *c) {

@@ -10,6 +10,7 @@
 #include "device_common.cuh"
 #include "fused.h"
 #include "gemm_stage.h"
+#include "warp_stage.h"
 
 namespace bbw {
 
@@ -27,6 +28,10 @@ struct AdjOps {
   // [Nq][ld(Np)], D^T [3][Np][ld(Np)], LIFT^T per face [4][Np][ld(Nfp)]
   float *PqT = nullptr, *VqT = nullptr, *DTp = nullptr, *LTp = nullptr;
 };
+
+// configuration code of the warp-matrix stage: 16 elements per warp, operators
+// in shared memory where they fit, and bit 11
+constexpr int kWarpConfig = 8 | 1 << 8 | 1 << 10 | 1 << 11;
 
 // LSRK45 coefficients (Carpenter-Kennedy), cpp/src/StartUp3d.cpp:517-537
 extern const double kRK4A[5], kRK4B[5], kRK4C[5];
@@ -78,13 +83,18 @@ struct bbw_ctx {
   int *rec_elem = nullptr;
   float *rec_w = nullptr, *traces = nullptr;
   bbw::TcPlan tc;
+  bbw::WarpPlan wp;         // warp-matrix stage (wp.on: the context's stage runs on it)
+  uint4 *ops_wp = nullptr;
+  float *c2max = nullptr;   // [K] largest |c2q| of each element
+  float *c2p = nullptr;     // [K][Nq rounded up to 16] c2q padded with zeros
   bbw::GemmStage *gs = nullptr;  // precision-study GEMM form (null: fused or tensor-core stage)
   float *geo_tc = nullptr;
   void *ops_tc = nullptr;
   int *err = nullptr;
-  // one graph per starting buffer parity, for one LSRK45 step of size dt
-  cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
-  uint32_t graph_dt_bits[2] = {0, 0};
+  // one graph per starting buffer parity, for one LSRK45 step of size dt; the
+  // second pair for the adjoint's forward pass
+  cudaGraphExec_t step_graph[4] = {nullptr, nullptr, nullptr, nullptr};
+  uint32_t graph_dt_bits[4] = {0, 0, 0, 0};
   // host copies for the adjoint: dense operators of the chosen basis
   // (column-major Np x Np / Np x 4Nfp / Nq x Np / Np x Nq), Fmask, vmapP
   std::vector<float> hD[3], hLIFT, hVq, hPq;
@@ -92,6 +102,21 @@ struct bbw_ctx {
   bbw::AdjOps adj;
 };
 
+// one stage of the context in the form of its time loop (warp-matrix,
+// tensor-core or FP32 fused): elements [K0, Kc) (Kc = 0: the context's compute
+// range) of all shots
+bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
+                        float fdt, float cstage, cudaStream_t st, int K0 = 0, int Kc = 0);
+// one stage of the adjoint's forward pass and recomputation: the FP32 fused or
+// tensor-core stage, whose rounding the FP64 gradient is pinned to.  vq_out:
+// store the pre-c^2 cubature values ([S][Nq][K]); time: the clock the sources
+// read (null: the context's).
+bbw_status launch_tape_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa,
+                             float fb, float fdt, float cstage, cudaStream_t st,
+                             float *vq_out = nullptr, const double *time = nullptr);
+// nsteps LSRK45 steps on launch_stage (tape: on launch_tape_stage), one graph
+// launch each
+bbw_status run_steps(bbw_ctx *c, float dt, int nsteps, bool tape);
 
 // one LSRK45 step launched stage by stage that also stores each stage's
 // pre-c^2 cubature values at vq + i * vqn (capi.cu)

@@ -1,0 +1,4 @@
+#include "warp_stage.cuh"
+namespace bbw {
+BBW_WARP_STAGE_INSTANCE(4)
+}
