@@ -197,17 +197,6 @@ void dense_operators(int N, int Nq, const bbw_ops_desc *o, bool bb, bbw_ctx *c) 
   for (size_t i = 0; i < lift.size(); ++i) c->hLIFT[i] = (float)lift[i];
 }
 
-// one record per element: fgeo 16 | vgeo 9 | pad 3, and a tile's worth of
-// zero records after the last one
-std::vector<float> geometry_records(int K, const float *fgeo, const float *vgeo) {
-  std::vector<float> geo((size_t)(K + 16) * TC_GEO, 0.f);
-  for (int k = 0; k < K; ++k) {
-    std::memcpy(&geo[(size_t)k * TC_GEO], fgeo + (size_t)k * 16, 16 * sizeof(float));
-    std::memcpy(&geo[(size_t)k * TC_GEO + 16], vgeo + (size_t)k * 9, 9 * sizeof(float));
-  }
-  return geo;
-}
-
 // vmapP -> per face (neighbour << 8 | permutation id), permutation table
 bbw_status compress_connectivity(int N, int K, const int *Fmask, const int *vmapP,
                                  std::vector<int> &nbr, std::vector<int> &pats, int &npat) {
@@ -422,33 +411,36 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
       return s;
     }
   }
-  if (!gemm && precision != BBW_PREC_BF16X3 && warp_supported(N)) {
+  if (!gemm && (tcp || N <= 7) &&
+      ((s = upload<float>(&c->geo_tc, nullptr, (size_t)(K + 16) * TC_GEO, "bbw_create: geometry")) !=
+           BBW_OK ||
+       (s = geometry_records(K, c->vgeo, c->fgeo, c->geo_tc)) != BBW_OK)) {
+    release(c);
+    return s;
+  }
+  if (!gemm && precision != BBW_PREC_BF16X3 && N <= 7) {
     // FP32 contexts take four products per split pair, split FP16 three; BB
     // contexts the dense equivalents of their sparse operators
     WarpPlan &wp = c->wp;
     wp.N = N, wp.K = K, wp.Nq = Nq, wp.bc = bc, wp.products = precision == BBW_PREC_FP32 ? 4 : 3;
     wp.pat_off = pat_off, wp.table_ints = bb_off;  // Fmask and the face permutations
     std::vector<uint32_t> wops;
-    const std::vector<float> geo = geometry_records(K, m->fgeo, m->vgeo);
     warp_pack(wp, c->hD, c->hLIFT, c->hVq, c->hPq, wops);
     if ((s = upload(&c->ops_wp, reinterpret_cast<const uint4 *>(wops.data()), wops.size() / 4,
                     "bbw_create: split operators")) != BBW_OK ||
-        (s = upload(&c->geo_tc, geo.data(), geo.size(), "bbw_create: geometry")) != BBW_OK ||
         (s = upload<float>(&c->c2max, nullptr, K, "bbw_create: medium bound")) != BBW_OK ||
         (s = upload<float>(&c->c2p, nullptr, (size_t)K * ((Nq + 15) / 16 * 16),
                            "bbw_create: medium")) != BBW_OK ||
-        (s = warp_medium(K, Nq, c->c2q, c->c2max, c->c2p, c->stream)) != BBW_OK) {
+        (s = warp_medium(K, Nq, c->c2q, c->c2max, c->c2p)) != BBW_OK) {
       release(c);
       return s;
     }
     wp.geo = c->geo_tc, wp.c2p = c->c2p, wp.c2max = c->c2max;
     wp.nbr = c->nbr, wp.tables = c->tables, wp.ops = c->ops_wp, wp.time = c->d_time;
-    s = warp_prepare(wp);
-    if (s != BBW_OK && s != BBW_ERR_UNSUPPORTED) {
+    if ((s = warp_prepare(wp)) != BBW_OK) {
       release(c);
       return s;
     }
-    wp.on = s == BBW_OK;
   }
   if (tcp) {
     // geometry records, split-FP16 / split-BF16 operators in the canonical
@@ -460,7 +452,6 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
     tp.table_ints = bb_off, tp.pat_off = pat_off;
     tp.L = tc_layout(N, Nq, tp.table_ints);
     const TcLayout &TL = tp.L;
-    const std::vector<float> geo = geometry_records(K, m->fgeo, m->vgeo);
     // operator planes with MR (MRQ) stored rows, see tc_layout.  The dense
     // operators of the context's basis: for BB the dense equivalents of the
     // sparse derivative and of the L0 + degree-elevation lift
@@ -480,9 +471,7 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
     tc_pack_operator(c->hVq.data(), Nq, Np, 1, Nq, MRQ, TL.KV, &h[TL.oVq],
                      &h[TL.oVq + MRQ * TL.KV], tp.bf);
     uint16_t *dops = nullptr;
-    if ((!c->geo_tc &&
-         (s = upload(&c->geo_tc, geo.data(), geo.size(), "bbw_create: geometry")) != BBW_OK) ||
-        (s = upload(&dops, h.data(), h.size(), "bbw_create: tensor-core operators")) != BBW_OK ||
+    if ((s = upload(&dops, h.data(), h.size(), "bbw_create: tensor-core operators")) != BBW_OK ||
         (s = upload<int>(&c->err, nullptr, 1, "bbw_create: status")) != BBW_OK) {
       c->ops_tc = dops;
       release(c);
@@ -561,12 +550,13 @@ static void drop_graphs(bbw_ctx *c) {
 
 bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
                         float fdt, float cstage, cudaStream_t st, int K0, int Kc) {
-  if (c->wp.on && (c->wp.pinned || warp_preferred(c->N, (long long)c->S * c->K))) {
+  const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, (long long)c->S * c->K);
+  if (form != WARP_AUTO) {
     WarpPlan p = c->wp;
     p.S = c->S, p.K0 = K0, p.Kc = Kc > 0 ? Kc : c->plan.Kc, p.max_ctas = c->plan.max_ctas;
     p.src_tile = c->src_tile, p.src_elem = c->src_elem, p.src_vec = c->src_vec;
     p.f0 = c->plan.f0, p.tR = c->plan.tR, p.samp = c->plan.samp;
-    return warp_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
+    return warp_launch(p, form, Qin, Qout, res, fa, fb, fdt, cstage, st);
   }
   if (c->precision != BBW_PREC_FP32)
     return tc_launch(c->tc, Qin, Qout, res, fa, fb, fdt, cstage, st);
@@ -699,17 +689,16 @@ extern "C" bbw_status bbw_set_config(bbw_ctx *c, int config) {
   DeviceGuard dg(c ? c->device : -1);
   if (!c) return set_error(BBW_ERR_ARG, "bbw_set_config: ctx is NULL");
   const int W = config & 255;
-  if ((W != 8 && W != 16) || ((config >> 11) != 0 && config != kWarpConfig))
+  if ((W != 8 && W != 16) || ((config >> 11) != 0 && config != kWarpConfig && config != kGroupConfig))
     return set_error(BBW_ERR_ARG, "bbw_set_config: W must be 8 or 16, flags bits 8-10");
   if (c->precision != BBW_PREC_FP32) return BBW_OK;
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_config");
-  if (config == kWarpConfig) {
-    if (!c->ops_wp)
-      return set_error(BBW_ERR_UNSUPPORTED, "bbw_set_config: no warp-matrix stage at this size");
-    const bbw_status s = warp_prepare(c->wp);
-    if (s != BBW_OK) return s;
-    c->wp.on = c->wp.pinned = true;
+  if (config == kWarpConfig || config == kGroupConfig) {
+    const bool group = config == kGroupConfig;
+    if (!(group ? c->wp.group : c->wp.single))
+      return set_error(BBW_ERR_UNSUPPORTED, "bbw_set_config: no such form at this size");
+    c->wp.pinned = group ? WARP_GROUP : WARP_SINGLE, c->cta_form = false;
     drop_graphs(c);
     return BBW_OK;
   }
@@ -724,7 +713,7 @@ extern "C" bbw_status bbw_set_config(bbw_ctx *c, int config) {
   cudaFree(c->ops);
   c->ops = buf;
   c->plan = p;
-  c->wp.on = false;
+  c->cta_form = true;
   drop_graphs(c);
   return BBW_OK;
 }
@@ -773,12 +762,14 @@ extern "C" bbw_status bbw_autotune(bbw_ctx *c, float dt, int stages, int *config
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     if (e == cudaSuccess && (best < 0 || ms < best_ms)) best = code, best_ms = ms;
   };
-  if (c->ops_wp && warp_prepare(c->wp) == BBW_OK) {
+  for (int form = WARP_SINGLE; form <= WARP_GROUP; ++form) {
+    if (!(form == WARP_GROUP ? c->wp.group : c->wp.single)) continue;
     WarpPlan p = c->wp;
     p.S = c->S, p.Kc = c->plan.Kc, p.max_ctas = c->plan.max_ctas;
-    time_form(kWarpConfig, [&](const float *in, float *out, float fa, float fb) {
-      warp_launch(p, in, out, r, fa, fb, dt, 0.f, c->stream);
-    });
+    time_form(form == WARP_GROUP ? kGroupConfig : kWarpConfig,
+              [&](const float *in, float *out, float fa, float fb) {
+                warp_launch(p, form, in, out, r, fa, fb, dt, 0.f, c->stream);
+              });
   }
   for (int ei = 0; ei < 2 && e == cudaSuccess; ++ei)
   for (int wi = 0; wi < 2 && e == cudaSuccess; ++wi)
@@ -802,7 +793,7 @@ extern "C" bbw_status bbw_autotune(bbw_ctx *c, float dt, int stages, int *config
   if (best < 0) return set_error(BBW_ERR_UNSUPPORTED, "bbw_autotune: no variant fits");
   bbw_status s2 = bbw_set_config(c, best);
   if (s2 != BBW_OK) return s2;
-  if (config) *config = c->wp.on ? kWarpConfig : config_code(c->plan);
+  if (config) *config = best;
   return BBW_OK;
 }
 

@@ -373,7 +373,7 @@ extern "C" bbw_status bbw_curved_autotune(bbw_curved *h, float dt, int stages, i
   float best_ms = 0.f;
   int best = -1;
   bbw_status s = BBW_OK;
-  std::vector<int> codes = {kWarpConfig};
+  std::vector<int> codes = {kWarpConfig, kGroupConfig};
   for (int e16 = 0; e16 < 2; ++e16)
     for (int W = 8; W <= 16; W += 8)
       for (int v = 0; v < 4; ++v)

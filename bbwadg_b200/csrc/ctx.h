@@ -29,9 +29,10 @@ struct AdjOps {
   float *PqT = nullptr, *VqT = nullptr, *DTp = nullptr, *LTp = nullptr;
 };
 
-// configuration code of the warp-matrix stage: 16 elements per warp, operators
-// in shared memory where they fit, and bit 11
+// configuration codes of the warp-matrix stages: 16-element tiles, operators in
+// shared memory where they fit, and bit 11 (one warp per tile) or 12 (a group)
 constexpr int kWarpConfig = 8 | 1 << 8 | 1 << 10 | 1 << 11;
+constexpr int kGroupConfig = 8 | 1 << 8 | 1 << 10 | 1 << 12;
 
 // LSRK45 coefficients (Carpenter-Kennedy), cpp/src/StartUp3d.cpp:517-537
 extern const double kRK4A[5], kRK4B[5], kRK4C[5];
@@ -83,7 +84,8 @@ struct bbw_ctx {
   int *rec_elem = nullptr;
   float *rec_w = nullptr, *traces = nullptr;
   bbw::TcPlan tc;
-  bbw::WarpPlan wp;         // warp-matrix stage (wp.on: the context's stage runs on it)
+  bbw::WarpPlan wp;         // warp-matrix stages
+  bool cta_form = false;    // the caller or the autotuner chose a CTA-wide variant
   uint4 *ops_wp = nullptr;
   float *c2max = nullptr;   // [K] largest |c2q| of each element
   float *c2p = nullptr;     // [K][Nq rounded up to 16] c2q padded with zeros

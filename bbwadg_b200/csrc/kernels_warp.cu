@@ -12,36 +12,30 @@
 
 namespace bbw {
 
-#define BBW_WARP_DECL(n)                                                                     \
-  bbw_status warp_launch_##n(const WarpPlan &, const float *, float *, float *, float, float, \
-                             float, float, cudaStream_t);                                    \
-  bbw_status warp_prepare_##n(WarpPlan &);
-BBW_WARP_DECL(1) BBW_WARP_DECL(2) BBW_WARP_DECL(3) BBW_WARP_DECL(4)
-BBW_WARP_DECL(5) BBW_WARP_DECL(6) BBW_WARP_DECL(7) BBW_WARP_DECL(8)
-#undef BBW_WARP_DECL
+#define BBW_DECL(form, n)                                                                       \
+  bbw_status form##_launch_##n(const WarpPlan &, const float *, float *, float *, float, float, \
+                               float, float, cudaStream_t);                                     \
+  bbw_status form##_prepare_##n(WarpPlan &);
+BBW_DECL(warp, 1) BBW_DECL(warp, 2) BBW_DECL(warp, 3) BBW_DECL(warp, 4)
+BBW_DECL(group, 4) BBW_DECL(group, 5) BBW_DECL(group, 6) BBW_DECL(group, 7)
+#undef BBW_DECL
 
-bool warp_supported(int N) { return N >= 1 && N <= 8; }
-
-#define BBW_WARP_SWITCH(CALL)   \
-  switch (N) {                  \
-    case 1: CALL(1); break;     \
-    case 2: CALL(2); break;     \
-    case 3: CALL(3); break;     \
-    case 4: CALL(4); break;     \
-    case 5: CALL(5); break;     \
-    case 6: CALL(6); break;     \
-    case 7: CALL(7); break;     \
-    case 8: CALL(8); break;     \
-    default: return set_error(BBW_ERR_UNSUPPORTED, "warp-matrix stage: N out of range"); \
+bbw_status warp_launch(const WarpPlan &pl, int form, const float *Qin, float *Qout, float *res,
+                       float fa, float fb, float fdt, float cstage, cudaStream_t st) {
+  switch (pl.N + 16 * form) {
+#define CASE(f, form, n) \
+  case n + 16 * f: return form##_launch_##n(pl, Qin, Qout, res, fa, fb, fdt, cstage, st);
+    CASE(WARP_SINGLE, warp, 1)
+    CASE(WARP_SINGLE, warp, 2)
+    CASE(WARP_SINGLE, warp, 3)
+    CASE(WARP_SINGLE, warp, 4)
+    CASE(WARP_GROUP, group, 4)
+    CASE(WARP_GROUP, group, 5)
+    CASE(WARP_GROUP, group, 6)
+    CASE(WARP_GROUP, group, 7)
+#undef CASE
   }
-
-bbw_status warp_launch(const WarpPlan &pl, const float *Qin, float *Qout, float *res, float fa,
-                       float fb, float fdt, float cstage, cudaStream_t st) {
-  const int N = pl.N;
-#define CALL(n) return warp_launch_##n(pl, Qin, Qout, res, fa, fb, fdt, cstage, st)
-  BBW_WARP_SWITCH(CALL)
-#undef CALL
-  return BBW_OK;
+  return set_error(BBW_ERR_UNSUPPORTED, "warp-matrix stage: N out of range");
 }
 
 bbw_status warp_prepare(WarpPlan &pl) {
@@ -49,10 +43,19 @@ bbw_status warp_prepare(WarpPlan &pl) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   pl.nsm = nsm > 0 ? nsm : 148;
-  const int N = pl.N;
-#define CALL(n) return warp_prepare_##n(pl)
-  BBW_WARP_SWITCH(CALL)
-#undef CALL
+  bbw_status a = BBW_ERR_UNSUPPORTED, b = BBW_ERR_UNSUPPORTED;
+  switch (pl.N) {
+    case 1: a = warp_prepare_1(pl); break;
+    case 2: a = warp_prepare_2(pl); break;
+    case 3: a = warp_prepare_3(pl); break;
+    case 4: a = warp_prepare_4(pl), b = group_prepare_4(pl); break;
+    case 5: b = group_prepare_5(pl); break;
+    case 6: b = group_prepare_6(pl); break;
+    case 7: b = group_prepare_7(pl); break;
+  }
+  if (a != BBW_OK && a != BBW_ERR_UNSUPPORTED) return a;
+  if (b != BBW_OK && b != BBW_ERR_UNSUPPORTED) return b;
+  pl.single = a == BBW_OK, pl.group = b == BBW_OK;
   return BBW_OK;
 }
 
@@ -66,16 +69,12 @@ static float operator_scale(const float *a, size_t n) {
   return std::ldexp(1.f, std::min(std::max(14 - e, -100), 100));
 }
 
-static uint32_t pack_pair(float a, float b, bool lo) {
+// FP16 pair of two values: hi words, or what they leave (lo)
+static void pack_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
   const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
-  uint16_t x, y;
-  if (!lo) {
-    x = __half_as_ushort(ha), y = __half_as_ushort(hb);
-  } else {
-    x = __half_as_ushort(__float2half_rn(a - __half2float(ha)));
-    y = __half_as_ushort(__float2half_rn(b - __half2float(hb)));
-  }
-  return (uint32_t)x | (uint32_t)y << 16;
+  const __half la = __float2half_rn(a - __half2float(ha)), lb = __float2half_rn(b - __half2float(hb));
+  hi = (uint32_t)__half_as_ushort(ha) | (uint32_t)__half_as_ushort(hb) << 16;
+  lo = (uint32_t)__half_as_ushort(la) | (uint32_t)__half_as_ushort(lb) << 16;
 }
 
 // index of slot c of block b when n indices are stored in blocks of eight
@@ -86,19 +85,28 @@ static int warp_node(int n, int b, int c) {
 }
 
 // tile of row block j and columns of pair (k16) or block (k8) k of the nr x nc
-// column-major matrix A (row stride 1, column stride ld), zero outside
-static void pack_tile(std::vector<uint32_t> &out, const float *A, int nr, int nc, int nrp, int ncp,
-                      int ld, int j, int k, bool k16, float s) {
+// column-major matrix A (row stride 1, column stride ld), zero outside; nrp, ncp:
+// extents whose blocks the indices run over
+struct PackTile {
+  const float *A;
+  int nr, nc, nrp, ncp, ld, j, k;
+  bool k16;
+  float s;
+};
+
+static void pack_tile(const PackTile &q, uint32_t *out) {
   for (int lane = 0; lane < 32; ++lane) {
-    const int r = warp_node(nrp, j, lane / 4), c = 2 * (lane % 4);
+    const int r = warp_node(q.nrp, q.j, lane / 4), c = 2 * (lane % 4);
     auto at = [&](int b, int slot) {
-      const int col = warp_node(ncp, b, slot);
-      return r < nr && col < nc ? A[r + (size_t)col * ld] * s : 0.f;
+      const int col = warp_node(q.ncp, b, slot);
+      return r < q.nr && col < q.nc ? q.A[r + (size_t)col * q.ld] * q.s : 0.f;
     };
-    const int b0 = k16 ? 2 * k : k;
-    for (int lo = 0; lo < 2; ++lo) {
-      out.push_back(pack_pair(at(b0, c), at(b0, c + 1), lo));
-      if (k16) out.push_back(pack_pair(at(b0 + 1, c), at(b0 + 1, c + 1), lo));
+    if (q.k16) {
+      uint32_t *o = out + 4 * lane;
+      pack_pair(at(2 * q.k, c), at(2 * q.k, c + 1), o[0], o[2]);
+      pack_pair(at(2 * q.k + 1, c), at(2 * q.k + 1, c + 1), o[1], o[3]);
+    } else {
+      pack_pair(at(q.k, c), at(q.k, c + 1), out[2 * lane], out[2 * lane + 1]);
     }
   }
 }
@@ -113,35 +121,43 @@ void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<floa
   for (int d = 1; d < 3; ++d) sD = std::min(sD, operator_scale(D[d].data(), D[d].size()));
   const float sL = operator_scale(LIFT.data(), LIFT.size());
   const float sV = operator_scale(Vq.data(), Vq.size()), sP = operator_scale(Pq.data(), Pq.size());
-  out.clear();
-  auto at = [&]() { return (int)(out.size() / 4); };
+  std::vector<PackTile> tiles;
+  std::vector<size_t> offset;
+  size_t words = 0;
+  auto add = [&](const PackTile &q) {
+    tiles.push_back(q), offset.push_back(words);
+    words += q.k16 ? 128 : 64;
+  };
+  auto at = [&]() { return (int)(words / 4); };
   for (int d = 0; d < 3; ++d)
     for (int k = 0; k < KP; ++k)
-      for (int j = 0; j < NB; ++j) pack_tile(out, D[d].data(), Np, Np, Np, Np, Np, j, k, true, sD);
+      for (int j = 0; j < NB; ++j) add({D[d].data(), Np, Np, Np, Np, Np, j, k, true, sD});
   pl.oDt = at();
   for (int d = 0; d < 3 && KT; ++d)
-    for (int j = 0; j < NB; ++j) pack_tile(out, D[d].data(), Np, Np, Np, Np, Np, j, 2 * KP, false, sD);
+    for (int j = 0; j < NB; ++j) add({D[d].data(), Np, Np, Np, Np, Np, j, 2 * KP, false, sD});
   pl.oL = at();
   auto face = [&](int f) { return LIFT.data() + (size_t)f * Nfp * Np; };
   for (int f = 0; f < 4; ++f)
     for (int k = 0; k < FP; ++k)
-      for (int j = 0; j < NB; ++j) pack_tile(out, face(f), Np, Nfp, Np, Nfp, Np, j, k, true, sL);
+      for (int j = 0; j < NB; ++j) add({face(f), Np, Nfp, Np, Nfp, Np, j, k, true, sL});
   pl.oLt = at();
   for (int f = 0; f < 4 && FT; ++f)
-    for (int j = 0; j < NB; ++j) pack_tile(out, face(f), Np, Nfp, Np, Nfp, Np, j, 2 * FP, false, sL);
+    for (int j = 0; j < NB; ++j) add({face(f), Np, Nfp, Np, Nfp, Np, j, 2 * FP, false, sL});
   pl.oV = at();
   for (int c = 0; c < nch; ++c)
     for (int k = 0; k < KP; ++k)
-      for (int h = 0; h < 2; ++h)
-        pack_tile(out, Vq.data(), Nq, Np, Nq16, Np, Nq, 2 * c + h, k, true, sV);
+      for (int h = 0; h < 2; ++h) add({Vq.data(), Nq, Np, Nq16, Np, Nq, 2 * c + h, k, true, sV});
   pl.oVt = at();
   for (int c = 0; c < nch && KT; ++c)
-    for (int h = 0; h < 2; ++h)
-      pack_tile(out, Vq.data(), Nq, Np, Nq16, Np, Nq, 2 * c + h, 2 * KP, false, sV);
+    for (int h = 0; h < 2; ++h) add({Vq.data(), Nq, Np, Nq16, Np, Nq, 2 * c + h, 2 * KP, false, sV});
   pl.oP = at();
   for (int c = 0; c < nch; ++c)
-    for (int j = 0; j < NB; ++j) pack_tile(out, Pq.data(), Np, Nq, Np, Nq16, Np, j, c, true, sP);
+    for (int j = 0; j < NB; ++j) add({Pq.data(), Np, Nq, Np, Nq16, Np, j, c, true, sP});
   pl.ops_n = at();
+  out.resize(words);
+  const long long nt = (long long)tiles.size();
+#pragma omp parallel for schedule(static) num_threads(8) if (nt > 128)
+  for (long long i = 0; i < nt; ++i) pack_tile(tiles[i], &out[offset[i]]);
   pl.iD = 1.f / sD, pl.iL = 1.f / sL, pl.iV = 1.f / sV, pl.iP = 1.f / sP;
   double vn = 0.0;
   for (int q = 0; q < Nq; ++q) {
@@ -169,10 +185,27 @@ __global__ void k_medium(int K, int Nq, int Nq16, const float *__restrict__ c2q,
   if (lane == 0) c2max[k] = m;
 }
 
-bbw_status warp_medium(int K, int Nq, const float *c2q, float *c2max, float *c2p,
-                       cudaStream_t st) {
-  k_medium<<<(K + 7) / 8, 256, 0, st>>>(K, Nq, (Nq + 15) / 16 * 16, c2q, c2max, c2p);
-  return check_launch("medium bound");
+// one thread per float of the records: fgeo 16 | vgeo 9 | pad 3, rows past K zero
+__global__ void k_records(int K, const float *__restrict__ vgeo, const float *__restrict__ fgeo,
+                          float *__restrict__ geo) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long k = i / 28;
+  const int c = (int)(i - k * 28);
+  if (k >= K + 16) return;
+  geo[i] = k >= K || c >= 25 ? 0.f : c < 16 ? fgeo[k * 16 + c] : vgeo[k * 9 + c - 16];
+}
+
+bbw_status geometry_records(int K, const float *vgeo, const float *fgeo, float *geo) {
+  const long long n = (long long)(K + 16) * 28;
+  k_records<<<(int)((n + 255) / 256), 256>>>(K, vgeo, fgeo, geo);
+  const bbw_status s = check_launch("geometry records");
+  return s != BBW_OK ? s : set_cuda_error(cudaStreamSynchronize(nullptr), "geometry records");
+}
+
+bbw_status warp_medium(int K, int Nq, const float *c2q, float *c2max, float *c2p) {
+  k_medium<<<(K + 7) / 8, 256>>>(K, Nq, (Nq + 15) / 16 * 16, c2q, c2max, c2p);
+  const bbw_status s = check_launch("medium bound");
+  return s != BBW_OK ? s : set_cuda_error(cudaStreamSynchronize(nullptr), "medium bound");
 }
 
 }  // namespace bbw

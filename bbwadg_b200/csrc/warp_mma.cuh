@@ -1,0 +1,332 @@
+// Shared pieces of the stages on warp-level matrix instructions (warp_stage.cuh,
+// group_stage.cuh): mma.sync m16n8k16 on FP16 pairs with FP32 accumulation.
+//
+// Elements are the rows (M = 16) of every product and operator rows the
+// columns, so the accumulators of one contraction have the register layout of
+// the next one's A operand.  mma.sync gives 1024 FMA per cycle and SM here (8
+// cycles per m16n8k16 and SM quarter, measured; k8 costs the same), a quarter of
+// what tcgen05 does on full tiles, with a latency of 21 cycles and no TMEM
+// round trip: the contractions are skinny (K = Np, Nfp or Nq per element), and
+// the chain of dependent phases bounds them, not the tensor rate.
+//
+// FP32 values x are split into FP16 pairs x s = hi + lo with a power of two s
+// per element and operand, so each element keeps its own dynamic range; the
+// pair holds 23 bits.  With four products (hi hi, hi lo, lo hi, lo lo) the
+// contraction error is that of FP32 sums; the split-FP16 form uses three.
+#pragma once
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <type_traits>
+
+#include "device_common.cuh"
+#include "warp_stage.h"
+
+namespace bbw {
+
+struct WarpParams {
+  int K, K0, Kc, Nq, Nq16, bc, pat_off, table_ints, bs, ws, nt32;
+  int nit, ntile, step_shot, step_tile;  // items; tiles per shot; a group's stride in both
+  int oDt, oL, oLt, oV, oVt, oP, ops_n;  // operator offsets and size in uint4
+  float fa, fb, fdt, cstage;
+  float iD, iL, iV, iP, vnorm;      // inverse operator scales, max row sum of |Vq|
+  const float *__restrict__ Qin;
+  float *__restrict__ Qout;
+  float *__restrict__ res;
+  const float *__restrict__ geo;    // [K + 16][28]: fgeo 16 | vgeo 9 | pad
+  const float *__restrict__ c2p;    // [K][Nq16], zero past Nq
+  const float *__restrict__ c2max;
+  const int *__restrict__ nbr;
+  const int *__restrict__ tables;
+  const uint4 *__restrict__ ops;
+  const int *__restrict__ src_tile;
+  const int *__restrict__ src_elem;
+  const float *__restrict__ src_vec;
+  float f0, tR, samp;
+  const double *__restrict__ time;
+};
+
+__device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                      uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "{%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(b0));
+}
+
+// A operand of one k16 step: FP16 pairs of 16 elements x 16 columns.  Lane
+// l holds elements l/4 (indices 0, 2) and l/4 + 8 (1, 3) at columns
+// 4 (l%4) + {0, 1} (indices 0, 1) and + {2, 3}: the operators are packed with
+// the matching column order, so four consecutive nodes sit in one lane.
+struct Frag {
+  uint32_t h[4], l[4];
+};
+struct Frag8 {  // a k8 step: columns 2 (l%4) + {0, 1}
+  uint32_t h[2], l[2];
+};
+
+// x s = hi + lo for two values; s2 = (s, s)
+__device__ __forceinline__ void split2(float2 x, float2 s2, uint32_t &h, uint32_t &l) {
+  const float2 y = __fmul2_rn(x, s2);
+  const __half2 hh = __float22half2_rn(y);
+  const float2 f = __half22float2(hh);
+  const __half2 ll = __float22half2_rn(__fadd2_rn(y, make_float2(-f.x, -f.y)));
+  h = *reinterpret_cast<const uint32_t *>(&hh);
+  l = *reinterpret_cast<const uint32_t *>(&ll);
+}
+__device__ __forceinline__ float2 both(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 lo2(const float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4 v) { return make_float2(v.z, v.w); }
+// LSRK update of two values: r = fa r + fdt x (returned), q += fb r
+__device__ __forceinline__ float2 lsrk2(float2 r, float2 x, float2 fa, float2 fdt) {
+  return __ffma2_rn(fa, r, __fmul2_rn(fdt, x));
+}
+// rows a (elements l/4) and b (l/4 + 8), scaled by ca and cb
+__device__ __forceinline__ void split_frag(Frag &f, const float4 a, const float4 b, float ca,
+                                           float cb) {
+  split2(lo2(a), both(ca), f.h[0], f.l[0]);
+  split2(lo2(b), both(cb), f.h[1], f.l[1]);
+  split2(hi2(a), both(ca), f.h[2], f.l[2]);
+  split2(hi2(b), both(cb), f.h[3], f.l[3]);
+}
+__device__ __forceinline__ void split_frag(Frag8 &f, const float2 a, const float2 b, float ca,
+                                           float cb) {
+  split2(a, both(ca), f.h[0], f.l[0]);
+  split2(b, both(cb), f.h[1], f.l[1]);
+}
+
+// leading products into c, corrections into e (the same array, or its own so
+// that the small terms add up before they meet the large ones: the matrix
+// unit's sums round toward zero, so fewer large sums leave less bias)
+template <int PR>
+__device__ __forceinline__ void mma_tile(float (&c)[4], float (&e)[4], const Frag &x,
+                                         const uint4 b) {
+  mma16(c, x.h, b.x, b.y);
+  mma16(e, x.h, b.z, b.w);
+  mma16(e, x.l, b.x, b.y);
+  if constexpr (PR == 4) mma16(e, x.l, b.z, b.w);
+}
+template <int PR, int M>
+__device__ __forceinline__ void mma_tiles(float (&c)[M][4], float (&e)[M][4], const Frag &x,
+                                          const uint4 (&b)[M]) {
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma16(c[i], x.h, b[i].x, b[i].y);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma16(e[i], x.h, b[i].z, b[i].w);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma16(e[i], x.l, b[i].x, b[i].y);
+  if constexpr (PR == 4) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) mma16(e[i], x.l, b[i].z, b[i].w);
+  }
+}
+template <int PR, int M>
+__device__ __forceinline__ void mma_tiles(float (&c)[M][4], float (&e)[M][4], const Frag8 &x,
+                                          const uint2 (&b)[M]) {
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma8(c[i], x.h[0], x.h[1], b[i].x);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma8(e[i], x.h[0], x.h[1], b[i].y);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma8(e[i], x.l[0], x.l[1], b[i].x);
+  if constexpr (PR == 4) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) mma8(e[i], x.l[0], x.l[1], b[i].y);
+  }
+}
+
+__device__ __forceinline__ void mma_hl(float (&c)[4], const uint32_t (&a)[4], const uint4 b, bool lo) {
+  if (lo) mma16(c, a, b.z, b.w);
+  else mma16(c, a, b.x, b.y);
+}
+__device__ __forceinline__ void mma_hl(float (&c)[4], const uint32_t (&a)[2], const uint2 b, bool lo) {
+  mma8(c, a[0], a[1], lo ? b.y : b.x);
+}
+// two operands on the same tiles, interleaved: an accumulator is used again
+// only after the 21 cycles that a product takes
+template <int PR, int M, class F, class T>
+__device__ __forceinline__ void mma_pair(float (&c)[M][4], float (&e)[M][4], const F &x,
+                                         float (&cc)[M][4], float (&ee)[M][4], const F &y,
+                                         const T (&b)[M]) {
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma_hl(c[i], x.h, b[i], false);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma_hl(cc[i], y.h, b[i], false);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma_hl(e[i], x.h, b[i], true);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.h, b[i], true);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma_hl(e[i], x.l, b[i], false);
+#pragma unroll
+  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, b[i], false);
+  if constexpr (PR == 4) {
+#pragma unroll
+    for (int i = 0; i < M; ++i) mma_hl(e[i], x.l, b[i], true);
+#pragma unroll
+    for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, b[i], true);
+  }
+}
+
+// power of two that brings a maximum m below 2^15, as an exponent field; the
+// inverse is the field 254 - f.  Clamped so that both stay normal numbers
+// (m below 2^-99, zero included, takes 2^113).
+__device__ __forceinline__ int scale_field(float m) {
+  const int e = (int)((__float_as_uint(m) >> 23) & 255u);
+  return min(max(268 - e, 14), 240);
+}
+__device__ __forceinline__ float pow2_field(int f) { return __uint_as_float((uint32_t)f << 23); }
+
+// maximum over the four lanes that share an element row
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+__device__ __forceinline__ float max4(float m, const float4 v) {
+  return fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+__device__ __forceinline__ float max2(float m, const float2 v) {
+  return fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y)));
+}
+
+// x[n .. n+3] (n a multiple of 4) and x[n .. n+1] (n even) of a row of LEN
+// values, zero past its end; V: widest aligned access
+template <int LEN, int V>
+__device__ __forceinline__ float4 load4(const float *x, int n) {
+  if constexpr (V == 4) {
+    return n < LEN ? *reinterpret_cast<const float4 *>(x + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+  } else if constexpr (V == 2) {
+    const float2 z = make_float2(0.f, 0.f);
+    const float2 a = n < LEN ? *reinterpret_cast<const float2 *>(x + n) : z;
+    const float2 b = n + 2 < LEN ? *reinterpret_cast<const float2 *>(x + n + 2) : z;
+    return make_float4(a.x, a.y, b.x, b.y);
+  } else {
+    return make_float4(n < LEN ? x[n] : 0.f, n + 1 < LEN ? x[n + 1] : 0.f,
+                       n + 2 < LEN ? x[n + 2] : 0.f, n + 3 < LEN ? x[n + 3] : 0.f);
+  }
+}
+template <int LEN, int V>
+__device__ __forceinline__ float2 load2(const float *x, int n) {
+  if constexpr (V >= 2) {
+    return n < LEN ? *reinterpret_cast<const float2 *>(x + n) : make_float2(0.f, 0.f);
+  } else {
+    return make_float2(n < LEN ? x[n] : 0.f, n + 1 < LEN ? x[n + 1] : 0.f);
+  }
+}
+template <int LEN, int V>
+__device__ __forceinline__ void store4(float *x, int n, const float4 v) {
+  if constexpr (V == 4) {
+    if (n < LEN) *reinterpret_cast<float4 *>(x + n) = v;
+  } else if constexpr (V == 2) {
+    if (n < LEN) *reinterpret_cast<float2 *>(x + n) = make_float2(v.x, v.y);
+    if (n + 2 < LEN) *reinterpret_cast<float2 *>(x + n + 2) = make_float2(v.z, v.w);
+  } else {
+    if (n < LEN) x[n] = v.x;
+    if (n + 1 < LEN) x[n + 1] = v.y;
+    if (n + 2 < LEN) x[n + 2] = v.z;
+    if (n + 3 < LEN) x[n + 3] = v.w;
+  }
+}
+template <int LEN, int V>
+__device__ __forceinline__ void store2(float *x, int n, const float2 v) {
+  if constexpr (V >= 2) {
+    if (n < LEN) *reinterpret_cast<float2 *>(x + n) = v;
+  } else {
+    if (n < LEN) x[n] = v.x;
+    if (n + 1 < LEN) x[n + 1] = v.y;
+  }
+}
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
+
+// Ricker wavelet amp (1 - 2 a^2) exp(-a^2), a = pi f0 (t - tR)
+__device__ __forceinline__ float warp_ricker(float t, float f0, float tR, float amp) {
+  const float a = 3.14159265358979f * f0 * (t - tR);
+  return amp * (1.f - 2.f * a * a) * expf(-a * a);
+}
+
+// bulk L2 prefetch of [p, p + bytes), trimmed to 16-byte boundaries
+__device__ __forceinline__ void prefetch_l2(const void *p, size_t bytes) {
+  const size_t a = (reinterpret_cast<size_t>(p) + 15) & ~(size_t)15;
+  const size_t e = (reinterpret_cast<size_t>(p) + bytes) & ~(size_t)15;
+  if (e > a)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(a), "r"((uint32_t)(e - a)));
+}
+
+// res = fa res + fdt rhs, Q += fb res for four values
+__device__ __forceinline__ void lsrk4(const float4 r0, const float4 x, const float4 q0,
+                                      const WarpParams &P, float4 &r, float4 &q) {
+  const float2 a = lsrk2(lo2(r0), lo2(x), both(P.fa), both(P.fdt));
+  const float2 b = lsrk2(hi2(r0), hi2(x), both(P.fa), both(P.fdt));
+  const float2 c = __ffma2_rn(both(P.fb), a, lo2(q0)), d = __ffma2_rn(both(P.fb), b, hi2(q0));
+  r = make_float4(a.x, a.y, b.x, b.y), q = make_float4(c.x, c.y, d.x, d.y);
+}
+
+// sources of the tile's elements k0 .. k0 + 15, in the reference's place: added
+// to the projected rhs_p (acous_elas_cpp/okl/ElasKernelsWADG.okl:400-403).
+// add(row in the tile, amplitude, vector)
+template <class F>
+__device__ __forceinline__ void tile_sources(const WarpParams &P, int Np, int shot, int k0, F &&add) {
+  const int tb = shot * P.nt32 + k0 / 32, te = shot * P.nt32 + min(k0 + 15, P.K - 1) / 32;
+  const int j0 = __ldg(P.src_tile + tb), j1 = __ldg(P.src_tile + te + 1);
+  if (j1 <= j0) return;
+  const float amp = warp_ricker((float)(*P.time) + P.cstage * P.fdt, P.f0, P.tR, P.samp);
+  for (int s = j0; s < j1; ++s) {
+    const int e = __ldg(P.src_elem + s) - k0;
+    if (e >= 0 && e < 16) add(e, amp, P.src_vec + (size_t)s * Np);
+  }
+}
+
+// launch parameters common to both forms; the grid walks nit items
+inline WarpParams warp_params(const WarpPlan &pl, const float *Qin, float *Qout, float *res, float fa,
+                              float fb, float fdt, float cstage) {
+  WarpParams P{};
+  P.K = pl.K, P.K0 = pl.K0, P.Kc = pl.Kc > 0 ? pl.Kc : pl.K, P.Nq = pl.Nq, P.bc = pl.bc;
+  P.pat_off = pl.pat_off, P.table_ints = pl.table_ints, P.nt32 = (pl.K + 31) / 32;
+  P.Nq16 = (pl.Nq + 15) / 16 * 16;
+  P.oDt = pl.oDt, P.oL = pl.oL, P.oLt = pl.oLt, P.oV = pl.oV, P.oVt = pl.oVt, P.oP = pl.oP;
+  P.ops_n = pl.ops_n;
+  P.fa = fa, P.fb = fb, P.fdt = fdt, P.cstage = cstage;
+  P.iD = pl.iD, P.iL = pl.iL, P.iV = pl.iV, P.iP = pl.iP, P.vnorm = pl.vnorm;
+  P.Qin = Qin, P.Qout = Qout, P.res = res;
+  P.geo = pl.geo, P.c2p = pl.c2p, P.c2max = pl.c2max, P.nbr = pl.nbr;
+  P.tables = pl.tables, P.ops = pl.ops;
+  P.src_tile = pl.src_tile, P.src_elem = pl.src_elem, P.src_vec = pl.src_vec;
+  P.f0 = pl.f0, P.tR = pl.tR, P.samp = pl.samp, P.time = pl.time;
+  P.ntile = (P.Kc - P.K0 + 15) / 16;
+  P.nit = P.ntile * pl.S;
+  return P;
+}
+
+// items walked by `per_cta` workers (warps or groups) of each CTA; returns the grid
+inline int warp_grid(const WarpPlan &pl, int per_cta, WarpParams &P) {
+  const int ctas = pl.max_ctas > 0 && pl.max_ctas < pl.nsm ? pl.max_ctas : pl.nsm;
+  int grid = ctas;
+  if (P.nit <= ctas * per_cta) {
+    // at most one item per worker: spread the items over the SMs first
+    grid = P.nit < ctas ? P.nit : ctas;
+    P.bs = 1, P.ws = grid;
+  } else {
+    // a CTA's workers walk neighbouring tiles, whose traces they share in L1
+    P.bs = per_cta, P.ws = 1;
+  }
+  P.step_shot = grid * per_cta / P.ntile, P.step_tile = grid * per_cta % P.ntile;
+  return grid;
+}
+
+}  // namespace bbw

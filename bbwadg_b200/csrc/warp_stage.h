@@ -10,10 +10,13 @@
 
 namespace bbw {
 
+// which form of the stage a context runs (auto: stage_form's rule)
+enum WarpForm { WARP_AUTO = 0, WARP_SINGLE = 1, WARP_GROUP = 2 };
+
 struct WarpPlan {
-  bool on = false;       // the context may run its stage on this form
-  bool pinned = false;   // chosen by the autotuner or the caller
-  bool ops_sm = false;   // operators staged in shared memory
+  bool single = false, group = false;  // forms this context's sizes allow
+  int pinned = WARP_AUTO;              // form chosen by the autotuner or the caller
+  bool warp_ops = false, group_ops = false;  // operators staged in shared memory
   int products = 4;      // products per split pair (4: FP32 contexts, 3: split FP16)
   int N = 0, K = 0, K0 = 0, Kc = 0, Nq = 0, bc = 0, S = 1, nsm = 148, max_ctas = 0;
   int pat_off = 0, table_ints = 0;
@@ -39,22 +42,35 @@ struct WarpPlan {
 void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
                const std::vector<float> &Vq, const std::vector<float> &Pq,
                std::vector<uint32_t> &out);
-bool warp_supported(int N);
-// Whether the form is the default for `elements` (mesh elements times shots).
-// A warp takes a 16-element tile from end to end, so a mesh of few tiles
-// leaves most of the chip idle for the length of one tile, while the CTA-wide
-// forms put 8 or 16 warps on a tile.  us per stage, this form against the FP32
-// fused stage: N = 3, K = 3072: 11.5 / 10.2, K = 6000: 11.5 / 17.2; N = 5, K =
-// 3072: 24.6 / 23.8, K = 6000: 25.4 / 43.1; N = 8, K = 1296: 206 / 187, K = 6000:
-// 273 / 564.  At N = 6 and 7 it is the faster one from the smallest mesh on
-// (K = 384: 44.7 / 73.3 and 80.4 / 112).
-inline bool warp_preferred(int N, long long elements) {
-  return N == 6 || N == 7 || elements > 296 * 16;
-}
+// Sets the forms that fit (pl.single, pl.group).
 bbw_status warp_prepare(WarpPlan &pl);
-bbw_status warp_launch(const WarpPlan &pl, const float *Qin, float *Qout, float *res, float fa,
-                       float fb, float fdt, float cstage, cudaStream_t st);
+// The form for `elements` (mesh elements times shots) when none is pinned;
+// WARP_AUTO: the CTA-wide stages.  The forms give the same results bit for
+// bit.  us per stage, CTA-wide FP32 / one warp / group:
+//   N = 2  K = 1296: 7.4 / 9.9 / -      K = 6000: 12.0 / 10.2 / -
+//   N = 3  K = 3072: 10.2 / 11.5 / -    K = 6000: 17.2 / 11.5 / -
+//   N = 4  K = 3072: 16.8 / 18.2 / 13.5 K = 10368: 43.4 / 23.0 / 34.5
+//   N = 5  K = 384: 23.3 / 24.4 / 11.5  K = 196608: 879 / 422 / 414
+//   N = 6  K = 384: 73 / 45 / 29        K = 24576: 454 / 154 / 143
+//   N = 7  K = 384: 112 / 80 / 34       K = 24576: 706 / 327 / 257
+// One warp per tile pays once there are about two tiles per SM; the group
+// form, three tiles or more per SM at a time, up to the 592 tiles of its first
+// wave at N = 4, and at every size above.
+inline int stage_form(const WarpPlan &pl, long long elements) {
+  const long long tiles = elements / 16;
+  if (pl.pinned != WARP_AUTO) return pl.pinned;
+  if (pl.group && (pl.N >= 5 || tiles <= 4 * 148)) return WARP_GROUP;
+  return pl.single && tiles > 2 * 148 ? WARP_SINGLE : WARP_AUTO;
+}
+bbw_status warp_launch(const WarpPlan &pl, int form, const float *Qin, float *Qout, float *res,
+                       float fa, float fb, float fdt, float cstage, cudaStream_t st);
+// geometry records [K + 16][28] of the tensor-core and warp-matrix stages (device
+// pointers): fgeo 16 | vgeo 9 | pad, a tile's worth of zero records at the end
+// Both setup kernels run on the legacy stream, behind the copies and fills that
+// made their arguments, and have ended on return: the contexts' streams do
+// not wait for that stream.
+bbw_status geometry_records(int K, const float *vgeo, const float *fgeo, float *geo);
 // c2max[k] = max_q |c2q[k][q]|; c2p[k]: c2q[k] padded with zeros to a multiple of 16
-bbw_status warp_medium(int K, int Nq, const float *c2q, float *c2max, float *c2p, cudaStream_t st);
+bbw_status warp_medium(int K, int Nq, const float *c2q, float *c2max, float *c2p);
 
 }  // namespace bbw
