@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <vector>
@@ -43,10 +44,11 @@ struct bbw_curved {
   int cur = 0;
   std::vector<int> perm;              // new element index -> reference index
   CurvedStageArgs args{};
+  CurvedMma mma;                      // matrix form of the curved elements' stage
+  int *d_perm = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   uint32_t graph_dt_bits[2] = {0, 0};
   std::vector<void *> owned;
-  std::vector<float> host;            // permutation scratch
 };
 
 namespace {
@@ -86,6 +88,71 @@ std::vector<T> rows(const T *a, const std::vector<int> &perm, size_t w, int from
   return out;
 }
 
+float max_row_sum(const float *A, int nr, int nc) {  // column-major nr x nc
+  double m = 0.0;
+  for (int i = 0; i < nr; ++i) {
+    double s = 0.0;
+    for (int j = 0; j < nc; ++j) s += std::fabs((double)A[i + (size_t)j * nr]);
+    m = std::max(m, s);
+  }
+  return (float)m;
+}
+
+// split operators and tiled point data of the curved elements' matrix stage;
+// leaves h->mma.on false where it does not fit
+bbw_status setup_mma(bbw_curved *h, const bbw_curved_desc *d) {
+  const CurvedStageArgs &S = h->args;
+  CurvedMma &M = h->mma;
+  const int Np = h->Np, Nfp = NFP(h->N), Nq = S.Nq, Nfq = S.Nfq, Nr = S.Nr;
+  M.KC = S.KC, M.k_off = S.k_off, M.nt = (S.KC + 15) / 16;
+  M.nch = (Nq + 15) / 16, M.nchr = (Nr + 15) / 16, M.FC = (Nfq + 15) / 16;
+  bbw_status s = curved_mma_prepare(h->N, M);
+  if (s == BBW_ERR_UNSUPPORTED) return BBW_OK;
+  if (s != BBW_OK) return s;
+  std::vector<uint32_t> ops;
+  const size_t mq = (size_t)Nq * Np, mr = (size_t)Nr * Np;
+  const float *V[4] = {d->Vq, d->Vrq, d->Vsq, d->Vtq}, *P[4] = {d->Pq, d->Prq, d->Psq, d->Ptq};
+  const float sV = split_scale(V, 1, mq), sD = split_scale(V + 1, 3, mq);
+  const float *pf[1] = {d->Pfq};
+  const float sP = std::min(split_scale(P, 4, mq), split_scale(pf, 1, (size_t)Np * 4 * Nfq));
+  for (int i = 0; i < 4; ++i) {
+    split_rows(ops, V[i], Nq, Np, i == 0 ? sV : sD, M.oV[i], M.oVt[i]);
+    split_columns(ops, P[i], Np, Nq, sP, M.oP[i]);
+  }
+  const float sF = split_scale(&d->VfqFace, 1, (size_t)Nfq * Nfp);
+  split_rows(ops, d->VfqFace, Nfq, Nfp, sF, M.oF, M.oFt);
+  for (int f = 0; f < 4; ++f) {
+    int off = 0;
+    split_columns(ops, d->Pfq + (size_t)f * Nfq * Np, Np, Nfq, sP, off);
+    if (f == 0) M.oL = off;
+  }
+  const float sVr = split_scale(&d->Vq_reduced, 1, mr), sPr = split_scale(&d->Pq_reduced, 1, mr);
+  split_rows(ops, d->Vq_reduced, Nr, Np, sVr, M.oVr, M.oVrt);
+  split_columns(ops, d->Pq_reduced, Np, Nr, sPr, M.oPr);
+  M.iV = 1.f / sV, M.iD = 1.f / sD, M.iP = 1.f / sP, M.iF = 1.f / sF, M.iVr = 1.f / sVr,
+  M.iPr = 1.f / sPr;
+  M.vnorm = max_row_sum(d->Vq, Nq, Np), M.rnorm = max_row_sum(d->Vq_reduced, Nr, Np);
+  M.fnorm = max_row_sum(d->VfqFace, Nfq, Nfp);
+  M.dnorm = std::max(max_row_sum(d->Vrq, Nq, Np),
+                     std::max(max_row_sum(d->Vsq, Nq, Np), max_row_sum(d->Vtq, Nq, Np)));
+  uint4 *dops = nullptr;
+  float *gq = nullptr, *fq = nullptr, *jq = nullptr, *bound = nullptr;
+  const size_t nt = M.nt;
+  const float *none = nullptr;
+  if ((s = own_upload(h, &dops, reinterpret_cast<const uint4 *>(ops.data()), ops.size() / 4,
+                      "bbw_curved_create: split operators")) != BBW_OK ||
+      (s = own_upload(h, &gq, none, nt * M.nch * 10 * 256, "bbw_curved_create")) != BBW_OK ||
+      (s = own_upload(h, &fq, none, nt * 4 * M.FC * 4 * 256, "bbw_curved_create")) != BBW_OK ||
+      (s = own_upload(h, &jq, none, nt * M.nchr * 2 * 256, "bbw_curved_create")) != BBW_OK ||
+      (s = own_upload(h, &bound, none, (size_t)M.KC * 8, "bbw_curved_create")) != BBW_OK ||
+      (s = curved_mma_points(S, M, gq, fq, jq, bound)) != BBW_OK)
+    return s;
+  M.ops = dops, M.gq = gq, M.fq = fq, M.jq = jq, M.bound = bound;
+  M.Fmask = S.Fmask, M.vmapP = S.vmapP;
+  M.on = true;
+  return BBW_OK;
+}
+
 bbw_status stage(bbw_curved *h, float fa, float fb, float fdt) {
   const float *Qin = h->Q[h->cur];
   float *Qout = h->Q[h->cur ^ 1];
@@ -100,9 +167,15 @@ bbw_status stage(bbw_curved *h, float fa, float fb, float fdt) {
   if (s == BBW_OK && h->KP > 0)
     s = launch_stage(h->aff, Qin, Qout, h->res, fa, fb, fdt, 0.f, h->stream);
   if (s == BBW_OK && h->KC > 0) {
-    CurvedStageArgs A = h->args;
-    A.fa = fa, A.fb = fb, A.fdt = fdt;
-    s = curved_stage(h->N, A, Qin, Qout, h->res, cst);
+    if (h->mma.on) {
+      CurvedMma A = h->mma;
+      A.fa = fa, A.fb = fb, A.fdt = fdt;
+      s = curved_mma_stage(h->N, A, Qin, Qout, h->res, cst);
+    } else {
+      CurvedStageArgs A = h->args;
+      A.fa = fa, A.fb = fb, A.fdt = fdt;
+      s = curved_stage(h->N, A, Qin, Qout, h->res, cst);
+    }
   }
   if (both) {  // join: the next stage reads what both wrote (always joined)
     cudaError_t e = cudaEventRecord(h->join, h->side);
@@ -222,7 +295,9 @@ extern "C" bbw_status bbw_curved_create(const bbw_curved_desc *d, int device, bb
     A.Vqr = own_upload_c(h, d->Vq_reduced, mr, s), A.Pqr = own_upload_c(h, d->Pq_reduced, mr, s);
     A.Fmask = own_upload_c(h, d->Fmask, (size_t)NF, s);
     A.vmapP = own_upload_c(h, vmapP.data(), vmapP.size(), s);
+    if (s == BBW_OK && curved_mma_preferred(N, d->KCurved)) s = setup_mma(h, d);
   }
+  if (s == BBW_OK) s = own_upload(h, &h->d_perm, perm.data(), perm.size(), "bbw_curved_create");
   // one stage on the zero state (it stays zero) sets the kernels' launch
   // attributes outside any later graph capture
   if (s == BBW_OK) s = stage(h, 0.f, 0.f, 0.f);
@@ -245,27 +320,38 @@ extern "C" bbw_status bbw_curved_destroy(bbw_curved *h) {
   return BBW_OK;
 }
 
-// host [K][4][Np] in the reference's element order <-> device buffer
+// rows of w4 float4: to_new: out[i] = in[perm[i]], else out[perm[i]] = in[i]
+__global__ void k_permute_rows(int K, int w4, bool to_new, const int *__restrict__ perm,
+                               const float4 *__restrict__ in, float4 *__restrict__ out) {
+  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long i = j / w4;
+  if (i >= K) return;
+  const long long c = j - i * w4, o = (long long)__ldg(perm + i) * w4 + c;
+  if (to_new) out[j] = in[o];
+  else out[o] = in[j];
+}
+
+// host [K][4][Np] in the reference's element order <-> device buffer, permuted on
+// the device through the next state's buffer, which every stage writes in full.
+// Permuting on the host and copying through pageable memory took 9 ms of the 28
+// ms of 20 steps at N = 3, K = 82944 (26 MB each way).
 static bbw_status copy_state(bbw_curved *h, float *dev, const float *src, float *dst,
                              const char *what) {
   if (!h || (!src && !dst)) return set_error(BBW_ERR_ARG, what);
-  const size_t w = (size_t)4 * h->Np, n = (size_t)h->K * w;
-  h->host.resize(n);
-  cudaError_t e;
-  if (src) {
-    for (int i = 0; i < h->K; ++i)
-      std::memcpy(&h->host[i * w], src + (size_t)h->perm[i] * w, w * sizeof(float));
-    e = cudaMemcpyAsync(dev, h->host.data(), n * sizeof(float), cudaMemcpyHostToDevice,
-                        h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  } else {
-    e = cudaMemcpyAsync(h->host.data(), dev, n * sizeof(float), cudaMemcpyDeviceToHost,
-                        h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e == cudaSuccess)
-      for (int i = 0; i < h->K; ++i)
-        std::memcpy(dst + (size_t)h->perm[i] * w, &h->host[i * w], w * sizeof(float));
+  const size_t n = (size_t)h->K * 4 * h->Np;
+  float *tmp = h->Q[h->cur ^ 1];
+  const int blocks = (int)(((size_t)h->K * h->Np + 255) / 256);
+  const float4 *in = reinterpret_cast<const float4 *>(src ? tmp : dev);
+  float4 *out = reinterpret_cast<float4 *>(src ? dev : tmp);
+  cudaError_t e = cudaSuccess;
+  if (src) e = cudaMemcpyAsync(tmp, src, n * sizeof(float), cudaMemcpyHostToDevice, h->stream);
+  if (e == cudaSuccess) {
+    k_permute_rows<<<blocks, 256, 0, h->stream>>>(h->K, h->Np, src != nullptr, h->d_perm, in, out);
+    e = cudaGetLastError();
   }
+  if (e == cudaSuccess && dst)
+    e = cudaMemcpyAsync(dst, tmp, n * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   return set_cuda_error(e, what);
 }
 

@@ -140,31 +140,6 @@ struct TileHalf<N, true> {  // more than 32 nodes per face
   __device__ __forceinline__ void flux(A... x) const { a.flux(x...), b.flux(x...); }
 };
 
-// barrier of one group's warps (named barrier 1 + group)
-template <int GW>
-__device__ __forceinline__ void group_sync(int grp) {
-  if constexpr (GW == 1) __syncwarp();
-  else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + grp), "n"(32 * GW) : "memory");
-}
-
-// split operand step k of an array of KP k16 steps (hi words of 32 lanes, then
-// lo words) followed by the k8 step (hi, hi, lo, lo)
-__device__ __forceinline__ Frag get_frag(const uint4 *a, int k, int lane) {
-  const uint4 h = a[k * 64 + lane], l = a[k * 64 + 32 + lane];
-  return Frag{{h.x, h.y, h.z, h.w}, {l.x, l.y, l.z, l.w}};
-}
-__device__ __forceinline__ void put_frag(uint4 *a, int k, int lane, const Frag &f) {
-  a[k * 64 + lane] = make_uint4(f.h[0], f.h[1], f.h[2], f.h[3]);
-  a[k * 64 + 32 + lane] = make_uint4(f.l[0], f.l[1], f.l[2], f.l[3]);
-}
-__device__ __forceinline__ Frag8 get_frag8(const uint4 *a, int KP, int lane) {
-  const uint4 q = a[KP * 64 + lane];
-  return Frag8{{q.x, q.y}, {q.z, q.w}};
-}
-__device__ __forceinline__ void put_frag8(uint4 *a, int KP, int lane, const Frag8 &f) {
-  a[KP * 64 + lane] = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
-}
-
 // the eight (pair: M = 2 blocks) or four (M = 1) values of a unit in one field
 // for rows a and b, as they sit in memory
 template <int M>
@@ -504,7 +479,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const Frag y = get_frag(sA + (c + 1) * AS, k, lane);
-            mma_pair<PR, m>(d[c], e[c], x, dv, ev, y, b[c]);
+            mma_pair2<PR, m>(d[c], e[c], x, b[c], dv, ev, y, b[c]);
           }
         }
         if constexpr (KT) {
@@ -517,7 +492,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const Frag8 y = get_frag8(sA + (c + 1) * AS, KP, lane);
-            mma_pair<PR, m>(d[c], e[c], x, dv, ev, y, b[c]);
+            mma_pair2<PR, m>(d[c], e[c], x, b[c], dv, ev, y, b[c]);
           }
         }
 #pragma unroll

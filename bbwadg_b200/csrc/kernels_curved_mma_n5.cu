@@ -1,0 +1,4 @@
+#include "curved_mma.cuh"
+namespace bbw {
+BBW_CURVED_MMA_INSTANCE(5)
+}

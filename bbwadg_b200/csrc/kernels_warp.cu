@@ -111,6 +111,40 @@ static void pack_tile(const PackTile &q, uint32_t *out) {
   }
 }
 
+float split_scale(const float *const *A, int n, size_t len) {
+  float s = operator_scale(A[0], len);
+  for (int i = 1; i < n; ++i) s = std::min(s, operator_scale(A[i], len));
+  return s;
+}
+
+void split_rows(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off,
+                int &off_tail) {
+  const int nch = (nr + 15) / 16, NB = (nc + 7) / 8, KP = NB / 2, KT = NB % 2;
+  off = (int)(out.size() / 4);
+  for (int c = 0; c < nch; ++c)
+    for (int k = 0; k < KP; ++k)
+      for (int h = 0; h < 2; ++h) {
+        out.resize(out.size() + 128);
+        pack_tile({A, nr, nc, 16 * nch, nc, nr, 2 * c + h, k, true, s}, &out[out.size() - 128]);
+      }
+  off_tail = (int)(out.size() / 4);
+  for (int c = 0; c < nch && KT; ++c)
+    for (int h = 0; h < 2; ++h) {
+      out.resize(out.size() + 64);
+      pack_tile({A, nr, nc, 16 * nch, nc, nr, 2 * c + h, 2 * KP, false, s}, &out[out.size() - 64]);
+    }
+}
+
+void split_columns(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off) {
+  const int nch = (nc + 15) / 16, NB = (nr + 7) / 8;
+  off = (int)(out.size() / 4);
+  for (int c = 0; c < nch; ++c)
+    for (int j = 0; j < NB; ++j) {
+      out.resize(out.size() + 128);
+      pack_tile({A, nr, nc, nr, 16 * nch, nr, j, c, true, s}, &out[out.size() - 128]);
+    }
+}
+
 void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
                const std::vector<float> &Vq, const std::vector<float> &Pq,
                std::vector<uint32_t> &out) {

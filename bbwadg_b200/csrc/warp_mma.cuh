@@ -152,29 +152,29 @@ __device__ __forceinline__ void mma_hl(float (&c)[4], const uint32_t (&a)[4], co
 __device__ __forceinline__ void mma_hl(float (&c)[4], const uint32_t (&a)[2], const uint2 b, bool lo) {
   mma8(c, a[0], a[1], lo ? b.y : b.x);
 }
-// two operands on the same tiles, interleaved: an accumulator is used again
-// only after the 21 cycles that a product takes
+// two products x b and y bb, interleaved: an accumulator is used again only
+// after the 21 cycles that a product takes
 template <int PR, int M, class F, class T>
-__device__ __forceinline__ void mma_pair(float (&c)[M][4], float (&e)[M][4], const F &x,
-                                         float (&cc)[M][4], float (&ee)[M][4], const F &y,
-                                         const T (&b)[M]) {
+__device__ __forceinline__ void mma_pair2(float (&c)[M][4], float (&e)[M][4], const F &x,
+                                          const T (&b)[M], float (&cc)[M][4], float (&ee)[M][4],
+                                          const F &y, const T (&bb)[M]) {
 #pragma unroll
   for (int i = 0; i < M; ++i) mma_hl(c[i], x.h, b[i], false);
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(cc[i], y.h, b[i], false);
+  for (int i = 0; i < M; ++i) mma_hl(cc[i], y.h, bb[i], false);
 #pragma unroll
   for (int i = 0; i < M; ++i) mma_hl(e[i], x.h, b[i], true);
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.h, b[i], true);
+  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.h, bb[i], true);
 #pragma unroll
   for (int i = 0; i < M; ++i) mma_hl(e[i], x.l, b[i], false);
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, b[i], false);
+  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, bb[i], false);
   if constexpr (PR == 4) {
 #pragma unroll
     for (int i = 0; i < M; ++i) mma_hl(e[i], x.l, b[i], true);
 #pragma unroll
-    for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, b[i], true);
+    for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, bb[i], true);
   }
 }
 
@@ -275,6 +275,31 @@ __device__ __forceinline__ void lsrk4(const float4 r0, const float4 x, const flo
   const float2 b = lsrk2(hi2(r0), hi2(x), both(P.fa), both(P.fdt));
   const float2 c = __ffma2_rn(both(P.fb), a, lo2(q0)), d = __ffma2_rn(both(P.fb), b, hi2(q0));
   r = make_float4(a.x, a.y, b.x, b.y), q = make_float4(c.x, c.y, d.x, d.y);
+}
+
+// barrier of one group's warps (named barrier 1 + group)
+template <int GW>
+__device__ __forceinline__ void group_sync(int grp) {
+  if constexpr (GW == 1) __syncwarp();
+  else asm volatile("bar.sync %0, %1;\n" ::"r"(1 + grp), "n"(32 * GW) : "memory");
+}
+
+// split operand step k of an array of KP k16 steps (hi words of 32 lanes, then
+// lo words) followed by the k8 step (hi, hi, lo, lo)
+__device__ __forceinline__ Frag get_frag(const uint4 *a, int k, int lane) {
+  const uint4 h = a[k * 64 + lane], l = a[k * 64 + 32 + lane];
+  return Frag{{h.x, h.y, h.z, h.w}, {l.x, l.y, l.z, l.w}};
+}
+__device__ __forceinline__ void put_frag(uint4 *a, int k, int lane, const Frag &f) {
+  a[k * 64 + lane] = make_uint4(f.h[0], f.h[1], f.h[2], f.h[3]);
+  a[k * 64 + 32 + lane] = make_uint4(f.l[0], f.l[1], f.l[2], f.l[3]);
+}
+__device__ __forceinline__ Frag8 get_frag8(const uint4 *a, int KP, int lane) {
+  const uint4 q = a[KP * 64 + lane];
+  return Frag8{{q.x, q.y}, {q.z, q.w}};
+}
+__device__ __forceinline__ void put_frag8(uint4 *a, int KP, int lane, const Frag8 &f) {
+  a[KP * 64 + lane] = make_uint4(f.h[0], f.h[1], f.l[0], f.l[1]);
 }
 
 // sources of the tile's elements k0 .. k0 + 15, in the reference's place: added

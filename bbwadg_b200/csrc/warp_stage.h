@@ -39,6 +39,14 @@ struct WarpPlan {
 // Order: D [3][KP][NB] and its k8 tiles [3][NB], LIFT [4][FP][NB] and [4][NB],
 // Vq [chunk][KP][2] and [chunk][2], Pq [chunk][NB].  Sets the offsets, inverse
 // scales and vnorm of the plan.
+// common power-of-two scale of n operators of `len` values
+float split_scale(const float *const *A, int n, size_t len);
+// Tiles of one column-major nr x nc operator, appended to out: split_rows
+// with its rows in chunks of 16 ([chunk][k16 step][2], then the k8 tails [chunk][2]),
+// split_columns with its columns in chunks of 16 ([chunk][row block]).
+void split_rows(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off,
+                int &off_tail);
+void split_columns(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off);
 void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
                const std::vector<float> &Vq, const std::vector<float> &Pq,
                std::vector<uint32_t> &out);
