@@ -12,6 +12,7 @@
 
 #include "bbwadg.h"
 #include "device_common.cuh"
+#include "ref_mma.h"
 
 namespace bbw {
 
@@ -512,6 +513,46 @@ static bbw_status launch_surface_bern_slice(int K, int bc, const float *fgeo, co
 
 using namespace bbw;
 
+// The matrix forms (ref_mma.cuh) read and write whole vectors
+static bool vectors(const void *a, const void *b, const void *c = nullptr) {
+  return (((size_t)a | (size_t)b | (size_t)c) & 15) == 0;
+}
+// and split the operators in every CTA, which few elements do not repay.  us,
+// thread per node / matrix:
+//   volume   N = 2 K = 24576: 8.6 / 10.5   N = 3 K = 3072: 7.6 / 8.5, K = 10368: 9.4 / 8.4
+//            N = 4 K = 384: 16.7 / 10.6    N = 5 K = 384: 16.6 / 12.6, K = 24576: 76 / 29
+//            N = 6 K = 384: 16.7 / 20.8, K = 3072: 26.8 / 21.2   N = 7 K = 384: 41 / 35
+//   surface  N = 2 K = 24576: 12.4 / 14.4  N = 3 K = 384: 10.4 / 7.3, K = 24576: 22.7 / 16.6
+//            N = 5 K = 24576: 139 / 29     N = 6 K = 384: 14.5 / 16.3, K = 3072: 24.7 / 16.5
+//   update   N = 2 K = 10368: 12.4 / 16.4, K = 24576: 20.6 / 18.2
+//            N = 3 K = 3072: 12.4 / 12.4, K = 10368: 16.6 / 14.5
+//            N = 4 K = 3072: 17.8 / 16.5   N = 5 K = 384: 16.5 / 17.6, K = 24576: 154 / 83
+//            N = 6 K = 384: 24.7 / 32.9, K = 3072: 56 / 51   (N = 7: 214 points do not fit)
+enum { REF_VOLUME, REF_SURFACE, REF_UPDATE };
+static bool matrix_form(int kernel, int N, int K) {
+  constexpr int never = 1 << 30;
+  constexpr int from[3][8] = {{never, never, never, 8000, 0, 0, 1500, 0},
+                              {never, never, never, 0, 0, 0, 1000, 1000},
+                              {never, never, 20000, 4000, 1000, 1000, 2500, 2500}};
+  return N >= 1 && N <= 7 && K >= from[kernel][N];
+}
+
+#define BBW_MMA_SWITCH(CALL) \
+  switch (N) {               \
+    case 3: return CALL(3);  \
+    case 4: return CALL(4);  \
+    case 5: return CALL(5);  \
+    case 6: return CALL(6);  \
+    case 7: return CALL(7);  \
+  }
+static bool update_fits(int N, int Nq) {
+#define CALL(n) ref_update_fits_##n(Nq)
+  if (N == 2) return CALL(2);
+  BBW_MMA_SWITCH(CALL)
+#undef CALL
+  return false;
+}
+
 // node indices are int32, as the reference's vmapP: K * 4 * Np < 2^31
 static bool too_many_nodes(int N, int K) { return (long long)K * 4 * NP(N) >= (1LL << 31); }
 
@@ -524,6 +565,11 @@ extern "C" bbw_status bbw_rk_volume(int N, int K, const float *vgeo, const float
     return set_error(BBW_ERR_UNSUPPORTED, "bbw_rk_volume: K * 4 * Np must be below 2^31");
   if (K == 0) return BBW_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (matrix_form(REF_VOLUME, N, K) && vectors(Q, rhsQ)) {
+#define CALL(n) ref_volume_##n(K, vgeo, Dr, Ds, Dt, Q, rhsQ, st)
+    BBW_MMA_SWITCH(CALL)
+#undef CALL
+  }
 #define CALL(n) launch_volume<n>(K, K, vgeo, Dr, Ds, Dt, Q, rhsQ, st)
   switch (N) {
     case 1: return CALL(1);
@@ -549,6 +595,11 @@ extern "C" bbw_status bbw_rk_surface(int N, int K, int bc, const float *fgeo, co
     return set_error(BBW_ERR_UNSUPPORTED, "bbw_rk_surface: K * 4 * Np must be below 2^31");
   if (K == 0) return BBW_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (matrix_form(REF_SURFACE, N, K) && vectors(Q, rhsQ)) {
+#define CALL(n) ref_surface_##n(K, bc, fgeo, Fmask, vmapP, LIFT, Q, rhsQ, st)
+    BBW_MMA_SWITCH(CALL)
+#undef CALL
+  }
 #define CALL(n) launch_surface<n>(K, K, bc, fgeo, Fmask, vmapP, LIFT, Q, rhsQ, st)
   switch (N) {
     case 1: return CALL(1);
@@ -589,6 +640,12 @@ extern "C" bbw_status bbw_rk_update_wadg(int N, int K, int Nq, const float *Vq, 
     return set_error(BBW_ERR_UNSUPPORTED, "bbw_rk_update_wadg: K * 4 * Np must be below 2^31");
   if (K == 0) return BBW_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  if (matrix_form(REF_UPDATE, N, K) && vectors(Q, rhsQ, resQ) && update_fits(N, Nq)) {
+#define CALL(n) ref_update_##n(K, Nq, Vq, Pq, Jq, c2q, fa, fb, fdt, rhsQ, resQ, Q, st)
+    if (N == 2) return CALL(2);
+    BBW_MMA_SWITCH(CALL)
+#undef CALL
+  }
 #define CALL(n) launch_wadg<n>(K, Nq, Vq, Pq, Jq, c2q, fa, fb, fdt, rhsQ, resQ, Q, st)
   switch (N) {
     case 1: return CALL(1);

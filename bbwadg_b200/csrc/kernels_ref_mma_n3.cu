@@ -1,0 +1,5 @@
+#include "ref_mma.cuh"
+namespace bbw {
+BBW_REF_RHS_INSTANCE(3)
+BBW_REF_UPDATE_INSTANCE(3)
+}
