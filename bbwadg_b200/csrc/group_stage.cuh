@@ -213,9 +213,10 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
   const int nops = OPS ? P.ops_n : 0;
   int *sTab = reinterpret_cast<int *>(sOps + nops);
   float *scr = reinterpret_cast<float *>(sTab + P.table_ints) + grp * C::SCR;
-  if constexpr (OPS)
-    for (int i = tid; i < P.ops_n; i += C::T) sOps[i] = __ldg(P.ops + i);
-  for (int i = tid; i < P.table_ints; i += C::T) sTab[i] = __ldg(P.tables + i);
+  // operators and tables, all copies in flight with the first tile's
+  if constexpr (OPS) stage_async<C::T>(sOps, P.ops, P.ops_n);
+  stage_async<C::T>(reinterpret_cast<uint4 *>(sTab), reinterpret_cast<const uint4 *>(P.tables),
+                    P.table_ints / 4);
   float *sQ = scr;                                            // state rows, then
   uint4 *sA = reinterpret_cast<uint4 *>(scr);                 // split p, Ur, Us, Ut
   constexpr int AS = KP * 64 + KT * 32, FS = FP * 64 + FT * 32;  // uint4 per operand, per face
@@ -226,7 +227,6 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
   float *sGeo = scr + C::TILE + C::FLUX + C::RPF + C::WF;
   float4 *sMax = reinterpret_cast<float4 *>(sGeo + C::GEO);   // [GW][16] |p|, |u|, |v|, |w|
   float *sMaxR = sGeo + C::GEO + GW * 64, *sInv = sMaxR + GW * 16;  // [GW][16], [4][16]
-  __syncthreads();
   const uint4 *ops = OPS ? sOps : P.ops;
   const uint4 *oD = ops + lane, *oL = ops + P.oL + lane, *oV = ops + P.oV + lane,
               *oP = ops + P.oP + lane;
@@ -264,6 +264,8 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
     fetch_tile(nshot, P.K0 + ntl * 16);
     codes(P.K0 + ntl * 16, code0, code1);
   }
+  cp_async_wait();
+  __syncthreads();
   for (; it < P.nit; it += step) {
     const int shot = nshot, k0 = P.K0 + ntl * 16;
     nshot += P.step_shot, ntl += P.step_tile;

@@ -250,6 +250,13 @@ __device__ __forceinline__ void store2(float *x, int n, const float2 v) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const float *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }
+// n uint4 to shared memory by T threads
+template <int T>
+__device__ __forceinline__ void stage_async(uint4 *dst, const uint4 *src, int n) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n; i += T) cp_async16(d + 16 * i, reinterpret_cast<const float *>(src + i));
+}
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }

@@ -118,13 +118,13 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
   const int nops = OPS ? P.ops_n : 0;
   int *sTab = reinterpret_cast<int *>(sOps + nops);
   float *scr = reinterpret_cast<float *>(sTab + P.table_ints) + warp * C::SCR;
-  if constexpr (OPS)
-    for (int i = tid; i < P.ops_n; i += C::T) sOps[i] = __ldg(P.ops + i);
-  for (int i = tid; i < P.table_ints; i += C::T) sTab[i] = __ldg(P.tables + i);
+  // operators and tables, all copies in flight with the first tile's
+  if constexpr (OPS) stage_async<C::T>(sOps, P.ops, P.ops_n);
+  stage_async<C::T>(reinterpret_cast<uint4 *>(sTab), reinterpret_cast<const uint4 *>(P.tables),
+                    P.table_ints / 4);
   float *sQ = scr, *sF = scr + C::TILE;
   if constexpr (FB * 8 > Nfp)  // flux columns past Nfp meet zero operator columns
     for (int i = lane; i < C::FLUX; i += 32) sF[i] = 0.f;
-  __syncthreads();
   const uint4 *ops = OPS ? sOps : P.ops;
   const uint4 *oD = ops + lane, *oL = ops + P.oL + lane, *oV = ops + P.oV + lane,
               *oP = ops + P.oP + lane;
@@ -160,6 +160,8 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
     fetch_tile(nshot, P.K0 + ntl * 16);
     codes(P.K0 + ntl * 16, code0, code1);
   }
+  cp_async_wait();
+  __syncthreads();
   for (; it < P.nit; it += step) {
     const int shot = nshot, k0 = P.K0 + ntl * 16;
     nshot += P.step_shot, ntl += P.step_tile;
