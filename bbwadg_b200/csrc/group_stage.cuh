@@ -1,5 +1,5 @@
 // One LSRK stage with every contraction on warp-level matrix instructions
-// (warp_mma.cuh), a group of three or four warps per 16-element tile.
+// (warp_mma.cuh), a group of three to eight warps per 16-element tile.
 //
 // Replaces rk_volume + rk_surface + rk_update_WADG of the reference
 // (cpp/okl/WaveKernels.okl:44-260, cpp/okl/WaveKernelsWADG.okl:1760-1887).
@@ -7,11 +7,11 @@
 // The group's warps split the operator rows and hand the next contraction's
 // operand to each other as ready fragments in shared memory, with a named
 // barrier between phases.  Against one warp per tile (warp_stage.cuh) a tile's
-// chain is three to four times shorter, which counts where a mesh has few tiles
+// chain is three to eight times shorter, which counts where a mesh has few tiles
 // or an element much work.  The results are the same bit for bit.  us per
 // stage, CTA-wide FP32 stage / one warp / group: N = 5, K = 3072: 23.8 / 24.6 /
-// 14.7, K = 196608: 879 / 422 / 414; N = 7, K = 24576: 706 / 327 / 257; N = 4, K =
-// 3072: 16.8 / 18.2 / 13.5.  Bound by instruction and L1 wavefront rate together
+// 13.5, K = 196608: 879 / 422 / 418; N = 7, K = 24576: 706 / 327 / 173; N = 4, K =
+// 3072: 16.8 / 18.2 / 13.1.  Bound by instruction and L1 wavefront rate together
 // (issue 31 %, L1 data pipe 56 %, tensor 28 %); without the products 261 us,
 // without global loads 399, without stores 325 (N = 5, K = 196608).
 #pragma once
@@ -29,10 +29,12 @@ struct GroupCfg {
   static constexpr int NB = (Np + 7) / 8, KP = NB / 2, KT = NB % 2;
   static constexpr int FB = (Nfp + 7) / 8, FP = FB / 2, FT = FB % 2;
   // a unit of work is a pair of blocks (or the odd last one); GW warps per
-  // group, NG groups per CTA
+  // group, NG groups per CTA.  us per stage at K = 24576 with three or four
+  // warps and two units each, 168 registers / one unit per warp: N = 6 145 / 123,
+  // N = 7 254 / 173 (one group of 255 registers; two of 128: 205).
   static constexpr int U = KP + KT;
-  static constexpr int GW = N == 4 || N == 6 ? 3 : 4;  // units per warp: 1, 1, 2, 2 at N = 4 .. 7
-  static constexpr int NG = 12 / GW;
+  static constexpr int GW = U;  // 3, 4, 6, 8 at N = 4 .. 7
+  static constexpr int NG = N <= 6 ? 12 / GW : 1;
   static constexpr int W = GW * NG, T = 32 * W;
   static constexpr bool KEEP = U <= GW;  // a warp's old state stays in registers
   static constexpr bool OPS = N <= 5;    // operators in shared memory when they fit
@@ -46,7 +48,8 @@ struct GroupCfg {
   __host__ __device__ static constexpr int row(int e) { return e * EW + ((e + 1) >> 1) * ODD; }
   static constexpr int FLUX = 4 * FB * 128;    // split face fluxes
   static constexpr int RPF = NB * 128;         // split rhs_p
-  static constexpr int RC = 8;                 // cubature chunks per round
+  static constexpr int RC = GW == 6 ? 12 : 8;  // cubature chunks per round
+  static constexpr bool EARLY = !OPS;  // residual of p loaded before the projection
   static constexpr int SCR1 = 8 * FB * 8;      // one warp's face fluxes of eight elements
   static constexpr int WF = RC * 256 > GW * SCR1 ? RC * 256 : GW * SCR1;  // split cubature values
   static constexpr int GEO = 16 * 28;
@@ -199,6 +202,13 @@ struct Unit<1> {
     put_frag8(a, u, lane, f);
   }
 };
+
+// operator fragment from shared or global memory
+template <bool OPS, class T>
+__device__ __forceinline__ T op_load(const T *p) {
+  if constexpr (OPS) return *p;
+  else return __ldg(p);
+}
 
 template <int N, int PR, bool OPS>
 __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpParams P) {
@@ -470,13 +480,23 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
       float rv[3][m][4], rr[m][4], rd[m][4];  // rr: lifted part, rd: divergence
       {
         float d[3][m][4] = {}, e[3][m][4] = {}, dv[m][4] = {}, ev[m][4] = {};
-#pragma unroll
-        for (int k = 0; k < KP; ++k) {
-          uint4 b[3][m];
+        // from L2 the next step's operators are loaded during a step's products
+        // (48 per warp, about the latency): with the projection's below N = 7
+        // 207 -> 183, N = 6 134 -> 129 us per stage
+        uint4 bk[2][3][m];
+        auto load_d = [&](int k) {
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int i = 0; i < m; ++i) b[c][i] = oD[((c * KP + k) * NB + 2 * u + i) * 32];
+            for (int i = 0; i < m; ++i)
+              bk[k & 1][c][i] = op_load<OPS>(oD + ((c * KP + k) * NB + 2 * u + i) * 32);
+        };
+        if constexpr (!OPS && KP > 0) load_d(0);
+#pragma unroll
+        for (int k = 0; k < KP; ++k) {
+          if (OPS) load_d(k);
+          else if (k + 1 < KP) load_d(k + 1);
+          const uint4 (&b)[3][m] = bk[k & 1];
           const Frag x = get_frag(sA, k, lane);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -489,7 +509,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int i = 0; i < m; ++i) b[c][i] = oDt[(c * NB + 2 * u + i) * 32];
+            for (int i = 0; i < m; ++i) b[c][i] = op_load<OPS>(oDt + (c * NB + 2 * u + i) * 32);
           const Frag8 x = get_frag8(sA, KP, lane);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
@@ -532,7 +552,11 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           xa[c] = lo2(qa[c + 1]), xb[c] = lo2(qb[c + 1]);
         }
       }
-#pragma unroll
+      // rolled up the loop needs fewer registers: us per stage unrolled / rolled,
+      // N = 6 131 / 123, N = 7 184 / 178 (K = 24576), N = 5 (K = 82944) split FP16
+      // 177 / 167, but FP32 182 / 186
+      constexpr int LU = OPS && PR == 4 ? 2 : 1;
+#pragma unroll LU
       for (int f0 = 0; f0 < 4; f0 += 2) {
         // corrections of all steps first, then the leading products: the
         // matrix unit rounds toward zero, so few large sums
@@ -548,12 +572,12 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           for (int k = 0; k < FP; ++k) {
             x[j][k] = get_frag(sFr + f * FS, k, lane);
 #pragma unroll
-            for (int i = 0; i < m; ++i) b[j][k][i] = oL[((f * FP + k) * NB + 2 * u + i) * 32];
+            for (int i = 0; i < m; ++i) b[j][k][i] = op_load<OPS>(oL + ((f * FP + k) * NB + 2 * u + i) * 32);
           }
           if constexpr (FT) {
             x8[j] = get_frag8(sFr + f * FS, FP, lane);
 #pragma unroll
-            for (int i = 0; i < m; ++i) b8[j][i] = oLt[(f * NB + 2 * u + i) * 32];
+            for (int i = 0; i < m; ++i) b8[j][i] = op_load<OPS>(oLt + (f * NB + 2 * u + i) * 32);
           }
         }
         auto all = [&](auto &&op) {
@@ -666,6 +690,23 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
     const int nch = P.Nq16 / 16;
     group_sync<GW>(grp);  // rhs_p ready
 
+    // residual of p: loaded here it is in flight during the projection, where
+    // the registers allow (N = 7 187 -> 173 us per stage, N = 4 19.3 -> 19.7)
+    float4 ra[UW], rb[UW];
+    auto load_rp = [&]() {
+#pragma unroll
+      for (int i = 0; i < UW; ++i) {
+        const int u = w + i * GW;
+        if (u < KP) {
+          ra[i] = load4<Np, V>(Ra, 16 * u + 4 * t), rb[i] = load4<Np, V>(Rb, 16 * u + 4 * t);
+        } else if (u < C::U) {
+          const float2 x = load2<Np, V>(Ra, 16 * u + 2 * t), y = load2<Np, V>(Rb, 16 * u + 2 * t);
+          ra[i] = make_float4(x.x, x.y, 0.f, 0.f), rb[i] = make_float4(y.x, y.y, 0.f, 0.f);
+        }
+      }
+    };
+    if constexpr (C::EARLY) load_rp();
+
     // ---- 5. WADG projection of rhs_p, RC chunks of 16 cubature points at a
     //         time: Vq and c2 of the warp's chunks, then Pq of its units
     float o[UW][2][4], oe[UW][2][4];
@@ -683,10 +724,17 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
       for (int c = c0 + w; c < cend; c += GW) {
         const float4 za = __ldg(Ca + c * 4), zb = __ldg(Cb + c * 4);
         float v[6][4] = {};
+        uint4 bv[OPS ? 1 : KP][2];
+        if constexpr (!OPS)
+#pragma unroll
+          for (int k = 0; k < KP; ++k)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) bv[k][i] = __ldg(oV + ((c * KP + k) * 2 + i) * 32);
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
           const Frag x = get_frag(sR, k, lane);
-          const uint4 b0 = oV[((c * KP + k) * 2) * 32], b1 = oV[((c * KP + k) * 2 + 1) * 32];
+          const uint4 b0 = OPS ? oV[((c * KP + k) * 2) * 32] : bv[OPS ? 0 : k][0],
+                      b1 = OPS ? oV[((c * KP + k) * 2 + 1) * 32] : bv[OPS ? 0 : k][1];
           mma16(v[0], x.h, b0.x, b0.y);
           mma16(v[1], x.h, b1.x, b1.y);
           mma16(v[2], x.h, b0.z, b0.w);
@@ -700,7 +748,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
         }
         if constexpr (KT) {
           const Frag8 x = get_frag8(sR, KP, lane);
-          const uint2 b0 = oVt[(c * 2) * 32], b1 = oVt[(c * 2 + 1) * 32];
+          const uint2 b0 = op_load<OPS>(oVt + (c * 2) * 32), b1 = op_load<OPS>(oVt + (c * 2 + 1) * 32);
           mma8(v[0], x.h[0], x.h[1], b0.x);
           mma8(v[1], x.h[0], x.h[1], b1.x);
           mma8(v[2], x.h[0], x.h[1], b0.y);
@@ -720,6 +768,34 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
         const float4 xb = make_float4(v[0][2] * vib * zb.x, v[0][3] * vib * zb.y,
                                       v[1][2] * vib * zb.z, v[1][3] * vib * zb.w);
         Unit<2>::split(sW, c - c0, lane, xa, xb, da, db);
+      }
+      if constexpr (!OPS && UW == 1) {
+        // operators from L2: the next four chunks' loads in flight
+        uint4 b[4][2];
+        auto load_p = [&](int c) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              b[j][i] = __ldg(oP + (min(c + j, nch - 1) * NB + min(2 * w + i, NB - 1)) * 32);
+        };
+        load_p(c0);
+        group_sync<GW>(grp);  // the round's values ready
+#pragma unroll 1
+        for (int c = c0; c < cend; c += 4) {
+          uint4 bb[4][2];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) bb[j][0] = b[j][0], bb[j][1] = b[j][1];
+          if (c + 4 < cend) load_p(c + 4);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (c + j >= cend) break;
+            const Frag x = get_frag(sW, c + j - c0, lane);
+            if (w < KP) mma_tiles<PR, 2>(o[0], oe[0], x, bb[j]);
+            else if (w < C::U) mma_tile<PR>(o[0][0], oe[0][0], x, bb[j][0]);
+          }
+        }
+        continue;
       }
       group_sync<GW>(grp);  // the round's values ready
 #pragma unroll 2
@@ -761,12 +837,18 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           }
         }
       });
-    auto update_p = [&](auto M, int u, const float (&x)[2][4]) {
+    auto update_p = [&](auto M, int u, int i, const float (&x)[2][4]) {
       using Un = Unit<decltype(M)::value>;
       using T = typename Un::T;
       const int n = Un::node(u, t);
-      const T ra = Un::template load<Np, V>(Ra, n), rb = Un::template load<Np, V>(Rb, n);
-      T pa, pb, fa, fb;
+      T pa, pb, fa, fb, sa, sb;
+      if constexpr (!C::EARLY) {
+        sa = Un::template load<Np, V>(Ra, n), sb = Un::template load<Np, V>(Rb, n);
+      } else if constexpr (decltype(M)::value == 2) {
+        sa = ra[i], sb = rb[i];
+      } else {
+        sa = lo2(ra[i]), sb = lo2(rb[i]);
+      }
       if constexpr (!C::KEEP) {
         pa = Un::template load<Np, V>(Qs + ea, n), pb = Un::template load<Np, V>(Qs + eb, n);
       } else if constexpr (decltype(M)::value == 2) {
@@ -780,12 +862,12 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
         fa = make_float2(x[0][0], x[0][1]), fb = make_float2(x[0][2], x[0][3]);
       }
       T y, q;
-      Un::lsrk(ra, fa, pa, P, y, q);
+      Un::lsrk(sa, fa, pa, P, y, q);
       if (va) {
         Un::template store<Np, V>(Ra, n, y);
         Un::template store<Np, V>(Oa, n, q);
       }
-      Un::lsrk(rb, fb, pb, P, y, q);
+      Un::lsrk(sb, fb, pb, P, y, q);
       if (vb) {
         Un::template store<Np, V>(Rb, n, y);
         Un::template store<Np, V>(Ob, n, q);
@@ -795,9 +877,9 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
     for (int i = 0; i < UW; ++i) {
       const int u = w + i * GW;
       if (u < KP) {
-        if constexpr (KP > 0) update_p(std::integral_constant<int, 2>(), u, o[i]);
+        if constexpr (KP > 0) update_p(std::integral_constant<int, 2>(), u, i, o[i]);
       } else if (u < C::U) {
-        if constexpr (KT > 0) update_p(std::integral_constant<int, 1>(), u, o[i]);
+        if constexpr (KT > 0) update_p(std::integral_constant<int, 1>(), u, i, o[i]);
       }
     }
   }
