@@ -63,6 +63,7 @@ void release(bbw_ctx *c) {
   cudaFree(c->fgeo);
   cudaFree(c->c2q);
   cudaFree(c->ops);
+  cudaFree(c->ops_narrow);
   cudaFree(c->nbr);
   cudaFree(c->tables);
   cudaFree(c->d_time);
@@ -241,6 +242,23 @@ bbw_status compress_connectivity(int N, int K, const int *Fmask, const int *vmap
 
 }  // namespace
 
+// the fused stage's plan and packed operators with W warps and E-element tiles
+static bbw_status make_variant(bbw_ctx *c, int W, int E, int want_ops, int want_pipe,
+                               FusedPlan &p, float **ops_buf) {
+  FusedOps fo;
+  pack_fused_ops(c->N, c->Nq, fused_groups(W, E), c->variant == BBW_BB, c->hD[0].data(), c->hD[1].data(),
+                 c->hD[2].data(), c->hLIFT.data(), c->hVq.data(), c->hPq.data(), fo);
+  bbw_status s = upload(ops_buf, fo.ops.data(), fo.ops.size(), "fused stage: operators");
+  if (s != BBW_OK) return s;
+  p = c->plan;
+  p.W = W, p.E = E;
+  p.ops = *ops_buf, p.ops_floats = (int)fo.ops.size();
+  p.off_lift = fo.off_lift, p.off_pq = fo.off_pq, p.off_vq = fo.off_vq;
+  p.RQ = fo.RQ, p.PRQ = fo.PRQ;
+  p.want_ops = want_ops, p.want_pipe = want_pipe;
+  return fused_prepare(p);
+}
+
 extern "C" bbw_status bbw_create(const bbw_mesh_desc *m, const bbw_ops_desc *o, int variant,
                                  int bc, bbw_ctx **out) {
   return bbw_create_ex(m, o, variant, bc, BBW_PREC_FP32, out);
@@ -403,6 +421,14 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
     return s;
   }
   c->precision = precision;
+  if (precision == BBW_PREC_FP32 && N <= 3 &&
+      (s = make_variant(c, bb && N == 3 ? 16 : 8, 16, 1, 0, c->narrow, &c->ops_narrow)) != BBW_OK) {
+    if (s != BBW_ERR_UNSUPPORTED) {
+      release(c);
+      return s;
+    }
+    c->narrow.W = 0;  // does not fit with a large cubature
+  }
   if (gemm) {
     c->gs = new GemmStage;
     if ((s = gemm_stage_create(*c->gs, N, K, Nq, bc, precision, c->hD, c->hLIFT, c->hVq,
@@ -548,6 +574,14 @@ static void drop_graphs(bbw_ctx *c) {
   }
 }
 
+// At N <= 3 16-element tiles halve a tile's chain of rows per thread; they pay
+// while every SM has at most one.  us per stage, 32 / 16 elements: N = 1, K =
+// 2058: 5.4 / 4.9; N = 2: 7.4 / 6.2; N = 3: 10.2 / 7.8, BB 13.5 / 9.3; N = 3, K =
+// 3072: 10.3 / 10.7.  The results are the same bit for bit.
+static bool narrow_tiles(const bbw_ctx *c) {
+  return c->narrow.W > 0 && (long long)c->S * ((c->K + 15) / 16) <= c->plan.nsm;
+}
+
 bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
                         float fdt, float cstage, cudaStream_t st, int K0, int Kc) {
   const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, (long long)c->S * c->K);
@@ -561,6 +595,13 @@ bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, f
   if (c->precision != BBW_PREC_FP32)
     return tc_launch(c->tc, Qin, Qout, res, fa, fb, fdt, cstage, st);
   FusedPlan p = c->plan;
+  if (!c->cta_form && narrow_tiles(c)) {
+    const FusedPlan &v = c->narrow;
+    p.W = v.W, p.E = v.E, p.RQ = v.RQ, p.PRQ = v.PRQ;
+    p.ops = v.ops, p.ops_floats = v.ops_floats, p.ops_smem = v.ops_smem;
+    p.off_lift = v.off_lift, p.off_pq = v.off_pq, p.off_vq = v.off_vq;
+    p.pipe = v.pipe, p.smem = v.smem;
+  }
   p.K0 = K0;
   if (Kc > 0) p.Kc = Kc;
   return fused_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
@@ -665,22 +706,6 @@ extern "C" bbw_status bbw_steps(bbw_ctx *c, float dt, int nsteps) {
 // plan of the fused stage with W warps, E-element tiles and the requested
 // placement; the packed operators are uploaded to *ops_buf (owned by the
 // caller)
-static bbw_status make_variant(bbw_ctx *c, int W, int E, int want_ops, int want_pipe,
-                               FusedPlan &p, float **ops_buf) {
-  FusedOps fo;
-  pack_fused_ops(c->N, c->Nq, fused_groups(W, E), c->variant == BBW_BB, c->hD[0].data(), c->hD[1].data(),
-                 c->hD[2].data(), c->hLIFT.data(), c->hVq.data(), c->hPq.data(), fo);
-  bbw_status s = upload(ops_buf, fo.ops.data(), fo.ops.size(), "fused stage: operators");
-  if (s != BBW_OK) return s;
-  p = c->plan;
-  p.W = W, p.E = E;
-  p.ops = *ops_buf, p.ops_floats = (int)fo.ops.size();
-  p.off_lift = fo.off_lift, p.off_pq = fo.off_pq, p.off_vq = fo.off_vq;
-  p.RQ = fo.RQ, p.PRQ = fo.PRQ;
-  p.want_ops = want_ops, p.want_pipe = want_pipe;
-  return fused_prepare(p);
-}
-
 static int config_code(const FusedPlan &p) {
   return p.W | (p.ops_smem > 0 ? 1 << 8 : 0) | (p.pipe ? 1 << 9 : 0) | (p.E == 16 ? 1 << 10 : 0);
 }

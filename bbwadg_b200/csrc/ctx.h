@@ -72,6 +72,8 @@ struct bbw_ctx {
   float *vgeo = nullptr, *fgeo = nullptr, *c2q = nullptr, *ops = nullptr;
   int *nbr = nullptr, *tables = nullptr;
   bbw::FusedPlan plan;
+  bbw::FusedPlan narrow;    // fused stage on 16-element tiles (W = 0: none), few elements
+  float *ops_narrow = nullptr;
   int precision = BBW_PREC_FP32;
   int S = 1;  // shots
   double *d_time = nullptr;
