@@ -583,11 +583,12 @@ static bool narrow_tiles(const bbw_ctx *c) {
 }
 
 bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
-                        float fdt, float cstage, cudaStream_t st, int K0, int Kc) {
+                        float fdt, float cstage, cudaStream_t st, int K0, int Kc, bool chained) {
   const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, (long long)c->S * c->K);
   if (form != WARP_AUTO) {
     WarpPlan p = c->wp;
     p.S = c->S, p.K0 = K0, p.Kc = Kc > 0 ? Kc : c->plan.Kc, p.max_ctas = c->plan.max_ctas;
+    p.chained = chained;
     p.src_tile = c->src_tile, p.src_elem = c->src_elem, p.src_vec = c->src_vec;
     p.f0 = c->plan.f0, p.tR = c->plan.tR, p.samp = c->plan.samp;
     return warp_launch(p, form, Qin, Qout, res, fa, fb, fdt, cstage, st);
@@ -602,7 +603,7 @@ bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, f
     p.off_lift = v.off_lift, p.off_pq = v.off_pq, p.off_vq = v.off_vq;
     p.pipe = v.pipe, p.smem = v.smem;
   }
-  p.K0 = K0;
+  p.K0 = K0, p.chained = chained;
   if (Kc > 0) p.Kc = Kc;
   return fused_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
 }
@@ -622,19 +623,25 @@ bbw_status launch_tape_stage(bbw_ctx *c, const float *Qin, float *Qout, float *r
   return fused_launch(p, Qin, Qout, res, fa, fb, fdt, cstage, st);
 }
 
-extern "C" bbw_status bbw_stage_ex(bbw_ctx *c, float fa, float fb, float fdt, float cstage) {
-  DeviceGuard dg(c ? c->device : -1);
-  if (!c) return set_error(BBW_ERR_ARG, "bbw_stage: ctx is NULL");
+// chained: the launch before it in the stream is this context's previous stage
+static bbw_status one_stage(bbw_ctx *c, float fa, float fb, float fdt, float cstage, bool chained) {
   bbw_status s;
   if (c->gs) {
     const GemmInputs in = {c->vgeo, c->fgeo, c->c2q, c->nbr, c->tables, c->plan.pat_off};
     s = gemm_stage_launch(*c->gs, in, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt,
                           c->stream);
   } else {
-    s = launch_stage(c, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, cstage, c->stream);
+    s = launch_stage(c, c->Q[c->cur], c->Q[c->cur ^ 1], c->res, fa, fb, fdt, cstage, c->stream, 0, 0,
+                     chained);
   }
   if (s == BBW_OK) c->cur ^= 1;
   return s;
+}
+
+extern "C" bbw_status bbw_stage_ex(bbw_ctx *c, float fa, float fb, float fdt, float cstage) {
+  DeviceGuard dg(c ? c->device : -1);
+  if (!c) return set_error(BBW_ERR_ARG, "bbw_stage: ctx is NULL");
+  return one_stage(c, fa, fb, fdt, cstage, false);
 }
 
 extern "C" bbw_status bbw_stage(bbw_ctx *c, float fa, float fb, float fdt) {
@@ -655,7 +662,7 @@ static bbw_status one_step(bbw_ctx *c, float dt, bool tape, float *vq, size_t vq
                             vq ? vq + (size_t)i * vqn : nullptr);
       if (s == BBW_OK) c->cur ^= 1;
     } else {
-      s = bbw_stage_ex(c, fa, fb, dt, cs);
+      s = one_stage(c, fa, fb, dt, cs, i > 0);
     }
     if (s != BBW_OK) return s;
   }

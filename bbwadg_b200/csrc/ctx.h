@@ -110,7 +110,8 @@ struct bbw_ctx {
 // tensor-core or FP32 fused): elements [K0, Kc) (Kc = 0: the context's compute
 // range) of all shots
 bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
-                        float fdt, float cstage, cudaStream_t st, int K0 = 0, int Kc = 0);
+                        float fdt, float cstage, cudaStream_t st, int K0 = 0, int Kc = 0,
+                        bool chained = false);
 // one stage of the adjoint's forward pass and recomputation: the FP32 fused or
 // tensor-core stage, whose rounding the FP64 gradient is pinned to.  vq_out:
 // store the pre-c^2 cubature values ([S][Nq][K]); time: the clock the sources

@@ -31,6 +31,7 @@ struct FusedPlan {
   int table_ints = 0, pat_off = 0, bb_off = 0;
   int S = 1, nsm = 148;  // shots per launch, SM count
   int max_ctas = 0;      // cap on the persistent grid (0: one CTA per SM)
+  bool chained = false;  // launched right behind another stage kernel
   const int *src_off = nullptr, *src_elem = nullptr;  // sources (null: none)
   const float *src_vec = nullptr;
   float f0 = 0.f, tR = 0.f, samp = 0.f;

@@ -266,10 +266,10 @@ __global__ void __launch_bounds__(FusedCfg<N, W_, E_>::T, 1) k_fused_stage(Fused
         if (pat != 255 && rel >= (unsigned)ne_b) {  // neighbours inside the tile: from smem
           const float *q2 = P.Qin + shot * sstride + (size_t)(code >> 8) * 4 * Np +
                             sPat[pat * Nfp + (m - f * Nfp)];
-          nb[j][0] = __ldg(q2);
-          nb[j][1] = __ldg(q2 + Np);
-          nb[j][2] = __ldg(q2 + 2 * Np);
-          nb[j][3] = __ldg(q2 + 3 * Np);
+          nb[j][0] = q2[0];
+          nb[j][1] = q2[Np];
+          nb[j][2] = q2[2 * Np];
+          nb[j][3] = q2[3 * Np];
         }
       }
     }
@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(FusedCfg<N, W_, E_>::T, 1) k_fused_stage(Fused
   const int nvt = P.S * ntiles;  // (shot, tile) work items
   int vt = blockIdx.x, b = 0;
   float nb[FIT][4];
+  stage_wait();
   __syncthreads();  // tables staged
   if (vt < nvt) {
     issue_tile(vt, sIn, IN_ALL);
@@ -639,7 +640,7 @@ __global__ void __launch_bounds__(FusedCfg<N, W_, E_>::T, 1) k_fused_stage(Fused
 #pragma unroll
         for (int j = 0; j < UIT; ++j) {
           const int i = tid + j * T;
-          qold[PIPE ? 0 : j] = i < ne * 4 * Np ? __ldg(qin + i) : 0.f;
+          qold[PIPE ? 0 : j] = i < ne * 4 * Np ? qin[i] : 0.f;
         }
       }
 #pragma unroll
@@ -710,16 +711,16 @@ static bbw_status launch_fused(const FusedPlan &pl, const float *Qin, float *Qou
   }
   if (pl.W == 8) {
     constexpr int T = 256;
-    if (os && pl.pipe) k_fused_stage<N, BB, true, true, 8, E><<<grid, T, sm, st>>>(P);
-    else if (os) k_fused_stage<N, BB, true, false, 8, E><<<grid, T, sm, st>>>(P);
-    else if (pl.pipe) k_fused_stage<N, BB, false, true, 8, E><<<grid, T, sm, st>>>(P);
-    else k_fused_stage<N, BB, false, false, 8, E><<<grid, T, sm, st>>>(P);
+    if (os && pl.pipe) launch_stage_kernel(k_fused_stage<N, BB, true, true, 8, E>, grid, T, sm, st, pl.chained, P);
+    else if (os) launch_stage_kernel(k_fused_stage<N, BB, true, false, 8, E>, grid, T, sm, st, pl.chained, P);
+    else if (pl.pipe) launch_stage_kernel(k_fused_stage<N, BB, false, true, 8, E>, grid, T, sm, st, pl.chained, P);
+    else launch_stage_kernel(k_fused_stage<N, BB, false, false, 8, E>, grid, T, sm, st, pl.chained, P);
   } else {
     constexpr int T = 512;
-    if (os && pl.pipe) k_fused_stage<N, BB, true, true, 16, E><<<grid, T, sm, st>>>(P);
-    else if (os) k_fused_stage<N, BB, true, false, 16, E><<<grid, T, sm, st>>>(P);
-    else if (pl.pipe) k_fused_stage<N, BB, false, true, 16, E><<<grid, T, sm, st>>>(P);
-    else k_fused_stage<N, BB, false, false, 16, E><<<grid, T, sm, st>>>(P);
+    if (os && pl.pipe) launch_stage_kernel(k_fused_stage<N, BB, true, true, 16, E>, grid, T, sm, st, pl.chained, P);
+    else if (os) launch_stage_kernel(k_fused_stage<N, BB, true, false, 16, E>, grid, T, sm, st, pl.chained, P);
+    else if (pl.pipe) launch_stage_kernel(k_fused_stage<N, BB, false, true, 16, E>, grid, T, sm, st, pl.chained, P);
+    else launch_stage_kernel(k_fused_stage<N, BB, false, false, 16, E>, grid, T, sm, st, pl.chained, P);
   }
   return check_launch("fused stage");
 }

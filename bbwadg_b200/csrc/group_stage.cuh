@@ -60,7 +60,7 @@ struct GroupCfg {
 // Gather of face f of eight elements h8 .. h8 + 7 of the tile, nodes I0 .. I0 +
 // NI - 1: EPI elements per pass, lane = (element, node), so a pass reads the
 // face nodes of a neighbour's row together.
-template <int N, int I0, int NI>
+template <int N, int I0, int NI, bool CHAINED>
 struct TileFace {
   using C = GroupCfg<N>;
   static constexpr int EPI = NI >= 32 ? 1 : (32 / NI > 8 ? 8 : 32 / NI);
@@ -92,7 +92,7 @@ struct TileFace {
       const int nn = sTab[(wall ? f * C::Nfp : pat_off + pat * C::Nfp) + i];
       const float *x = Qs + (size_t)(cd >> 8) * C::EW + nn;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) X[it][c] = __ldg(x + c * C::Np);
+      for (int c = 0; c < 4; ++c) X[it][c] = load_trace<CHAINED>(x + c * C::Np);
     }
   }
   // upwind pressure flux to sF[element][8 FB].  A wall's + trace is the own
@@ -123,20 +123,20 @@ struct TileFace {
   }
 };
 
-template <int N, bool WIDE>
+template <int N, bool CHAINED, bool WIDE>
 struct TileHalf;
-template <int N>
-struct TileHalf<N, false> {
-  TileFace<N, 0, NFP(N)> a;
+template <int N, bool CHAINED>
+struct TileHalf<N, CHAINED, false> {
+  TileFace<N, 0, NFP(N), CHAINED> a;
   template <class... A>
   __device__ __forceinline__ void load(A... x) { a.load(x...); }
   template <class... A>
   __device__ __forceinline__ void flux(A... x) const { a.flux(x...); }
 };
-template <int N>
-struct TileHalf<N, true> {  // more than 32 nodes per face
-  TileFace<N, 0, 32> a;
-  TileFace<N, 32, (NFP(N) > 32 ? NFP(N) - 32 : 1)> b;
+template <int N, bool CHAINED>
+struct TileHalf<N, CHAINED, true> {  // more than 32 nodes per face
+  TileFace<N, 0, 32, CHAINED> a;
+  TileFace<N, 32, (NFP(N) > 32 ? NFP(N) - 32 : 1), CHAINED> b;
   template <class... A>
   __device__ __forceinline__ void load(A... x) { a.load(x...), b.load(x...); }
   template <class... A>
@@ -270,10 +270,11 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
   int it = blockIdx.x * P.bs + grp * P.ws;
   int code0 = 0, code1 = 0;
   int nshot = it / P.ntile, ntl = it - nshot * P.ntile;  // the next item
-  if (it < P.nit) {
-    fetch_tile(nshot, P.K0 + ntl * 16);
-    codes(P.K0 + ntl * 16, code0, code1);
-  }
+  if (it < P.nit) codes(P.K0 + ntl * 16, code0, code1);
+  // operators from L2 leave nothing to stage early, and the gather's read-only
+  // path is worth more (N = 7: 178 against 182 us per stage chained)
+  if constexpr (OPS) stage_wait();
+  if (it < P.nit) fetch_tile(nshot, P.K0 + ntl * 16);
   cp_async_wait();
   __syncthreads();
   for (; it < P.nit; it += step) {
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
     // ---- 1. face fluxes, eight elements of one face at a time, and the
     //         maxima of the warp's own nodes
     {
-      TileHalf<N, (Nfp > 32)> x;
+      TileHalf<N, OPS, (Nfp > 32)> x;
       x.load(Qs, sTab, P.pat_off, w >> 1, w & 1 ? code1 : code0, lane);
       cp_async_wait();
       group_sync<GW>(grp);  // the tile has landed
@@ -902,13 +903,13 @@ static bbw_status group_launch_n(const WarpPlan &pl, const float *Qin, float *Qo
   const size_t sm = group_smem<N>(pl, os);
   if constexpr (C::OPS) {
     if (os) {
-      if (pl.products == 4) k_group_stage<N, 4, true><<<grid, C::T, sm, st>>>(P);
-      else k_group_stage<N, 3, true><<<grid, C::T, sm, st>>>(P);
+      if (pl.products == 4) launch_stage_kernel(k_group_stage<N, 4, true>, grid, C::T, sm, st, pl.chained, P);
+      else launch_stage_kernel(k_group_stage<N, 3, true>, grid, C::T, sm, st, pl.chained, P);
       return check_launch("group-matrix stage");
     }
   }
-  if (pl.products == 4) k_group_stage<N, 4, false><<<grid, C::T, sm, st>>>(P);
-  else k_group_stage<N, 3, false><<<grid, C::T, sm, st>>>(P);
+  if (pl.products == 4) launch_stage_kernel(k_group_stage<N, 4, false>, grid, C::T, sm, st, false, P);
+  else launch_stage_kernel(k_group_stage<N, 3, false>, grid, C::T, sm, st, false, P);
   return check_launch("group-matrix stage");
 }
 

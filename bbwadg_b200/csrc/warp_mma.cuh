@@ -247,6 +247,16 @@ __device__ __forceinline__ void store2(float *x, int n, const float2 v) {
   }
 }
 
+// A value of a neighbour's state.  CHAINED: by the coherent path, as the stage
+// before may still run when this kernel starts; not volatile, so that loads
+// schedule freely: the address comes from a table that is read after stage_wait.
+template <bool CHAINED>
+__device__ __forceinline__ float load_trace(const float *x) {
+  if constexpr (!CHAINED) return __ldg(x);
+  float v;
+  asm("ld.global.f32 %0, [%1];\n" : "=f"(v) : "l"(x));
+  return v;
+}
 __device__ __forceinline__ void cp_async16(uint32_t dst, const float *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
 }

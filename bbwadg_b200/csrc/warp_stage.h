@@ -19,6 +19,7 @@ struct WarpPlan {
   bool warp_ops = false, group_ops = false;  // operators staged in shared memory
   int products = 4;      // products per split pair (4: FP32 contexts, 3: split FP16)
   int N = 0, K = 0, K0 = 0, Kc = 0, Nq = 0, bc = 0, S = 1, nsm = 148, max_ctas = 0;
+  bool chained = false;  // launched right behind another stage kernel
   int pat_off = 0, table_ints = 0;
   int oDt = 0, oL = 0, oLt = 0, oV = 0, oVt = 0, oP = 0, ops_n = 0;
   float iD = 1.f, iL = 1.f, iV = 1.f, iP = 1.f, vnorm = 1.f;
