@@ -7,7 +7,7 @@
 // 8-shot N = 4 workload on 24 576 elements takes 90 GB), which is all the
 // reverse sweep needs, or the state at every `checkpoint_every`-th step
 // start, from which bbw_backward recomputes each segment forward once with
-// the same stage kernel.  The stages are reversed with the adjoint kernels
+// the same stage kernel (launch_tape_stage).  The stages are reversed with the adjoint kernels
 // of kernels_adj.cu.  The c^2 gradient is accumulated in
 // FP64.  There is no reference counterpart; the forward operators are the
 // reference's rk_volume / rk_surface / rk_update_WADG

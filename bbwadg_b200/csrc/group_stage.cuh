@@ -10,9 +10,9 @@
 // chain is three to eight times shorter, which counts where a mesh has few tiles
 // or an element much work.  The results are the same bit for bit.  us per
 // stage, CTA-wide FP32 stage / one warp / group: N = 5, K = 3072: 23.8 / 24.6 /
-// 13.5, K = 196608: 879 / 422 / 418; N = 7, K = 24576: 706 / 327 / 173; N = 4, K =
-// 3072: 16.8 / 18.2 / 13.1.  Bound by instruction and L1 wavefront rate together
-// (issue 31 %, L1 data pipe 56 %, tensor 28 %); without the products 261 us,
+// 13.6, K = 196608: 879 / 422 / 411; N = 7, K = 24576: 706 / 327 / 178; N = 4, K =
+// 3072: 16.8 / 18.2 / 12.7.  Bound by instruction and L1 wavefront rate together
+// (issue 34 %, L1 data pipe 58 %, tensor 28 %); without the products 261 us,
 // without global loads 399, without stores 325 (N = 5, K = 196608).
 #pragma once
 #include <vector>
@@ -31,7 +31,7 @@ struct GroupCfg {
   // a unit of work is a pair of blocks (or the odd last one); GW warps per
   // group, NG groups per CTA.  us per stage at K = 24576 with three or four
   // warps and two units each, 168 registers / one unit per warp: N = 6 145 / 123,
-  // N = 7 254 / 173 (one group of 255 registers; two of 128: 205).
+  // N = 7 254 / 178 (one group of 255 registers; two of 128: 205).
   static constexpr int U = KP + KT;
   static constexpr int GW = U;  // 3, 4, 6, 8 at N = 4 .. 7
   static constexpr int NG = N <= 6 ? 12 / GW : 1;

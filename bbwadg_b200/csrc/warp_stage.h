@@ -56,12 +56,12 @@ bbw_status warp_prepare(WarpPlan &pl);
 // The form for `elements` (mesh elements times shots) when none is pinned;
 // WARP_AUTO: the CTA-wide stages.  The forms give the same results bit for
 // bit.  us per stage, CTA-wide FP32 / one warp / group:
-//   N = 2  K = 1296: 7.4 / 9.9 / -      K = 6000: 12.0 / 10.2 / -
-//   N = 3  K = 3072: 10.2 / 11.5 / -    K = 6000: 17.2 / 11.5 / -
-//   N = 4  K = 3072: 16.8 / 18.2 / 13.5 K = 10368: 43.4 / 23.0 / 34.5
-//   N = 5  K = 384: 23.3 / 24.4 / 11.5  K = 196608: 879 / 422 / 414
-//   N = 6  K = 384: 73 / 45 / 29        K = 24576: 454 / 154 / 143
-//   N = 7  K = 384: 112 / 80 / 34       K = 24576: 706 / 327 / 257
+//   N = 2  K = 1296: 5.4 / 9.4 / -      K = 6000: 12.0 / 9.4 / -
+//   N = 3  K = 3072: 9.4 / 10.7 / -     K = 6000: 17.2 / 10.7 / -
+//   N = 4  K = 3072: 16.8 / 17.6 / 12.7 K = 10368: 43.4 / 22.3 / 34.1
+//   N = 5  K = 384: 23.3 / 24.4 / 10.6  K = 196608: 879 / 422 / 411
+//   N = 6  K = 384: 73 / 45 / 17        K = 24576: 454 / 154 / 123
+//   N = 7  K = 384: 112 / 80 / 17       K = 24576: 706 / 327 / 178
 // One warp per tile pays once there are about two tiles per SM; the group
 // form, three tiles or more per SM at a time, up to the 592 tiles of its first
 // wave at N = 4, and at every size above.

@@ -12,11 +12,11 @@ rule), [-1,1]^3 split into 32^3 hexes x 6 tets, c^2 = 1 + 0.5 sin sin sin +
 The state (3 x 176 MB) exceeds the 126 MB L2, so no flush is needed between
 steps.
 
-The headline form is the tensor-core stage (nodal-f16x3): FP32 state, the
-dense contractions on tcgen05 as three FP16 products per split pair with
-FP32 accumulation.  Its error against the FP64 restatement is the FP32
+The headline form is the split-FP16 stage (nodal-f16x3): FP32 state, the
+dense contractions on the tensor cores as three FP16 products per split pair
+with FP32 accumulation.  Its error against the FP64 restatement is the FP32
 stage's (the line's `precision` object gives both, measured in the same
-run); the FP32 CUDA-core stage and the BB stage run beside it
+run); the FP32 stage and the BB stage run beside it
 (`side_by_side`).
 
 * value      device-timed throughput of the fused stage kernels, inputs
@@ -416,7 +416,7 @@ def precision_workload(args, torch):
                 err, rel = p.l2_error(Q, nsteps * dt, cavity_mode)
                 row = {"N": N, "n": nh, "K": p.K, "precision": prec, "steps": nsteps,
                        "form": ("fused FP32" if prec == "fp32" else
-                                "tensor-core stage" if (N <= 5 and prec != "tf32") else
+                                "split stage" if (N <= 5 and prec != "tf32") else
                                 "GEMM precision form"),
                        "rel_l2_vs_exact": rel, "ms_per_step": 1e3 * el / nsteps}
                 if nh == 8:
@@ -748,8 +748,9 @@ def main():
                                             autotuned=head["tuned"]),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
-                     "kernel": ("k_tc_stage<%d>" % N_ORDER) if args.variant.endswith("f16x3")
-                     else "k_fused_stage<%d,%s>" % (N_ORDER, args.variant == "bb"),
+                     "kernel": "k_fused_stage<%d,%s>" % (N_ORDER, args.variant == "bb")
+                     if head["tuned"] and head["tuned"]["warps"] >= 8
+                     else "k_group_stage<%d>" % N_ORDER,
                      "peak_kind": peak_kind},
         "e2e": {"value": world * head["dofs"] / head["e2e_s"], "unit": "DOF-stage/s",
                 "h2d_bytes_per_step": head["state_bytes"] / args.steps,

@@ -237,17 +237,22 @@ typedef struct bbw_ops_desc {
   const float *Vq, *Pq;
 } bbw_ops_desc;
 
-/* Arithmetic of the fused stage.  FP32: CUDA-core FP32 throughout.
- * F16X3: the dense contractions (Dr/Ds/Dt, LIFT, Vq, Pq) on the tensor cores
- * as three FP16 products per split pair (A_hi x_hi + A_hi x_lo + A_lo x_hi,
- * per-tile power-of-two scaling, FP32 accumulation); state, fluxes and the
- * update stay FP32.  BF16X3: the same with BF16 pairs (16 significant bits
- * per pair instead of 22; the split-BF16 form of the precision study).  Both
+/* Arithmetic of the fused stage.  FP32: FP32 state, fluxes, sums and update,
+ * FP32-class error; at N <= 7 larger meshes run the dense contractions
+ * (Dr/Ds/Dt, LIFT, Vq, Pq) on warp-level matrix instructions, every FP32 value
+ * as an FP16 pair of 23 bits with a power-of-two scale per element and all four
+ * products (FP32 accumulation), smaller ones and N = 8 on the CUDA cores; the
+ * two agree to rounding.
+ * F16X3: the contractions as three FP16 products per split pair (A_hi x_hi +
+ * A_hi x_lo + A_lo x_hi, power-of-two scaling, FP32 accumulation); state, fluxes
+ * and the update stay FP32.  BF16X3: the same with BF16 pairs (16 significant
+ * bits per pair instead of 22; the split-BF16 form of the precision study).  Both
  * run N in [2, 5] (Np <= 64: each operator's rows fit one M = 64 MMA and all
  * operators one SM's shared memory), Nq <= 128, batched shots and sources,
  * nodal or BB (BB: the dense equivalents of the sparse BB derivative and
  * lift applied to BB coefficients), and the adjoint (its forward and
- * recomputation run the same stage). */
+ * recomputation run the CUDA-core or the tcgen05 stage, which agree with the
+ * time loop's to rounding). */
 enum { BBW_PREC_FP32 = 0, BBW_PREC_F16X3 = 1, BBW_PREC_BF16X3 = 2, BBW_PREC_TF32 = 3 };
 /* Precision-study form: F16X3 and BF16X3 at orders the fused tensor-core
  * stage does not take (N >= 6, or Nq > 128), and TF32 at every order, run
@@ -296,7 +301,9 @@ bbw_status bbw_run(bbw_ctx *ctx, double final_time, float dt);
  * rows per thread group ceil(Np / (32 W / E)); operators in shared or global
  * memory; single or double-buffered input tiles), `stages` launches each on
  * scratch copies of the state, and keeps the fastest.  *config (may be NULL)
- * = W | ops_in_smem << 8 | pipelined << 9 | (E == 16) << 10.
+ * = W | ops_in_smem << 8 | pipelined << 9 | (E == 16) << 10, or, with the
+ * other bits 8, ops_in_smem and E == 16, the warp-matrix stages: 1 << 11 (one
+ * warp per 16-element tile, N <= 4), 1 << 12 (a group of warps, N = 4 .. 7).
  * The state is not modified.  No-op for the tensor-core stage.  The
  * reference's counterpart is its hand-swept KblkV/KblkS/KblkU block sizes
  * (cpp/src/WaveOKL3d.cpp:1618-1650, cpp/profileKernels). */
@@ -475,8 +482,9 @@ typedef struct bbw_tape bbw_tape;
 /* Replaces c^2 / J at the cubature points ([K][Nq], host). */
 bbw_status bbw_set_c2q(bbw_ctx *ctx, const float *c2q);
 
-/* Advances nsteps steps of dt exactly as bbw_steps does (receivers must be
- * set; traces land at the current step count onwards) and returns a tape
+/* Advances nsteps steps of dt as bbw_steps does, on the CUDA-core or tcgen05
+ * stage whose rounding the FP64 gradient is pinned to (the time loop's stage
+ * agrees with it to FP32 rounding; receivers must be set; traces land at the current step count onwards) and returns a tape
  * for bbw_backward: bbw_forward_ex with BBW_TAPE_CUBATURE (every stage's
  * cubature values when they fit, else the state at every
  * checkpoint_every-th step start).  No counterpart in the reference. */
