@@ -54,8 +54,9 @@ void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<floa
 // Sets the forms that fit (pl.single, pl.group).
 bbw_status warp_prepare(WarpPlan &pl);
 // The form for `elements` (mesh elements times shots) when none is pinned;
-// WARP_AUTO: the CTA-wide stages.  The forms give the same results bit for
-// bit.  us per stage, CTA-wide FP32 / one warp / group:
+// WARP_AUTO: the CTA-wide stages.  One warp and group give the same results
+// bit for bit, the CTA-wide stages the same to FP32 rounding.  us per stage,
+// CTA-wide FP32 / one warp / group:
 //   N = 2  K = 1296: 5.4 / 9.4 / -      K = 6000: 12.0 / 9.4 / -
 //   N = 3  K = 3072: 9.4 / 10.7 / -     K = 6000: 17.2 / 10.7 / -
 //   N = 4  K = 3072: 16.8 / 17.6 / 12.7 K = 10368: 43.4 / 22.3 / 34.1
