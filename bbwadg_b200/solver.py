@@ -47,29 +47,29 @@ def _i32(a):
     return np.ascontiguousarray(a, np.int32)
 
 
-# the warp-matrix stages' codes by warps per tile (4 stands for a group of any size)
-_MATRIX_CODES = {1: 8 | 1 << 8 | 1 << 10 | 1 << 11, 4: 8 | 1 << 8 | 1 << 10 | 1 << 12}
+# the warp-matrix stages' codes, by the name their `pipelined` field takes: one
+# warp or a group of warps per 16-element tile
+_MATRIX_CODES = {"warp": 8 | 1 << 8 | 1 << 10 | 1 << 11, "group": 8 | 1 << 8 | 1 << 10 | 1 << 12}
 
 
 def encode_config(warps, ops_in_smem, pipelined, tile=32):
-    """Configuration code of a stage variant (bbw_set_config): warps 8 or 16
-    per CTA, or 1 / 4 (one warp / a group of warps per tile of 16, operators in
-    shared memory, not pipelined) for the warp-matrix stages."""
+    """Configuration code of a stage variant (bbw_set_config); pipelined is a
+    flag, or "warp" / "group" for the warp-matrix stages (the rest as
+    decode_config gives it)."""
     if tile not in (16, 32):
         raise ValueError("tile must be 16 or 32")
-    if warps in _MATRIX_CODES and ops_in_smem and not pipelined and tile == 16:
-        return _MATRIX_CODES[warps]
+    if isinstance(pipelined, str):
+        return _MATRIX_CODES[pipelined]
     return (int(warps) | (int(bool(ops_in_smem)) << 8) | (int(bool(pipelined)) << 9)
             | (int(tile == 16) << 10))
 
 
 def decode_config(code):
     """Fields of a configuration code as bbw_autotune returns it."""
-    for warps, matrix in _MATRIX_CODES.items():
-        if code == matrix:
-            return dict(warps=warps, ops_in_smem=True, pipelined=False, tile=16, code=code)
+    form = [k for k, v in _MATRIX_CODES.items() if v == code]
     return dict(warps=code & 255, ops_in_smem=bool(code >> 8 & 1),
-                pipelined=bool(code >> 9 & 1), tile=16 if code >> 10 & 1 else 32, code=code)
+                pipelined=form[0] if form else bool(code >> 9 & 1),
+                tile=16 if code >> 10 & 1 else 32, code=code)
 
 
 class WaveSolver:

@@ -749,7 +749,7 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic,
                      "kernel": "k_fused_stage<%d,%s>" % (N_ORDER, args.variant == "bb")
-                     if head["tuned"] and head["tuned"]["warps"] >= 8
+                     if head["tuned"] and not isinstance(head["tuned"]["pipelined"], str)
                      else "k_group_stage<%d>" % N_ORDER,
                      "peak_kind": peak_kind},
         "e2e": {"value": world * head["dofs"] / head["e2e_s"], "unit": "DOF-stage/s",
