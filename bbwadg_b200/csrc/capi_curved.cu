@@ -109,7 +109,7 @@ bbw_status setup_mma(bbw_curved *h, const bbw_curved_desc *d) {
   bbw_status s = curved_mma_prepare(h->N, M);
   if (s == BBW_ERR_UNSUPPORTED) return BBW_OK;
   if (s != BBW_OK) return s;
-  std::vector<uint32_t> ops;
+  SplitOps ops;
   const size_t mq = (size_t)Nq * Np, mr = (size_t)Nr * Np;
   const float *V[4] = {d->Vq, d->Vrq, d->Vsq, d->Vtq}, *P[4] = {d->Pq, d->Prq, d->Psq, d->Ptq};
   const float sV = split_scale(V, 1, mq), sD = split_scale(V + 1, 3, mq);
@@ -135,11 +135,13 @@ bbw_status setup_mma(bbw_curved *h, const bbw_curved_desc *d) {
   M.fnorm = max_row_sum(d->VfqFace, Nfq, Nfp);
   M.dnorm = std::max(max_row_sum(d->Vrq, Nq, Np),
                      std::max(max_row_sum(d->Vsq, Nq, Np), max_row_sum(d->Vtq, Nq, Np)));
+  M.oM = (int)(ops.w.size() / 4);
+  const std::vector<uint32_t> words = ops.words();
   uint4 *dops = nullptr;
   float *gq = nullptr, *fq = nullptr, *jq = nullptr, *bound = nullptr;
   const size_t nt = M.nt;
   const float *none = nullptr;
-  if ((s = own_upload(h, &dops, reinterpret_cast<const uint4 *>(ops.data()), ops.size() / 4,
+  if ((s = own_upload(h, &dops, reinterpret_cast<const uint4 *>(words.data()), words.size() / 4,
                       "bbw_curved_create: split operators")) != BBW_OK ||
       (s = own_upload(h, &gq, none, nt * M.nch * 10 * 256, "bbw_curved_create")) != BBW_OK ||
       (s = own_upload(h, &fq, none, nt * 4 * M.FC * 4 * 256, "bbw_curved_create")) != BBW_OK ||

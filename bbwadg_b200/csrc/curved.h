@@ -36,6 +36,7 @@ struct CurvedMma {
   int oV[4] = {}, oVt[4] = {}, oP[4] = {};  // Vq Vrq Vsq Vtq, k8 tails, Pq Prq Psq Ptq
   int oF = 0, oFt = 0, oL = 0;              // VfqFace, Pfq by face and chunk
   int oVr = 0, oVrt = 0, oPr = 0;           // update's Vq, Pq
+  int oM = 0;                               // plane of the rests
   float iV = 1.f, iD = 1.f, iP = 1.f, iF = 1.f, iVr = 1.f, iPr = 1.f;  // inverse scales
   float vnorm = 1.f, dnorm = 1.f, fnorm = 1.f, rnorm = 1.f;            // row sums
   float fa = 0.f, fb = 0.f, fdt = 0.f;

@@ -6,7 +6,8 @@
 // 3024-3195, 1760-1887), as k_curved_stage (kernels_curved.cu) does with a thread
 // per output: twenty Np x Nq contractions per element, and one operator load
 // and one shared load per FMA there.  Here elements are matrix rows; operands
-// are FP16 pairs scaled per element and field (four products, the FP32 error),
+// are FP16 pairs scaled per element and field, operators pairs and a rest (the
+// FP32 error, warp_mma.cuh),
 // operator tiles come through L1 and the point values stay in registers.
 #pragma once
 #include "curved.h"
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
                  float *__restrict__ res) {
   using C = CurvedCfg<N, GWP>;
   constexpr int Np = C::Np, Nfp = C::Nfp, NB = C::NB, KP = C::KP, KT = C::KT, EW = C::EW;
-  constexpr int FP = C::FP, FT = C::FT, V = C::V, GW = C::GW, AS = C::AS, PR = 4;
+  constexpr int FP = C::FP, FT = C::FT, V = C::V, GW = C::GW, AS = C::AS, PR = 4, PD = 5;
   extern __shared__ __align__(16) float smem_f[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int grp = warp / GW, w = warp - grp * GW, g = lane >> 2, t = lane & 3;
@@ -52,8 +53,11 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
   float4 *sMax = reinterpret_cast<float4 *>(scr + C::TILE + C::WF);  // [GW][16]
   float *sInv = scr + C::TILE + C::WF + GW * 64;            // [4][16] face scales
   uint4 *sFc = reinterpret_cast<uint4 *>(sInv + 64);        // [4][FC][4] split fluxes
-  const uint4 *ops = A.ops + lane;
-  auto tail = [&](int off) { return reinterpret_cast<const uint2 *>(A.ops + off) + lane; };
+  using O16 = Ops<uint4, PR, true>;
+  using O8 = Ops<uint2, PR, true>;
+  using T16 = OpTile<uint4>;
+  auto op = [&](int off) { return O16(A.ops, A.ops + A.oM, off, lane); };
+  auto tail = [&](int off) { return O8(A.ops, A.ops + A.oM, off, lane); };
 
   for (int it = blockIdx.x * C::NG + grp; it < A.nt; it += gridDim.x * C::NG) {
     const int r0 = it * 16, rl = A.KC - 1;
@@ -136,34 +140,37 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
       }
 #pragma unroll 1
       for (int ch = 0; ch < A.FC; ++ch) {
-        float v[7][2][4] = {};
+        float v[7][2][4];
+        auto each = [&](float (&o)[7][4], const auto &x, const auto b) {
 #pragma unroll
-        for (int s = 0; s < FP; ++s) {
-          const uint4 b[2] = {__ldg(ops + A.oF + ((ch * FP + s) * 2) * 32),
-                              __ldg(ops + A.oF + ((ch * FP + s) * 2 + 1) * 32)};
-          auto each = [&](const uint32_t (Frag::*p)[4], bool lo) {
+          for (int p = 0; p < kProducts; ++p)
 #pragma unroll
-            for (int c = 0; c < 7; ++c)
+            for (int c = 0; c < 7; ++c) mma_step<PR>(o[c], x(c), b, p);
+        };
 #pragma unroll
-              for (int i = 0; i < 2; ++i) mma_hl(v[c][i], fx[c][s].*p, b[i], lo);
-          };
-          each(&Frag::l, true);
-          each(&Frag::h, true);
-          each(&Frag::l, false);
-          each(&Frag::h, false);
-        }
-        if constexpr (FT) {
-          const uint2 b[2] = {__ldg(tail(A.oFt) + (ch * 2) * 32), __ldg(tail(A.oFt) + (ch * 2 + 1) * 32)};
-          auto each = [&](const uint32_t (Frag8::*p)[2], bool lo) {
+        for (int i = 0; i < 2; ++i) {
+          float s7[7][4];
 #pragma unroll
-            for (int c = 0; c < 7; ++c)
+          for (int s = 0; s < FP; ++s) {
+            each(s7, [&](int c) { return fx[c][s]; }, op(A.oF)[((ch * FP + s) * 2 + i) * 32]);
 #pragma unroll
-              for (int i = 0; i < 2; ++i) mma_hl(v[c][i], f8[c].*p, b[i], lo);
-          };
-          each(&Frag8::l, true);
-          each(&Frag8::h, true);
-          each(&Frag8::l, false);
-          each(&Frag8::h, false);
+            for (int c = 0; c < 7; ++c) {
+              if (s > 0) add4(v[c][i], s7[c]);
+              else
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[c][i][q] = s7[c][q];
+            }
+          }
+          if constexpr (FT) {
+            each(s7, [&](int c) { return f8[c]; }, tail(A.oFt)[(ch * 2 + i) * 32]);
+#pragma unroll
+            for (int c = 0; c < 7; ++c) {
+              if (FP > 0) add4(v[c][i], s7[c]);
+              else
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[c][i][q] = s7[c][q];
+            }
+          }
         }
         // points 16 ch + 4 t + 0 .. 3: row h, point 2 i + j of the four
         float fl[4][2][4];
@@ -268,7 +275,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int h = 0; h < 2; ++h) isc[c][h] = (1.f / sc[c][h]) * (c == 0 ? A.iD : A.iV);
-      float o[4][2][4] = {}, oe[4][2][4] = {};
+      float o[4][2][4] = {};
 #pragma unroll 1
       for (int c0 = 0; c0 < A.nch; c0 += C::RC) {
         const int cend = min(A.nch, c0 + C::RC);
@@ -276,27 +283,27 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll 1
         for (int c = c0 + w; c < cend; c += GW) {
           // u, v, w with Vq; p with Vrq, Vsq, Vtq
-          float v[6][2][4] = {}, e[6][2][4] = {};
+          float v[6][2][4] = {};
 #pragma unroll
           for (int k = 0; k < KP; ++k) {
             const Frag p = get_frag(sA, k, lane);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-              const uint4 *D = ops + A.oV[1 + d] + ((c * KP + k) * 2) * 32;
-              const uint4 *Q = ops + A.oV[0] + ((c * KP + k) * 2) * 32;
-              const uint4 bd[2] = {__ldg(D), __ldg(D + 32)}, bq[2] = {__ldg(Q), __ldg(Q + 32)};
+              const O16 D = op(A.oV[1 + d]) + ((c * KP + k) * 2) * 32;
+              const O16 Q = op(A.oV[0]) + ((c * KP + k) * 2) * 32;
+              const T16 bd[2] = {D[0], D[32]}, bq[2] = {Q[0], Q[32]};
               const Frag u = get_frag(sA + (1 + d) * AS, k, lane);
-              mma_pair2<PR, 2>(v[3 + d], e[3 + d], p, bd, v[d], e[d], u, bq);
+              mma_pair2<PD, PR>(v[3 + d], p, bd, v[d], u, bq);
             }
           }
           if constexpr (KT) {
             const Frag8 p = get_frag8(sA, KP, lane);
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-              const uint2 *D = tail(A.oVt[1 + d]) + (c * 2) * 32, *Q = tail(A.oVt[0]) + (c * 2) * 32;
-              const uint2 bd[2] = {__ldg(D), __ldg(D + 32)}, bq[2] = {__ldg(Q), __ldg(Q + 32)};
+              const O8 D = tail(A.oVt[1 + d]) + (c * 2) * 32, Q = tail(A.oVt[0]) + (c * 2) * 32;
+              const OpTile<uint2> bd[2] = {D[0], D[32]}, bq[2] = {Q[0], Q[32]};
               const Frag8 u = get_frag8(sA + (1 + d) * AS, KP, lane);
-              mma_pair2<PR, 2>(v[3 + d], e[3 + d], p, bd, v[d], e[d], u, bq);
+              mma_pair2<PD, PR>(v[3 + d], p, bd, v[d], u, bq);
             }
           }
           const float *G = A.gq + ((size_t)it * A.nch + c) * 10 * 256;
@@ -314,10 +321,10 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const int i = q / 2, j = 2 * h + q % 2;
-              const float uq = (v[0][i][j] + e[0][i][j]) * isc[1][h], vq = (v[1][i][j] + e[1][i][j]) * isc[2][h],
-                          wq = (v[2][i][j] + e[2][i][j]) * isc[3][h];
-              const float dr = (v[3][i][j] + e[3][i][j]) * isc[0][h], ds = (v[4][i][j] + e[4][i][j]) * isc[0][h],
-                          dt = (v[5][i][j] + e[5][i][j]) * isc[0][h];
+              const float uq = v[0][i][j] * isc[1][h], vq = v[1][i][j] * isc[2][h],
+                          wq = v[2][i][j] * isc[3][h];
+              const float dr = v[3][i][j] * isc[0][h], ds = v[4][i][j] * isc[0][h],
+                          dt = v[5][i][j] * isc[0][h];
               const float J = G9[9][q];
 #pragma unroll
               for (int x = 0; x < 3; ++x) {
@@ -345,13 +352,13 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             const Frag x = get_frag(W + d * 64, 0, lane), y = get_frag(W + (3 + d) * 64, 0, lane);
-            const uint4 *Q = ops + A.oP[0] + at, *D = ops + A.oP[1 + d] + at;
+            const O16 Q = op(A.oP[0]) + at, D = op(A.oP[1 + d]) + at;
             if (pair) {
-              const uint4 bq[2] = {__ldg(Q), __ldg(Q + 32)}, bd[2] = {__ldg(D), __ldg(D + 32)};
-              mma_pair2<PR, 2>(o[1 + d], oe[1 + d], x, bq, o[0], oe[0], y, bd);
+              const T16 bq[2] = {Q[0], Q[32]}, bd[2] = {D[0], D[32]};
+              mma_pair2<PR, PD>(o[1 + d], x, bq, o[0], y, bd);
             } else {
-              mma_tile<PR>(o[1 + d][0], oe[1 + d][0], x, __ldg(Q));
-              mma_tile<PR>(o[0][0], oe[0][0], y, __ldg(D));
+              const T16 bq[1] = {Q[0]}, bd[1] = {D[0]};
+              mma_pair2<PR, PD>(one(o[1 + d]), x, bq, one(o[0]), y, bd);
             }
           }
         }
@@ -362,26 +369,26 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) r[c][i][j] = (o[c][i][j] + oe[c][i][j]) * (j < 2 ? ia : ib);
+          for (int j = 0; j < 4; ++j) r[c][i][j] = o[c][i][j] * (j < 2 ? ia : ib);
     }
 
     // ---- 4. lifted fluxes
 #pragma unroll 1
     for (int f = 0; f < 4 && mine; ++f) {
-      float o[4][2][4] = {}, oe[4][2][4] = {};
+      float o[4][2][4] = {};
 #pragma unroll 1
       for (int ch = 0; ch < A.FC; ++ch) {
         const uint4 *W = sFc + (f * A.FC + ch) * 4 * 64;
-        const uint4 *B = ops + A.oL + ((f * A.FC + ch) * NB + 2 * w) * 32;
-        const uint4 b[2] = {__ldg(B), pair ? __ldg(B + 32) : make_uint4(0, 0, 0, 0)};
+        const O16 B = op(A.oL) + ((f * A.FC + ch) * NB + 2 * w) * 32;
+        const T16 b[2] = {B[0], B[pair ? 32 : 0]};
 #pragma unroll
         for (int c = 0; c < 4; c += 2) {
           const Frag x = get_frag(W + c * 64, 0, lane), y = get_frag(W + (c + 1) * 64, 0, lane);
           if (pair) {
-            mma_pair2<PR, 2>(o[c], oe[c], x, b, o[c + 1], oe[c + 1], y, b);
+            mma_pair2<PR, PR>(o[c], x, b, o[c + 1], y, b);
           } else {
-            mma_tile<PR>(o[c][0], oe[c][0], x, b[0]);
-            mma_tile<PR>(o[c + 1][0], oe[c + 1][0], y, b[0]);
+            const T16 b1[1] = {b[0]};
+            mma_pair2<PR, PR>(one(o[c]), x, b1, one(o[c + 1]), y, b1);
           }
         }
       }
@@ -392,7 +399,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            r[c][i][j] = fmaf(o[c][i][j] + oe[c][i][j], j < 2 ? ia : ib, r[c][i][j]);
+            r[c][i][j] = fmaf(o[c][i][j], j < 2 ? ia : ib, r[c][i][j]);
     }
 
     // ---- 5. rk_update_WADG: interpolate, weight with 1/J (c2/J on p), project
@@ -415,7 +422,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
       split_unit(xa, xb);
       group_sync<GW>(grp);
     }
-    float o[4][2][4] = {}, oe[4][2][4] = {};
+    float o[4][2][4] = {};
     float oinv[4][2];
     {
       float isc[4][2], d[4][2];
@@ -436,37 +443,37 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
         if (c0 > 0) group_sync<GW>(grp);
 #pragma unroll 1
         for (int c = c0 + w; c < cend; c += GW) {
-          float v[4][2][4] = {}, e[4][2][4] = {};
+          float v[4][2][4] = {};
 #pragma unroll
           for (int k = 0; k < KP; ++k) {
-            const uint4 *B = ops + A.oVr + ((c * KP + k) * 2) * 32;
-            const uint4 b2[2] = {__ldg(B), __ldg(B + 32)};
+            const O16 B = op(A.oVr) + ((c * KP + k) * 2) * 32;
+            const T16 b2[2] = {B[0], B[32]};
 #pragma unroll
             for (int x = 0; x < 4; x += 2)
-              mma_pair2<PR, 2>(v[x], e[x], get_frag(sA + x * AS, k, lane), b2, v[x + 1], e[x + 1],
-                               get_frag(sA + (x + 1) * AS, k, lane), b2);
+              mma_pair2<PR, PR>(v[x], get_frag(sA + x * AS, k, lane), b2, v[x + 1],
+                            get_frag(sA + (x + 1) * AS, k, lane), b2);
           }
           if constexpr (KT) {
-            const uint2 *B = tail(A.oVrt) + (c * 2) * 32;
-            const uint2 b2[2] = {__ldg(B), __ldg(B + 32)};
+            const O8 B = tail(A.oVrt) + (c * 2) * 32;
+            const OpTile<uint2> b2[2] = {B[0], B[32]};
 #pragma unroll
             for (int x = 0; x < 4; x += 2)
-              mma_pair2<PR, 2>(v[x], e[x], get_frag8(sA + x * AS, KP, lane), b2, v[x + 1], e[x + 1],
-                               get_frag8(sA + (x + 1) * AS, KP, lane), b2);
+              mma_pair2<PR, PR>(v[x], get_frag8(sA + x * AS, KP, lane), b2, v[x + 1],
+                            get_frag8(sA + (x + 1) * AS, KP, lane), b2);
           }
           const float *G = A.jq + ((size_t)it * A.nchr + c) * 2 * 256;
           const float4 *pa = reinterpret_cast<const float4 *>(G + g * 16) + t, *pb = pa + 32;
           const float4 ja = __ldg(pa), jb = __ldg(pb), za = __ldg(pa + 64), zb = __ldg(pb + 64);
 #pragma unroll
           for (int x = 0; x < 4; ++x) {
-            float4 ya = make_float4((v[x][0][0] + e[x][0][0]) * isc[x][0] * ja.x,
-                                    (v[x][0][1] + e[x][0][1]) * isc[x][0] * ja.y,
-                                    (v[x][1][0] + e[x][1][0]) * isc[x][0] * ja.z,
-                                    (v[x][1][1] + e[x][1][1]) * isc[x][0] * ja.w);
-            float4 yb = make_float4((v[x][0][2] + e[x][0][2]) * isc[x][1] * jb.x,
-                                    (v[x][0][3] + e[x][0][3]) * isc[x][1] * jb.y,
-                                    (v[x][1][2] + e[x][1][2]) * isc[x][1] * jb.z,
-                                    (v[x][1][3] + e[x][1][3]) * isc[x][1] * jb.w);
+            float4 ya = make_float4(v[x][0][0] * isc[x][0] * ja.x,
+                                    v[x][0][1] * isc[x][0] * ja.y,
+                                    v[x][1][0] * isc[x][0] * ja.z,
+                                    v[x][1][1] * isc[x][0] * ja.w);
+            float4 yb = make_float4(v[x][0][2] * isc[x][1] * jb.x,
+                                    v[x][0][3] * isc[x][1] * jb.y,
+                                    v[x][1][2] * isc[x][1] * jb.z,
+                                    v[x][1][3] * isc[x][1] * jb.w);
             if (x == 0) {
               ya = make_float4(ya.x * za.x, ya.y * za.y, ya.z * za.z, ya.w * za.w);
               yb = make_float4(yb.x * zb.x, yb.y * zb.y, yb.z * zb.z, yb.w * zb.w);
@@ -480,16 +487,16 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll 1
         for (int c = c0; c < cend && mine; ++c) {
           const uint4 *W = sW + (c - c0) * 4 * 64;
-          const uint4 *B = ops + A.oPr + (c * NB + 2 * w) * 32;
-          const uint4 b2[2] = {__ldg(B), pair ? __ldg(B + 32) : make_uint4(0, 0, 0, 0)};
+          const O16 B = op(A.oPr) + (c * NB + 2 * w) * 32;
+          const T16 b2[2] = {B[0], B[pair ? 32 : 0]};
 #pragma unroll
           for (int x = 0; x < 4; x += 2) {
             const Frag f0 = get_frag(W + x * 64, 0, lane), f1 = get_frag(W + (x + 1) * 64, 0, lane);
             if (pair) {
-              mma_pair2<PR, 2>(o[x], oe[x], f0, b2, o[x + 1], oe[x + 1], f1, b2);
+              mma_pair2<PR, PR>(o[x], f0, b2, o[x + 1], f1, b2);
             } else {
-              mma_tile<PR>(o[x][0], oe[x][0], f0, b2[0]);
-              mma_tile<PR>(o[x + 1][0], oe[x + 1][0], f1, b2[0]);
+              const T16 b1[1] = {b2[0]};
+              mma_pair2<PR, PR>(one(o[x]), f0, b1, one(o[x + 1]), f1, b1);
             }
           }
         }
@@ -506,11 +513,11 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
         const float s = oinv[c][h];
         const float4 q = h ? qb[c] : qa[c];
         if (!mine || !(h ? vb : va)) continue;
-        const float2 x0 = make_float2((o[c][0][2 * h] + oe[c][0][2 * h]) * s,
-                                      (o[c][0][2 * h + 1] + oe[c][0][2 * h + 1]) * s);
+        const float2 x0 = make_float2(o[c][0][2 * h] * s,
+                                      o[c][0][2 * h + 1] * s);
         if (pair) {
-          const float2 x1 = make_float2((o[c][1][2 * h] + oe[c][1][2 * h]) * s,
-                                        (o[c][1][2 * h + 1] + oe[c][1][2 * h + 1]) * s);
+          const float2 x1 = make_float2(o[c][1][2 * h] * s,
+                                        o[c][1][2 * h + 1] * s);
           const int n = 16 * w + 4 * t;
           const float4 old = load4<Np, V>(res + at, n);
           const float2 y0 = lsrk2(lo2(old), x0, fa2, fd2), y1 = lsrk2(hi2(old), x1, fa2, fd2);

@@ -37,7 +37,9 @@ struct GroupCfg {
   static constexpr int NG = N <= 6 ? 12 / GW : 1;
   static constexpr int W = GW * NG, T = 32 * W;
   static constexpr bool KEEP = U <= GW;  // a warp's old state stays in registers
-  static constexpr bool OPS = N <= 5;    // operators in shared memory when they fit
+  // operators in shared memory when they fit; else their rests (a fifth of them;
+  // rests from L2 as well / from shared memory: N = 7, K = 24576 219 / 207 us per stage)
+  static constexpr bool OPS = N <= 5;
   static constexpr int V = Np % 4 == 0 ? 4 : Np % 2 == 0 ? 2 : 1;  // vector width of a row
   // state tile of a group: rows of 4 Np floats, padded so that two rows of a
   // pair start 16 banks apart (a 16-byte access serves two rows at a time).
@@ -46,15 +48,16 @@ struct GroupCfg {
   static constexpr int ROWS = 16 * EW + 8 * ODD;
   static constexpr int TILE = ROWS > 512 * NB ? ROWS : 512 * NB;
   __host__ __device__ static constexpr int row(int e) { return e * EW + ((e + 1) >> 1) * ODD; }
-  static constexpr int FLUX = 4 * FB * 128;    // split face fluxes
-  static constexpr int RPF = NB * 128;         // split rhs_p
+  // split face fluxes, then split rhs_p over them
+  static constexpr int FLUX = 4 * FB * 128;
+  static_assert(NB <= 4 * FB, "rhs_p fits over the fluxes");
   static constexpr int RC = GW == 6 ? 12 : 8;  // cubature chunks per round
-  static constexpr bool EARLY = !OPS;  // residual of p loaded before the projection
+  static constexpr bool EARLY = !OPS;    // residual of p loaded before the projection
   static constexpr int SCR1 = 8 * FB * 8;      // one warp's face fluxes of eight elements
   static constexpr int WF = RC * 256 > GW * SCR1 ? RC * 256 : GW * SCR1;  // split cubature values
   static constexpr int GEO = 16 * 28;
   static constexpr int MISC = GW * 16 * 4 + GW * 16 + 64;  // maxima of the state, of rhs_p, face scales
-  static constexpr int SCR = TILE + FLUX + RPF + WF + GEO + MISC;  // floats per group
+  static constexpr int SCR = TILE + FLUX + WF + GEO + MISC;  // floats per group
 };
 
 // Gather of face f of eight elements h8 .. h8 + 7 of the tile, nodes I0 .. I0 +
@@ -203,14 +206,7 @@ struct Unit<1> {
   }
 };
 
-// operator fragment from shared or global memory
-template <bool OPS, class T>
-__device__ __forceinline__ T op_load(const T *p) {
-  if constexpr (OPS) return *p;
-  else return __ldg(p);
-}
-
-template <int N, int PR, bool OPS>
+template <int N, int PR, int PLACE>
 __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpParams P) {
   using C = GroupCfg<N>;
   constexpr int Np = C::Np, Nfp = C::Nfp, NB = C::NB, KP = C::KP, KT = C::KT, EW = C::EW;
@@ -220,29 +216,33 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
   const int grp = warp / GW, w = warp - grp * GW;
   const int g = lane >> 2, t = lane & 3;
   uint4 *sOps = reinterpret_cast<uint4 *>(smem_raw);
-  const int nops = OPS ? P.ops_n : 0;
+  constexpr bool OPS = PLACE == OPS_SHARED;
+  const int nops = OPS ? P.ops_n : PLACE == OPS_RESTS ? P.ops_n - P.oM : 0;
   int *sTab = reinterpret_cast<int *>(sOps + nops);
   float *scr = reinterpret_cast<float *>(sTab + P.table_ints) + grp * C::SCR;
   // operators and tables, all copies in flight with the first tile's
   if constexpr (OPS) stage_async<C::T>(sOps, P.ops, P.ops_n);
+  if constexpr (PLACE == OPS_RESTS) stage_async<C::T>(sOps, P.ops + P.oM, nops);
   stage_async<C::T>(reinterpret_cast<uint4 *>(sTab), reinterpret_cast<const uint4 *>(P.tables),
                     P.table_ints / 4);
   float *sQ = scr;                                            // state rows, then
   uint4 *sA = reinterpret_cast<uint4 *>(scr);                 // split p, Ur, Us, Ut
   constexpr int AS = KP * 64 + KT * 32, FS = FP * 64 + FT * 32;  // uint4 per operand, per face
   uint4 *sFr = reinterpret_cast<uint4 *>(scr + C::TILE);      // split face fluxes
-  uint4 *sR = reinterpret_cast<uint4 *>(scr + C::TILE + C::FLUX);             // split rhs_p
-  uint4 *sW = reinterpret_cast<uint4 *>(scr + C::TILE + C::FLUX + C::RPF);    // split c2 Vq rhs_p
-  float *sF = scr + C::TILE + C::FLUX + C::RPF + w * C::SCR1;  // before that, face fluxes
-  float *sGeo = scr + C::TILE + C::FLUX + C::RPF + C::WF;
+  uint4 *sR = sFr;                                            // split rhs_p, once these are consumed
+  uint4 *sW = reinterpret_cast<uint4 *>(scr + C::TILE + C::FLUX);    // split c2 Vq rhs_p
+  float *sF = scr + C::TILE + C::FLUX + w * C::SCR1;  // before that, face fluxes
+  float *sGeo = scr + C::TILE + C::FLUX + C::WF;
   float4 *sMax = reinterpret_cast<float4 *>(sGeo + C::GEO);   // [GW][16] |p|, |u|, |v|, |w|
   float *sMaxR = sGeo + C::GEO + GW * 64, *sInv = sMaxR + GW * 16;  // [GW][16], [4][16]
   const uint4 *ops = OPS ? sOps : P.ops;
-  const uint4 *oD = ops + lane, *oL = ops + P.oL + lane, *oV = ops + P.oV + lane,
-              *oP = ops + P.oP + lane;
-  const uint2 *oDt = reinterpret_cast<const uint2 *>(ops + P.oDt) + lane,
-              *oLt = reinterpret_cast<const uint2 *>(ops + P.oLt) + lane,
-              *oVt = reinterpret_cast<const uint2 *>(ops + P.oVt) + lane;
+  constexpr int PD = PR == 4 ? 5 : PR;  // derivatives: large terms cancel
+  using O16 = Ops<uint4, PR, !OPS, PLACE == OPS_L2>;
+  using O8 = Ops<uint2, PR, !OPS, PLACE == OPS_L2>;
+  const void *rests = PLACE == OPS_RESTS ? sOps : ops + P.oM;
+  const O16 oD(ops, rests, 0, lane), oL(ops, rests, P.oL, lane), oV(ops, rests, P.oV, lane),
+      oP(ops, rests, P.oP, lane);
+  const O8 oDt(ops, rests, P.oDt, lane), oLt(ops, rests, P.oLt, lane), oVt(ops, rests, P.oVt, lane);
   const int klast = P.Kc - 1;
   const size_t shot_stride = (size_t)P.K * EW;
   const int step = gridDim.x * C::NG;
@@ -480,42 +480,42 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
       using T = typename Un::T;
       float rv[3][m][4], rr[m][4], rd[m][4];  // rr: lifted part, rd: divergence
       {
-        float d[3][m][4] = {}, e[3][m][4] = {}, dv[m][4] = {}, ev[m][4] = {};
+        float d[3][m][4] = {}, dv[m][4] = {};
         // from L2 the next step's operators are loaded during a step's products
         // (48 per warp, about the latency): with the projection's below N = 7
         // 207 -> 183, N = 6 134 -> 129 us per stage
-        uint4 bk[2][3][m];
+        OpTile<uint4> bk[2][3][m];
         auto load_d = [&](int k) {
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int i = 0; i < m; ++i)
-              bk[k & 1][c][i] = op_load<OPS>(oD + ((c * KP + k) * NB + 2 * u + i) * 32);
+              bk[k & 1][c][i] = oD[((c * KP + k) * NB + 2 * u + i) * 32];
         };
         if constexpr (!OPS && KP > 0) load_d(0);
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
           if (OPS) load_d(k);
           else if (k + 1 < KP) load_d(k + 1);
-          const uint4 (&b)[3][m] = bk[k & 1];
+          const OpTile<uint4> (&b)[3][m] = bk[k & 1];
           const Frag x = get_frag(sA, k, lane);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const Frag y = get_frag(sA + (c + 1) * AS, k, lane);
-            mma_pair2<PR, m>(d[c], e[c], x, b[c], dv, ev, y, b[c]);
+            mma_pair2<PD, PD>(d[c], x, b[c], dv, y, b[c]);
           }
         }
         if constexpr (KT) {
-          uint2 b[3][m];
+          OpTile<uint2> b[3][m];
 #pragma unroll
           for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int i = 0; i < m; ++i) b[c][i] = op_load<OPS>(oDt + (c * NB + 2 * u + i) * 32);
+            for (int i = 0; i < m; ++i) b[c][i] = oDt[(c * NB + 2 * u + i) * 32];
           const Frag8 x = get_frag8(sA, KP, lane);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const Frag8 y = get_frag8(sA + (c + 1) * AS, KP, lane);
-            mma_pair2<PR, m>(d[c], e[c], x, b[c], dv, ev, y, b[c]);
+            mma_pair2<PD, PD>(d[c], x, b[c], dv, y, b[c]);
           }
         }
 #pragma unroll
@@ -529,11 +529,10 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           for (int i = 0; i < m; ++i)
 #pragma unroll
             for (int v = 2 * h; v < 2 * h + 2; ++v) {
-              const float a = d[0][i][v] + e[0][i][v], b = d[1][i][v] + e[1][i][v],
-                          c = d[2][i][v] + e[2][i][v];
+              const float a = d[0][i][v], b = d[1][i][v], c = d[2][i][v];
 #pragma unroll
               for (int x = 0; x < 3; ++x) rv[x][i][v] = H[x] * a + H[3 + x] * b + H[6 + x] * c;
-              rd[i][v] = dv[i][v] + ev[i][v], rr[i][v] = 0.f;
+              rd[i][v] = dv[i][v], rr[i][v] = 0.f;
             }
         }
       }
@@ -553,19 +552,16 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           xa[c] = lo2(qa[c + 1]), xb[c] = lo2(qb[c + 1]);
         }
       }
-      // rolled up the loop needs fewer registers: us per stage unrolled / rolled,
-      // N = 6 131 / 123, N = 7 184 / 178 (K = 24576), N = 5 (K = 82944) split FP16
-      // 177 / 167, but FP32 182 / 186
-      constexpr int LU = OPS && PR == 4 ? 2 : 1;
+      // rolled up or not by registers; us per stage unrolled / rolled: N = 5 (K =
+      // 196608) 448 / 429, split FP16 (K = 82944) 167 / 171; N = 4 (K = 3072) 13.3 / 14.0
+      constexpr int LU = OPS && (N == 4 || PR == 3) ? 2 : 1;
 #pragma unroll LU
       for (int f0 = 0; f0 < 4; f0 += 2) {
-        // corrections of all steps first, then the leading products: the
-        // matrix unit rounds toward zero, so few large sums
         float L[2][m][4] = {};
         Frag x[2][FP > 0 ? FP : 1];
-        uint4 b[2][FP > 0 ? FP : 1][m];
+        OpTile<uint4> b[2][FP > 0 ? FP : 1][m];
         Frag8 x8[2];
-        uint2 b8[2][m];
+        OpTile<uint2> b8[2][m];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const int f = f0 + j;
@@ -573,35 +569,17 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           for (int k = 0; k < FP; ++k) {
             x[j][k] = get_frag(sFr + f * FS, k, lane);
 #pragma unroll
-            for (int i = 0; i < m; ++i) b[j][k][i] = op_load<OPS>(oL + ((f * FP + k) * NB + 2 * u + i) * 32);
+            for (int i = 0; i < m; ++i) b[j][k][i] = oL[((f * FP + k) * NB + 2 * u + i) * 32];
           }
           if constexpr (FT) {
             x8[j] = get_frag8(sFr + f * FS, FP, lane);
 #pragma unroll
-            for (int i = 0; i < m; ++i) b8[j][i] = op_load<OPS>(oLt + (f * NB + 2 * u + i) * 32);
+            for (int i = 0; i < m; ++i) b8[j][i] = oLt[(f * NB + 2 * u + i) * 32];
           }
         }
-        auto all = [&](auto &&op) {
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int i = 0; i < m; ++i) op(j, i);
-        };
-#pragma unroll
-        for (int k = 0; k < FP; ++k) {
-          if constexpr (PR == 4) all([&](int j, int i) { mma_hl(L[j][i], x[j][k].l, b[j][k][i], true); });
-          all([&](int j, int i) { mma_hl(L[j][i], x[j][k].h, b[j][k][i], true); });
-          all([&](int j, int i) { mma_hl(L[j][i], x[j][k].l, b[j][k][i], false); });
-        }
-        if constexpr (FT) {
-          if constexpr (PR == 4) all([&](int j, int i) { mma_hl(L[j][i], x8[j].l, b8[j][i], true); });
-          all([&](int j, int i) { mma_hl(L[j][i], x8[j].h, b8[j][i], true); });
-          all([&](int j, int i) { mma_hl(L[j][i], x8[j].l, b8[j][i], false); });
-          all([&](int j, int i) { mma_hl(L[j][i], x8[j].h, b8[j][i], false); });
-        }
-#pragma unroll
-        for (int k = 0; k < FP; ++k)
-          all([&](int j, int i) { mma_hl(L[j][i], x[j][k].h, b[j][k][i], false); });
+        for (int k = 0; k < FP; ++k) mma_pair2<PR, PR>(L[0], x[0][k], b[0][k], L[1], x[1][k], b[1][k]);
+        if constexpr (FT) mma_pair2<PR, PR>(L[0], x8[0], b8[0], L[1], x8[1], b8[1]);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -710,13 +688,13 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 
     // ---- 5. WADG projection of rhs_p, RC chunks of 16 cubature points at a
     //         time: Vq and c2 of the warp's chunks, then Pq of its units
-    float o[UW][2][4], oe[UW][2][4];
+    float o[UW][2][4];
 #pragma unroll
     for (int i = 0; i < UW; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) o[i][j][v] = oe[i][j][v] = 0.f;
+        for (int v = 0; v < 4; ++v) o[i][j][v] = 0.f;
 #pragma unroll 1
     for (int c0 = 0; c0 < nch; c0 += C::RC) {
       const int cend = min(nch, c0 + C::RC);
@@ -724,45 +702,25 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 #pragma unroll 1
       for (int c = c0 + w; c < cend; c += GW) {
         const float4 za = __ldg(Ca + c * 4), zb = __ldg(Cb + c * 4);
-        float v[6][4] = {};
-        uint4 bv[OPS ? 1 : KP][2];
+        float v[2][4] = {};
+        OpTile<uint4> bv[OPS ? 1 : KP][2];
         if constexpr (!OPS)
 #pragma unroll
           for (int k = 0; k < KP; ++k)
 #pragma unroll
-            for (int i = 0; i < 2; ++i) bv[k][i] = __ldg(oV + ((c * KP + k) * 2 + i) * 32);
+            for (int i = 0; i < 2; ++i) bv[k][i] = oV[((c * KP + k) * 2 + i) * 32];
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
           const Frag x = get_frag(sR, k, lane);
-          const uint4 b0 = OPS ? oV[((c * KP + k) * 2) * 32] : bv[OPS ? 0 : k][0],
-                      b1 = OPS ? oV[((c * KP + k) * 2 + 1) * 32] : bv[OPS ? 0 : k][1];
-          mma16(v[0], x.h, b0.x, b0.y);
-          mma16(v[1], x.h, b1.x, b1.y);
-          mma16(v[2], x.h, b0.z, b0.w);
-          mma16(v[3], x.h, b1.z, b1.w);
-          mma16(v[4], x.l, b0.x, b0.y);
-          mma16(v[5], x.l, b1.x, b1.y);
-          if constexpr (PR == 4) {
-            mma16(v[2], x.l, b0.z, b0.w);
-            mma16(v[3], x.l, b1.z, b1.w);
-          }
+          const OpTile<uint4> b[2] = {OPS ? oV[((c * KP + k) * 2) * 32] : bv[OPS ? 0 : k][0],
+                                      OPS ? oV[((c * KP + k) * 2 + 1) * 32] : bv[OPS ? 0 : k][1]};
+          mma_tiles<PR>(v, x, b);
         }
         if constexpr (KT) {
           const Frag8 x = get_frag8(sR, KP, lane);
-          const uint2 b0 = op_load<OPS>(oVt + (c * 2) * 32), b1 = op_load<OPS>(oVt + (c * 2 + 1) * 32);
-          mma8(v[0], x.h[0], x.h[1], b0.x);
-          mma8(v[1], x.h[0], x.h[1], b1.x);
-          mma8(v[2], x.h[0], x.h[1], b0.y);
-          mma8(v[3], x.h[0], x.h[1], b1.y);
-          mma8(v[4], x.l[0], x.l[1], b0.x);
-          mma8(v[5], x.l[0], x.l[1], b1.x);
-          if constexpr (PR == 4) {
-            mma8(v[2], x.l[0], x.l[1], b0.y);
-            mma8(v[3], x.l[0], x.l[1], b1.y);
-          }
+          const OpTile<uint2> b[2] = {oVt[(c * 2) * 32], oVt[(c * 2 + 1) * 32]};
+          mma_tiles<PR>(v, x, b);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[0][i] += v[2][i] + v[4][i], v[1][i] += v[3][i] + v[5][i];
         // points 16 c + 4 t + 0 .. 3 of the two rows
         const float4 xa = make_float4(v[0][0] * via * za.x, v[0][1] * via * za.y,
                                       v[1][0] * via * za.z, v[1][1] * via * za.w);
@@ -772,19 +730,19 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
       }
       if constexpr (!OPS && UW == 1) {
         // operators from L2: the next four chunks' loads in flight
-        uint4 b[4][2];
+        OpTile<uint4> b[4][2];
         auto load_p = [&](int c) {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
 #pragma unroll
             for (int i = 0; i < 2; ++i)
-              b[j][i] = __ldg(oP + (min(c + j, nch - 1) * NB + min(2 * w + i, NB - 1)) * 32);
+              b[j][i] = oP[(min(c + j, nch - 1) * NB + min(2 * w + i, NB - 1)) * 32];
         };
         load_p(c0);
         group_sync<GW>(grp);  // the round's values ready
 #pragma unroll 1
         for (int c = c0; c < cend; c += 4) {
-          uint4 bb[4][2];
+          OpTile<uint4> bb[4][2];
 #pragma unroll
           for (int j = 0; j < 4; ++j) bb[j][0] = b[j][0], bb[j][1] = b[j][1];
           if (c + 4 < cend) load_p(c + 4);
@@ -792,8 +750,8 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           for (int j = 0; j < 4; ++j) {
             if (c + j >= cend) break;
             const Frag x = get_frag(sW, c + j - c0, lane);
-            if (w < KP) mma_tiles<PR, 2>(o[0], oe[0], x, bb[j]);
-            else if (w < C::U) mma_tile<PR>(o[0][0], oe[0][0], x, bb[j][0]);
+            if (w < KP) mma_tiles<PR>(o[0], x, bb[j]);
+            else if (w < C::U) mma_tile<PR>(o[0][0], x, bb[j][0]);
           }
         }
         continue;
@@ -806,10 +764,10 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
         for (int i = 0; i < UW; ++i) {
           const int u = w + i * GW;
           if (u < KP) {
-            const uint4 b[2] = {oP[(c * NB + 2 * u) * 32], oP[(c * NB + 2 * u + 1) * 32]};
-            mma_tiles<PR, 2>(o[i], oe[i], x, b);
+            const OpTile<uint4> b[2] = {oP[(c * NB + 2 * u) * 32], oP[(c * NB + 2 * u + 1) * 32]};
+            mma_tiles<PR>(o[i], x, b);
           } else if (u < C::U) {
-            mma_tile<PR>(o[i][0], oe[i][0], x, oP[(c * NB + 2 * u) * 32]);
+            mma_tile<PR>(o[i][0], x, oP[(c * NB + 2 * u) * 32]);
           }
         }
       }
@@ -821,7 +779,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) o[i][j][v] = (o[i][j][v] + oe[i][j][v]) * (v < 2 ? oia : oib);
+        for (int v = 0; v < 4; ++v) o[i][j][v] *= v < 2 ? oia : oib;
     if (P.src_tile)
       tile_sources(P, Np, shot, k0, [&](int e, float amp, const float *vec) {
 #pragma unroll
@@ -888,45 +846,56 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 
 // ---------------------------------------------------------------- host side
 template <int N>
-static size_t group_smem(const WarpPlan &pl, bool ops) {
+static size_t group_smem(const WarpPlan &pl, int place) {
   using C = GroupCfg<N>;
-  return (ops ? (size_t)pl.ops_n * 16 : 0) + (size_t)pl.table_ints * 4 + (size_t)C::NG * C::SCR * 4;
+  const int n = place == OPS_SHARED ? pl.ops_n : place == OPS_RESTS ? pl.ops_n - pl.oM : 0;
+  return (size_t)n * 16 + (size_t)pl.table_ints * 4 + (size_t)C::NG * C::SCR * 4;
 }
 
+template <int N, int PR, int PLACE>
+static bbw_status group_launch_as(const WarpPlan &pl, const WarpParams &P, int grid, cudaStream_t st) {
+  using C = GroupCfg<N>;
+  launch_stage_kernel(k_group_stage<N, PR, PLACE>, grid, C::T, group_smem<N>(pl, PLACE), st,
+                      PLACE == OPS_SHARED && pl.chained, P);
+  return check_launch("group-matrix stage");
+}
+
+// split FP16 contexts (three products) exist at N <= 5
 template <int N>
 static bbw_status group_launch_n(const WarpPlan &pl, const float *Qin, float *Qout, float *res,
                                  float fa, float fb, float fdt, float cstage, cudaStream_t st) {
   using C = GroupCfg<N>;
   WarpParams P = warp_params(pl, Qin, Qout, res, fa, fb, fdt, cstage);
   const int grid = warp_grid(pl, C::NG, P);
-  const bool os = pl.group_ops;
-  const size_t sm = group_smem<N>(pl, os);
   if constexpr (C::OPS) {
-    if (os) {
-      if (pl.products == 4) launch_stage_kernel(k_group_stage<N, 4, true>, grid, C::T, sm, st, pl.chained, P);
-      else launch_stage_kernel(k_group_stage<N, 3, true>, grid, C::T, sm, st, pl.chained, P);
-      return check_launch("group-matrix stage");
-    }
+    if (pl.products == 3)
+      return pl.group_ops == OPS_SHARED ? group_launch_as<N, 3, OPS_SHARED>(pl, P, grid, st)
+                                        : group_launch_as<N, 3, OPS_L2>(pl, P, grid, st);
+    if (pl.group_ops == OPS_SHARED) return group_launch_as<N, 4, OPS_SHARED>(pl, P, grid, st);
   }
-  if (pl.products == 4) launch_stage_kernel(k_group_stage<N, 4, false>, grid, C::T, sm, st, false, P);
-  else launch_stage_kernel(k_group_stage<N, 3, false>, grid, C::T, sm, st, false, P);
-  return check_launch("group-matrix stage");
+  return pl.group_ops == OPS_RESTS ? group_launch_as<N, 4, OPS_RESTS>(pl, P, grid, st)
+                                   : group_launch_as<N, 4, OPS_L2>(pl, P, grid, st);
 }
 
 template <int N>
 static bbw_status group_prepare_n(WarpPlan &pl) {
-  const int maxsm = device_smem_optin();
-  pl.group_ops = GroupCfg<N>::OPS && group_smem<N>(pl, true) <= (size_t)maxsm;
-  if (group_smem<N>(pl, pl.group_ops) > (size_t)maxsm)
+  using C = GroupCfg<N>;
+  const size_t maxsm = (size_t)device_smem_optin();
+  if (!C::OPS && pl.products == 3)
+    return set_error(BBW_ERR_UNSUPPORTED, "group-matrix stage: three products at N <= 5 only");
+  pl.group_ops = C::OPS && group_smem<N>(pl, OPS_SHARED) <= maxsm ? OPS_SHARED
+                 : pl.products == 4 && group_smem<N>(pl, OPS_RESTS) <= maxsm ? OPS_RESTS : OPS_L2;
+  if (group_smem<N>(pl, pl.group_ops) > maxsm)
     return set_error(BBW_ERR_UNSUPPORTED, "group-matrix stage: does not fit in shared memory");
-  std::vector<const void *> fn = {(const void *)k_group_stage<N, 3, false>,
-                                  (const void *)k_group_stage<N, 4, false>};
-  if constexpr (GroupCfg<N>::OPS) {
-    fn.push_back((const void *)k_group_stage<N, 3, true>);
-    fn.push_back((const void *)k_group_stage<N, 4, true>);
+  std::vector<const void *> fn = {(const void *)k_group_stage<N, 4, OPS_L2>,
+                                  (const void *)k_group_stage<N, 4, OPS_RESTS>};
+  if constexpr (C::OPS) {
+    fn.push_back((const void *)k_group_stage<N, 4, OPS_SHARED>);
+    fn.push_back((const void *)k_group_stage<N, 3, OPS_SHARED>);
+    fn.push_back((const void *)k_group_stage<N, 3, OPS_L2>);
   }
   for (const void *f : fn) {
-    const bbw_status s = ensure_smem_limit(f, maxsm, "group-matrix stage attribute");
+    const bbw_status s = ensure_smem_limit(f, (int)maxsm, "group-matrix stage attribute");
     if (s != BBW_OK) return s;
   }
   return BBW_OK;

@@ -5,6 +5,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <utility>
 
 #include "device_common.cuh"
 #include "internal.h"
@@ -59,22 +61,34 @@ bbw_status warp_prepare(WarpPlan &pl) {
   return BBW_OK;
 }
 
-// power of two that brings the largest |a| into [2^13, 2^14)
+// power of two that brings the largest |a| into [2^14, 2^15): the rest of a pair,
+// 2^-24 of it, then is a byte of three significant bits
 static float operator_scale(const float *a, size_t n) {
   float m = 0.f;
   for (size_t i = 0; i < n; ++i) m = std::max(m, std::fabs(a[i]));
   if (!(m > 0.f) || !std::isfinite(m)) return 1.f;
   int e = 0;
   std::frexp(m, &e);  // m in [2^(e-1), 2^e)
-  return std::ldexp(1.f, std::min(std::max(14 - e, -100), 100));
+  return std::ldexp(1.f, std::min(std::max(15 - e, -100), 100));
 }
 
-// FP16 pair of two values: hi words, or what they leave (lo)
-static void pack_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
-  const __half ha = __float2half_rn(a), hb = __float2half_rn(b);
-  const __half la = __float2half_rn(a - __half2float(ha)), lb = __float2half_rn(b - __half2float(hb));
-  hi = (uint32_t)__half_as_ushort(ha) | (uint32_t)__half_as_ushort(hb) << 16;
-  lo = (uint32_t)__half_as_ushort(la) | (uint32_t)__half_as_ushort(lb) << 16;
+// operator entry times its scale (1 + kRoundingBias) as FP16 hi and lo and the
+// top byte of an FP16 rest
+struct Parts {
+  std::vector<uint32_t> w;  // hi | lo << 16
+  std::vector<uint8_t> m;
+  int nr = 0;
+};
+static void split_entry(double a, uint32_t &w, uint8_t &m) {
+  const __half h = __double2half(a), l = __double2half(a - __half2float(h));
+  w = (uint32_t)__half_as_ushort(h) | (uint32_t)__half_as_ushort(l) << 16;
+  m = rest_byte(__half_as_ushort(__double2half(a - __half2float(h) - __half2float(l))));
+}
+// the column-major nr x nc matrix A times s
+static void split_matrix(Parts &p, const float *A, int nr, int nc, float s) {
+  const size_t n = (size_t)nr * nc;
+  p.nr = nr, p.w.resize(n), p.m.resize(n);
+  for (size_t i = 0; i < n; ++i) split_entry((double)A[i] * s * (1.0 + kRoundingBias), p.w[i], p.m[i]);
 }
 
 // index of slot c of block b when n indices are stored in blocks of eight
@@ -84,29 +98,36 @@ static int warp_node(int n, int b, int c) {
   return 16 * (b / 2) + 4 * (c / 2) + 2 * (b % 2) + c % 2;
 }
 
-// tile of row block j and columns of pair (k16) or block (k8) k of the nr x nc
-// column-major matrix A (row stride 1, column stride ld), zero outside; nrp, ncp:
-// extents whose blocks the indices run over
+// tile of row block j and columns of pair (k16) or block (k8) k of the matrix
+// at p.w + at (nr x nc), zero outside; nrp, ncp: extents whose blocks the
+// indices run over
 struct PackTile {
-  const float *A;
-  int nr, nc, nrp, ncp, ld, j, k;
+  const Parts *p;
+  size_t at;
+  int nr, nc, nrp, ncp, j, k;
   bool k16;
-  float s;
 };
 
-static void pack_tile(const PackTile &q, uint32_t *out) {
+static void pack_tile(const PackTile &q, uint32_t *out, uint8_t *rest) {
   for (int lane = 0; lane < 32; ++lane) {
     const int r = warp_node(q.nrp, q.j, lane / 4), c = 2 * (lane % 4);
-    auto at = [&](int b, int slot) {
-      const int col = warp_node(q.ncp, b, slot);
-      return r < q.nr && col < q.nc ? q.A[r + (size_t)col * q.ld] * q.s : 0.f;
+    // entries c and c + 1 of block b: words of hi, lo; bytes of the rest
+    auto words = [&](int b, uint32_t &hi, uint32_t &lo, uint8_t *m) {
+      uint32_t x[2];
+      for (int i = 0; i < 2; ++i) {
+        const int col = warp_node(q.ncp, b, c + i);
+        const bool in = r < q.nr && col < q.nc;
+        const size_t e = q.at + r + (size_t)col * q.nr;
+        x[i] = in ? q.p->w[e] : 0u, m[i] = in ? q.p->m[e] : 0;
+      }
+      hi = (x[0] & 0xffffu) | x[1] << 16, lo = x[0] >> 16 | (x[1] & 0xffff0000u);
     };
     if (q.k16) {
       uint32_t *o = out + 4 * lane;
-      pack_pair(at(2 * q.k, c), at(2 * q.k, c + 1), o[0], o[2]);
-      pack_pair(at(2 * q.k + 1, c), at(2 * q.k + 1, c + 1), o[1], o[3]);
+      words(2 * q.k, o[0], o[2], rest + 4 * lane);
+      words(2 * q.k + 1, o[1], o[3], rest + 4 * lane + 2);
     } else {
-      pack_pair(at(q.k, c), at(q.k, c + 1), out[2 * lane], out[2 * lane + 1]);
+      words(q.k, out[2 * lane], out[2 * lane + 1], rest + 2 * lane);
     }
   }
 }
@@ -117,32 +138,39 @@ float split_scale(const float *const *A, int n, size_t len) {
   return s;
 }
 
-void split_rows(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off,
-                int &off_tail) {
-  const int nch = (nr + 15) / 16, NB = (nc + 7) / 8, KP = NB / 2, KT = NB % 2;
-  off = (int)(out.size() / 4);
-  for (int c = 0; c < nch; ++c)
-    for (int k = 0; k < KP; ++k)
-      for (int h = 0; h < 2; ++h) {
-        out.resize(out.size() + 128);
-        pack_tile({A, nr, nc, 16 * nch, nc, nr, 2 * c + h, k, true, s}, &out[out.size() - 128]);
-      }
-  off_tail = (int)(out.size() / 4);
-  for (int c = 0; c < nch && KT; ++c)
-    for (int h = 0; h < 2; ++h) {
-      out.resize(out.size() + 64);
-      pack_tile({A, nr, nc, 16 * nch, nc, nr, 2 * c + h, 2 * KP, false, s}, &out[out.size() - 64]);
-    }
+static void append(SplitOps &out, const PackTile &q) {
+  const size_t n = q.k16 ? 128 : 64, at = out.w.size();
+  out.w.resize(at + n), out.m.resize(at + n);
+  pack_tile(q, &out.w[at], &out.m[at]);
 }
 
-void split_columns(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off) {
-  const int nch = (nc + 15) / 16, NB = (nr + 7) / 8;
-  off = (int)(out.size() / 4);
+void split_rows(SplitOps &out, const float *A, int nr, int nc, float s, int &off, int &off_tail) {
+  const int nch = (nr + 15) / 16, NB = (nc + 7) / 8, KP = NB / 2, KT = NB % 2;
+  Parts p;
+  split_matrix(p, A, nr, nc, s);
+  off = (int)(out.w.size() / 4);
   for (int c = 0; c < nch; ++c)
-    for (int j = 0; j < NB; ++j) {
-      out.resize(out.size() + 128);
-      pack_tile({A, nr, nc, nr, 16 * nch, nr, j, c, true, s}, &out[out.size() - 128]);
-    }
+    for (int k = 0; k < KP; ++k)
+      for (int h = 0; h < 2; ++h) append(out, {&p, 0, nr, nc, 16 * nch, nc, 2 * c + h, k, true});
+  off_tail = (int)(out.w.size() / 4);
+  for (int c = 0; c < nch && KT; ++c)
+    for (int h = 0; h < 2; ++h) append(out, {&p, 0, nr, nc, 16 * nch, nc, 2 * c + h, 2 * KP, false});
+}
+
+void split_columns(SplitOps &out, const float *A, int nr, int nc, float s, int &off) {
+  const int nch = (nc + 15) / 16, NB = (nr + 7) / 8;
+  Parts p;
+  split_matrix(p, A, nr, nc, s);
+  off = (int)(out.w.size() / 4);
+  for (int c = 0; c < nch; ++c)
+    for (int j = 0; j < NB; ++j) append(out, {&p, 0, nr, nc, nr, 16 * nch, j, c, true});
+}
+
+std::vector<uint32_t> SplitOps::words() const {
+  std::vector<uint32_t> all(w);
+  all.resize(w.size() + m.size() / 4);
+  std::memcpy(all.data() + w.size(), m.data(), m.size());
+  return all;
 }
 
 void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
@@ -155,6 +183,14 @@ void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<floa
   for (int d = 1; d < 3; ++d) sD = std::min(sD, operator_scale(D[d].data(), D[d].size()));
   const float sL = operator_scale(LIFT.data(), LIFT.size());
   const float sV = operator_scale(Vq.data(), Vq.size()), sP = operator_scale(Pq.data(), Pq.size());
+  Parts D3[3], L, V, P;
+#pragma omp parallel for schedule(dynamic) num_threads(6) if (Np > 30)
+  for (int i = 0; i < 6; ++i) {
+    if (i < 3) split_matrix(D3[i], D[i].data(), Np, Np, sD);
+    else if (i == 3) split_matrix(L, LIFT.data(), Np, 4 * Nfp, sL);
+    else if (i == 4) split_matrix(V, Vq.data(), Nq, Np, sV);
+    else split_matrix(P, Pq.data(), Np, Nq, sP);
+  }
   std::vector<PackTile> tiles;
   std::vector<size_t> offset;
   size_t words = 0;
@@ -165,33 +201,36 @@ void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<floa
   auto at = [&]() { return (int)(words / 4); };
   for (int d = 0; d < 3; ++d)
     for (int k = 0; k < KP; ++k)
-      for (int j = 0; j < NB; ++j) add({D[d].data(), Np, Np, Np, Np, Np, j, k, true, sD});
+      for (int j = 0; j < NB; ++j) add({&D3[d], 0, Np, Np, Np, Np, j, k, true});
   pl.oDt = at();
   for (int d = 0; d < 3 && KT; ++d)
-    for (int j = 0; j < NB; ++j) add({D[d].data(), Np, Np, Np, Np, Np, j, 2 * KP, false, sD});
+    for (int j = 0; j < NB; ++j) add({&D3[d], 0, Np, Np, Np, Np, j, 2 * KP, false});
   pl.oL = at();
-  auto face = [&](int f) { return LIFT.data() + (size_t)f * Nfp * Np; };
+  auto face = [&](int f) { return (size_t)f * Nfp * Np; };
   for (int f = 0; f < 4; ++f)
     for (int k = 0; k < FP; ++k)
-      for (int j = 0; j < NB; ++j) add({face(f), Np, Nfp, Np, Nfp, Np, j, k, true, sL});
+      for (int j = 0; j < NB; ++j) add({&L, face(f), Np, Nfp, Np, Nfp, j, k, true});
   pl.oLt = at();
   for (int f = 0; f < 4 && FT; ++f)
-    for (int j = 0; j < NB; ++j) add({face(f), Np, Nfp, Np, Nfp, Np, j, 2 * FP, false, sL});
+    for (int j = 0; j < NB; ++j) add({&L, face(f), Np, Nfp, Np, Nfp, j, 2 * FP, false});
   pl.oV = at();
   for (int c = 0; c < nch; ++c)
     for (int k = 0; k < KP; ++k)
-      for (int h = 0; h < 2; ++h) add({Vq.data(), Nq, Np, Nq16, Np, Nq, 2 * c + h, k, true, sV});
+      for (int h = 0; h < 2; ++h) add({&V, 0, Nq, Np, Nq16, Np, 2 * c + h, k, true});
   pl.oVt = at();
   for (int c = 0; c < nch && KT; ++c)
-    for (int h = 0; h < 2; ++h) add({Vq.data(), Nq, Np, Nq16, Np, Nq, 2 * c + h, 2 * KP, false, sV});
+    for (int h = 0; h < 2; ++h) add({&V, 0, Nq, Np, Nq16, Np, 2 * c + h, 2 * KP, false});
   pl.oP = at();
   for (int c = 0; c < nch; ++c)
-    for (int j = 0; j < NB; ++j) add({Pq.data(), Np, Nq, Np, Nq16, Np, j, c, true, sP});
-  pl.ops_n = at();
-  out.resize(words);
+    for (int j = 0; j < NB; ++j) add({&P, 0, Np, Nq, Np, Nq16, j, c, true});
+  pl.oM = at();
+  SplitOps all;
+  all.w.resize(words), all.m.resize(words);
   const long long nt = (long long)tiles.size();
 #pragma omp parallel for schedule(static) num_threads(8) if (nt > 128)
-  for (long long i = 0; i < nt; ++i) pack_tile(tiles[i], &out[offset[i]]);
+  for (long long i = 0; i < nt; ++i) pack_tile(tiles[i], &all.w[offset[i]], &all.m[offset[i]]);
+  out = pl.products == 4 ? all.words() : std::move(all.w);
+  pl.ops_n = (int)(out.size() / 4);
   pl.iD = 1.f / sD, pl.iL = 1.f / sL, pl.iV = 1.f / sV, pl.iP = 1.f / sP;
   double vn = 0.0;
   for (int q = 0; q < Nq; ++q) {

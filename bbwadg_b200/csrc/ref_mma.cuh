@@ -2,7 +2,8 @@
 // (warp_mma.cuh) for the kernel-level entry points.
 //
 // The entry points take the reference's arrays as they are, so each CTA splits
-// the operators into shared memory first (a few microseconds), then its warps
+// the operators into shared memory first (a few microseconds; pairs and a rest,
+// as warp_pack does), then its warps
 // walk 16-element tiles.  The kernels with a thread per node (kernels_ref.cu)
 // spend one operator load and one or more shared loads per FMA; they stay for
 // small meshes, N = 8, and pointers that are not 16-byte aligned.
@@ -22,8 +23,8 @@ __device__ __forceinline__ int slot_index(int n, int b, int c) {
   return 16 * (b / 2) + 4 * (c / 2) + 2 * (b % 2) + c % 2;
 }
 
-// power of two that brings the CTA-wide maximum of |A| (n values) into [2^13,
-// 2^14), as an exponent field; sRed: one int of shared memory, zero on entry
+// power of two that brings the CTA-wide maximum of |A| (n values) into [2^14,
+// 2^15), as an exponent field; sRed: one int of shared memory, zero on entry
 __device__ __forceinline__ void block_max(int *sRed, const float *__restrict__ A, int n) {
   float m = 0.f;
   for (int i0 = threadIdx.x; i0 < n; i0 += 16 * blockDim.x) {  // sixteen loads in flight
@@ -40,34 +41,56 @@ __device__ __forceinline__ void block_max(int *sRed, const float *__restrict__ A
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((threadIdx.x & 31) == 0) atomicMax(sRed, __float_as_int(m));
 }
-__device__ __forceinline__ int operator_field(int red) { return scale_field(__int_as_float(red)) - 1; }
+__device__ __forceinline__ int operator_field(int red) { return scale_field(__int_as_float(red)); }
 
-// split tiles of the column-major nr x nc operator A times s into out: row blocks
-// rb, column pairs (k16) or the odd last block (k8); order [k][block]
+// two operator values as hi, lo and the bytes of the rest, larger by
+// kRoundingBias (split_entry, kernels_warp.cu)
+__device__ __forceinline__ void split_operator(float2 x, float s, uint32_t &h, uint32_t &l, uint32_t &m) {
+  const float2 y = __fmul2_rn(x, both(s));
+  const __half2 hh = __float22half2_rn(y);
+  const float2 f = __half22float2(hh);
+  const float2 r = __ffma2_rn(y, both((float)kRoundingBias), __fadd2_rn(y, make_float2(-f.x, -f.y)));
+  const __half2 ll = __float22half2_rn(r);
+  const float2 g = __half22float2(ll);
+  const __half2 mm = __float22half2_rn(__fadd2_rn(r, make_float2(-g.x, -g.y)));
+  h = *reinterpret_cast<const uint32_t *>(&hh);
+  l = *reinterpret_cast<const uint32_t *>(&ll);
+  m = rest_byte(__half_as_ushort(__low2half(mm))) | rest_byte(__half_as_ushort(__high2half(mm))) << 8;
+}
+// lane's words of a k16 (uint4) or k8 (uint2) tile: at(block, slot) gives the entries
+template <bool K16, class At>
+__device__ __forceinline__ void split_tile(uint32_t *out, uint32_t *rest, int i, int k, int c, float s,
+                                           At &&at) {
+  uint32_t h0, l0, m0;
+  if constexpr (K16) {
+    uint32_t h1, l1, m1;
+    split_operator(make_float2(at(2 * k, c), at(2 * k, c + 1)), s, h0, l0, m0);
+    split_operator(make_float2(at(2 * k + 1, c), at(2 * k + 1, c + 1)), s, h1, l1, m1);
+    reinterpret_cast<uint4 *>(out)[i] = make_uint4(h0, h1, l0, l1);
+    rest[i] = m0 | m1 << 16;
+  } else {
+    split_operator(make_float2(at(k, c), at(k, c + 1)), s, h0, l0, m0);
+    reinterpret_cast<uint2 *>(out)[i] = make_uint2(h0, l0);
+    reinterpret_cast<uint16_t *>(rest)[i] = (uint16_t)m0;
+  }
+}
+
+// split tiles of the column-major nr x nc operator A times s into word `off` of
+// the words at `out` (the rests in the plane at `rest`): row blocks rb, column
+// pairs (k16) or the odd last block (k8); order [k][block]
 template <bool K16>
-__device__ __forceinline__ void split_tiles(uint32_t *out, const float *__restrict__ A, int nr, int nc,
-                                            int nrp, int ncp, int nblk, int k0, int nk, bool k_inner,
-                                            float s) {
+__device__ __forceinline__ void split_tiles(uint32_t *out, uint32_t *rest, int off,
+                                            const float *__restrict__ A, int nr, int nc, int nrp,
+                                            int ncp, int nblk, int k0, int nk, float s) {
   const int tiles = nblk * nk;
 #pragma unroll 4
   for (int i = threadIdx.x; i < tiles * 32; i += blockDim.x) {
     const int tl = i >> 5, lane = i & 31;
-    const int j = k_inner ? tl / nk : tl % nblk, k = k0 + (k_inner ? tl % nk : tl / nblk);
-    const int r = slot_index(nrp, j, lane >> 2), c = 2 * (lane & 3);
-    auto at = [&](int b, int slot) {
+    const int r = slot_index(nrp, tl % nblk, lane >> 2);
+    split_tile<K16>(out + off, rest + off / 4, i, k0 + tl / nblk, 2 * (lane & 3), s, [&](int b, int slot) {
       const int col = slot_index(ncp, b, slot);
       return r < nr && col < nc ? __ldg(A + r + (size_t)col * nr) : 0.f;
-    };
-    uint32_t h0, l0;
-    if constexpr (K16) {
-      uint32_t h1, l1;
-      split2(make_float2(at(2 * k, c), at(2 * k, c + 1)), both(s), h0, l0);
-      split2(make_float2(at(2 * k + 1, c), at(2 * k + 1, c + 1)), both(s), h1, l1);
-      reinterpret_cast<uint4 *>(out)[i] = make_uint4(h0, h1, l0, l1);
-    } else {
-      split2(make_float2(at(k, c), at(k, c + 1)), both(s), h0, l0);
-      reinterpret_cast<uint2 *>(out)[i] = make_uint2(h0, l0);
-    }
+    });
   }
 }
 
@@ -107,9 +130,10 @@ __global__ void __launch_bounds__(256, 1)
                     const float *__restrict__ Ds, const float *__restrict__ Dt,
                     const float *__restrict__ Q, float *__restrict__ rhsQ) {
   using C = RefCfg<N>;
-  constexpr int Np = C::Np, NB = C::NB, KP = C::KP, KT = C::KT, EW = C::EW, V = C::V, PR = 4;
+  constexpr int Np = C::Np, NB = C::NB, KP = C::KP, KT = C::KT, EW = C::EW, V = C::V, PR = 4, PD = 5;
   extern __shared__ __align__(16) uint32_t smem_w[];
-  int *sRed = reinterpret_cast<int *>(smem_w + C::OPS_VOL);
+  uint32_t *rest = smem_w + C::OPS_VOL;
+  int *sRed = reinterpret_cast<int *>(rest + C::OPS_VOL / 4);
   const int nt = (K + 15) / 16;
   if (threadIdx.x == 0) *sRed = 0;
   __syncthreads();
@@ -119,16 +143,17 @@ __global__ void __launch_bounds__(256, 1)
   const float *D[3] = {Dr, Ds, Dt};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    split_tiles<true>(smem_w + c * KP * NB * 128, D[c], Np, Np, Np, Np, NB, 0, KP, false, pow2_field(of));
+    split_tiles<true>(smem_w, rest, c * KP * NB * 128, D[c], Np, Np, Np, Np, NB, 0, KP, pow2_field(of));
     if constexpr (KT)
-      split_tiles<false>(smem_w + 3 * KP * NB * 128 + c * NB * 64, D[c], Np, Np, Np, Np, NB, 2 * KP, 1,
-                         false, pow2_field(of));
+      split_tiles<false>(smem_w, rest, 3 * KP * NB * 128 + c * NB * 64, D[c], Np, Np, Np, Np, NB, 2 * KP,
+                         1, pow2_field(of));
   }
   __syncthreads();
   const float iD = pow2_field(254 - of);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const uint4 *oD = reinterpret_cast<const uint4 *>(smem_w) + lane;
-  const uint2 *oDt = reinterpret_cast<const uint2 *>(smem_w + 3 * KP * NB * 128) + lane;
+  const uint4 *ops = reinterpret_cast<const uint4 *>(smem_w);
+  const Ops<uint4, PR, false> oD(ops, rest, 0, lane);
+  const Ops<uint2, PR, false> oDt(ops, rest, 3 * KP * NB * 32, lane);
   for (int it = first_tile(nt, C::W, warp); it < nt; it += gridDim.x * C::W) {
     const int ka = min(it * 16 + g, K - 1), kb = min(it * 16 + g + 8, K - 1);
     const bool va = it * 16 + g < K, vb = it * 16 + g + 8 < K;
@@ -160,25 +185,25 @@ __global__ void __launch_bounds__(256, 1)
       if constexpr (KT) split_frag(fp8, ya, yb, pow2_field(sa), pow2_field(sb));
       // rhs of u, v, w at block j
       auto block = [&](int j, float (&rv)[3][4]) {
-        float d[3][4] = {}, e[3][4] = {};
+        float d[3][4] = {};
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
-          uint4 b[3];
+          OpTile<uint4> b[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) b[c] = oD[((c * KP + k) * NB + j) * 32];
-          mma_tiles<PR>(d, e, fp[k], b);
+          mma_tiles<PD>(d, fp[k], b);
         }
         if constexpr (KT) {
-          uint2 b[3];
+          OpTile<uint2> b[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) b[c] = oDt[(c * NB + j) * 32];
-          mma_tiles<PR>(d, e, fp8, b);
+          mma_tiles<PD>(d, fp8, b);
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
           const float *G = v < 2 ? Ga : Gb;
           const float s = v < 2 ? ia : ib;
-          const float a = (d[0][v] + e[0][v]) * s, b = (d[1][v] + e[1][v]) * s, c = (d[2][v] + e[2][v]) * s;
+          const float a = d[0][v] * s, b = d[1][v] * s, c = d[2][v] * s;
 #pragma unroll
           for (int x = 0; x < 3; ++x) rv[x][v] = G[x] * a + G[3 + x] * b + G[6 + x] * c;
         }
@@ -230,27 +255,26 @@ __global__ void __launch_bounds__(256, 1)
       }
       const int sa = scale_field(2.f * Ma), sb = scale_field(2.f * Mb);
       const float ca = pow2_field(sa), cb = pow2_field(sb);
-      float r[NB][4], e[NB][4];
+      float r[NB][4];
 #pragma unroll
       for (int j = 0; j < NB; ++j)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) r[j][v] = e[j][v] = 0.f;
-      auto accumulate = [&](const auto &u, const auto *B) {
-        using T = std::remove_const_t<std::remove_reference_t<decltype(*B)>>;
+        for (int v = 0; v < 4; ++v) r[j][v] = 0.f;
+      auto accumulate = [&](const auto &u, const auto B) {
+        using T = decltype(B[0]);
         constexpr int full = NB / 4 * 4, rem = NB % 4;
 #pragma unroll
         for (int j0 = 0; j0 < full; j0 += 4) {
           T b[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) b[j] = B[(j0 + j) * 32];
-          mma_tiles<PR>(*reinterpret_cast<float(*)[4][4]>(&r[j0]), *reinterpret_cast<float(*)[4][4]>(&e[j0]), u, b);
+          mma_tiles<PD>(*reinterpret_cast<float(*)[4][4]>(&r[j0]), u, b);
         }
         if constexpr (rem > 0) {
           T b[rem];
 #pragma unroll
           for (int j = 0; j < rem; ++j) b[j] = B[(full + j) * 32];
-          mma_tiles<PR>(*reinterpret_cast<float(*)[rem][4]>(&r[full]),
-                        *reinterpret_cast<float(*)[rem][4]>(&e[full]), u, b);
+          mma_tiles<PD>(*reinterpret_cast<float(*)[rem][4]>(&r[full]), u, b);
         }
       };
 #pragma unroll 1
@@ -296,7 +320,7 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
       for (int j = 0; j < NB; ++j)
 #pragma unroll
-        for (int v = 0; v < 4; ++v) r[j][v] = (r[j][v] + e[j][v]) * (v < 2 ? ia : ib);
+        for (int v = 0; v < 4; ++v) r[j][v] *= v < 2 ? ia : ib;
 #pragma unroll
       for (int k = 0; k < KP; ++k) {
         const int n = 16 * k + 4 * t;
@@ -358,7 +382,8 @@ __global__ void __launch_bounds__(256, 1)
   constexpr int Np = C::Np, Nfp = C::Nfp, NB = C::NB, KP = C::KP, KT = C::KT, EW = C::EW, V = C::V;
   constexpr int FB = C::FB, FP = C::FP, FT = C::FT;
   extern __shared__ __align__(16) uint32_t smem_w[];
-  int *sRed = reinterpret_cast<int *>(smem_w + C::OPS_SURF);
+  uint32_t *rest = smem_w + C::OPS_SURF;
+  int *sRed = reinterpret_cast<int *>(rest + C::OPS_SURF / 4);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   float *sF = reinterpret_cast<float *>(sRed + 4) + warp * C::FLUX;
   const int nt = (K + 15) / 16;
@@ -371,15 +396,16 @@ __global__ void __launch_bounds__(256, 1)
 #pragma unroll
   for (int f = 0; f < 4; ++f) {
     const float *L = LIFT + (size_t)f * Nfp * Np;
-    split_tiles<true>(smem_w + f * FP * NB * 128, L, Np, Nfp, Np, Nfp, NB, 0, FP, false, pow2_field(of));
+    split_tiles<true>(smem_w, rest, f * FP * NB * 128, L, Np, Nfp, Np, Nfp, NB, 0, FP, pow2_field(of));
     if constexpr (FT)
-      split_tiles<false>(smem_w + 4 * FP * NB * 128 + f * NB * 64, L, Np, Nfp, Np, Nfp, NB, 2 * FP, 1,
-                         false, pow2_field(of));
+      split_tiles<false>(smem_w, rest, 4 * FP * NB * 128 + f * NB * 64, L, Np, Nfp, Np, Nfp, NB, 2 * FP, 1,
+                         pow2_field(of));
   }
   __syncthreads();
   const float iL = pow2_field(254 - of);
-  const uint4 *oL = reinterpret_cast<const uint4 *>(smem_w) + lane;
-  const uint2 *oLt = reinterpret_cast<const uint2 *>(smem_w + 4 * FP * NB * 128) + lane;
+  const uint4 *ops = reinterpret_cast<const uint4 *>(smem_w);
+  const Ops<uint4, 4, false> oL(ops, rest, 0, lane);
+  const Ops<uint2, 4, false> oLt(ops, rest, 4 * FP * NB * 32, lane);
   for (int it = first_tile(nt, C::W, warp); it < nt; it += gridDim.x * C::W) {
     const int k0 = it * 16, ka = min(k0 + g, K - 1), kb = min(k0 + g + 8, K - 1);
     const bool va = k0 + g < K, vb = k0 + g + 8 < K;
@@ -430,37 +456,29 @@ __global__ void __launch_bounds__(256, 1)
     }
     // lifted fluxes of block j: four fields
     auto block = [&](int j, float (&r)[4][4]) {
-      // corrections of all steps first, then the leading products
       float L[4][4] = {};
+      auto step = [&](const auto &x, const auto (&b)[4]) {
+        float t4[4][4];
+#pragma unroll
+        for (int p = 0; p < kProducts; ++p)
+#pragma unroll
+          for (int f = 0; f < 4; ++f) mma_step<4>(t4[f], x(f), b[f], p);
+#pragma unroll
+        for (int f = 0; f < 4; ++f) add4(L[f], t4[f]);
+      };
 #pragma unroll
       for (int k = 0; k < FP; ++k) {
-        uint4 b[4];
+        OpTile<uint4> b[4];
 #pragma unroll
         for (int f = 0; f < 4; ++f) b[f] = oL[((f * FP + k) * NB + j) * 32];
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], ff[f][k].l, b[f], true);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], ff[f][k].h, b[f], true);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], ff[f][k].l, b[f], false);
+        step([&](int f) { return ff[f][k]; }, b);
       }
       if constexpr (FT) {
-        uint2 b[4];
+        OpTile<uint2> b[4];
 #pragma unroll
         for (int f = 0; f < 4; ++f) b[f] = oLt[(f * NB + j) * 32];
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], f8[f].l, b[f], true);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], f8[f].h, b[f], true);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], f8[f].l, b[f], false);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], f8[f].h, b[f], false);
+        step([&](int f) { return f8[f]; }, b);
       }
-#pragma unroll
-      for (int k = 0; k < FP; ++k)
-#pragma unroll
-        for (int f = 0; f < 4; ++f) mma_hl(L[f], ff[f][k].h, oL[((f * FP + k) * NB + j) * 32], false);
 #pragma unroll
       for (int x = 0; x < 4; ++x)
 #pragma unroll
@@ -522,8 +540,9 @@ __global__ void __launch_bounds__(RefCfg<N>::TU, 1)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int grp = warp / GW, w = warp - grp * GW;
   // operators: Vq [chunk][KP][2], its k8 tails [chunk][2], Pq [chunk][NB]
-  uint32_t *wVt = smem_w + nch * KP * 2 * 128, *wP = wVt + nch * KT * 2 * 64;
-  int *sRed = reinterpret_cast<int *>(wP + nch * NB * 128);
+  const int aVt = nch * KP * 2 * 128, aP = aVt + nch * KT * 2 * 64, aM = aP + nch * NB * 128;  // words
+  uint32_t *rest = smem_w + aM;
+  int *sRed = reinterpret_cast<int *>(rest + aM / 4);
   float *scr = reinterpret_cast<float *>(sRed + 4) + grp * C::UPD;
   const int nt = (K + 15) / 16;
   if (threadIdx.x < 2) sRed[threadIdx.x] = 0;
@@ -535,24 +554,20 @@ __global__ void __launch_bounds__(RefCfg<N>::TU, 1)
 #pragma unroll 4
   for (int i = threadIdx.x; i < nch * 2 * KP * 32; i += blockDim.x) {
     const int tl = i >> 5, l = i & 31, h = tl & 1, k = (tl >> 1) % (KP > 0 ? KP : 1), c = (tl >> 1) / (KP > 0 ? KP : 1);
-    const int r = slot_index(16 * nch, 2 * c + h, l >> 2), s = 2 * (l & 3);
-    auto at = [&](int b, int slot) {
+    const int r = slot_index(16 * nch, 2 * c + h, l >> 2);
+    split_tile<true>(smem_w, rest, i, k, 2 * (l & 3), pow2_field(ov), [&](int b, int slot) {
       const int col = slot_index(Np, b, slot);
       return r < Nq && col < Np ? __ldg(Vq + r + (size_t)col * Nq) : 0.f;
-    };
-    uint32_t h0, h1, l0, l1;
-    split2(make_float2(at(2 * k, s), at(2 * k, s + 1)), both(pow2_field(ov)), h0, l0);
-    split2(make_float2(at(2 * k + 1, s), at(2 * k + 1, s + 1)), both(pow2_field(ov)), h1, l1);
-    reinterpret_cast<uint4 *>(smem_w)[i] = make_uint4(h0, h1, l0, l1);
+    });
   }
   if constexpr (KT)
-    split_tiles<false>(wVt, Vq, Nq, Np, 16 * nch, Np, 2 * nch, 2 * KP, 1, false, pow2_field(ov));
-  split_tiles<true>(wP, Pq, Np, Nq, Np, 16 * nch, NB, 0, nch, false, pow2_field(op));
+    split_tiles<false>(smem_w, rest, aVt, Vq, Nq, Np, 16 * nch, Np, 2 * nch, 2 * KP, 1, pow2_field(ov));
+  split_tiles<true>(smem_w, rest, aP, Pq, Np, Nq, Np, 16 * nch, NB, 0, nch, pow2_field(op));
   __syncthreads();
   const float iV = pow2_field(254 - ov), iP = pow2_field(254 - op);
-  const uint4 *oV = reinterpret_cast<const uint4 *>(smem_w) + lane;
-  const uint2 *oVt = reinterpret_cast<const uint2 *>(wVt) + lane;
-  const uint4 *oP = reinterpret_cast<const uint4 *>(wP) + lane;
+  const uint4 *ops = reinterpret_cast<const uint4 *>(smem_w);
+  const Ops<uint4, PR, false> oV(ops, rest, 0, lane), oP(ops, rest, aP / 4, lane);
+  const Ops<uint2, PR, false> oVt(ops, rest, aVt / 4, lane);
   uint4 *sA = reinterpret_cast<uint4 *>(scr);                 // split rhs, four fields
   uint4 *sW = reinterpret_cast<uint4 *>(scr + 16 * AS);       // split point values [RC][4]
   float4 *sMax = reinterpret_cast<float4 *>(scr + 16 * AS + RC * 1024);  // [GW][16]
@@ -620,21 +635,21 @@ __global__ void __launch_bounds__(RefCfg<N>::TU, 1)
             wj[h][q] = i < Nq ? 1.f / __ldg(Jq + at) : 0.f;
             wc[h][q] = i < Nq ? __ldg(c2q + at) : 0.f;
           }
-        float v[4][2][4] = {}, e[4][2][4] = {};
+        float v[4][2][4] = {};
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
-          const uint4 b[2] = {oV[((c * KP + k) * 2) * 32], oV[((c * KP + k) * 2 + 1) * 32]};
+          const OpTile<uint4> b[2] = {oV[((c * KP + k) * 2) * 32], oV[((c * KP + k) * 2 + 1) * 32]};
 #pragma unroll
           for (int x = 0; x < 4; x += 2)
-            mma_pair2<PR, 2>(v[x], e[x], get_frag(sA + x * AS, k, lane), b, v[x + 1], e[x + 1],
-                             get_frag(sA + (x + 1) * AS, k, lane), b);
+            mma_pair2<PR, PR>(v[x], get_frag(sA + x * AS, k, lane), b, v[x + 1],
+                          get_frag(sA + (x + 1) * AS, k, lane), b);
         }
         if constexpr (KT) {
-          const uint2 b[2] = {oVt[(c * 2) * 32], oVt[(c * 2 + 1) * 32]};
+          const OpTile<uint2> b[2] = {oVt[(c * 2) * 32], oVt[(c * 2 + 1) * 32]};
 #pragma unroll
           for (int x = 0; x < 4; x += 2)
-            mma_pair2<PR, 2>(v[x], e[x], get_frag8(sA + x * AS, KP, lane), b, v[x + 1], e[x + 1],
-                             get_frag8(sA + (x + 1) * AS, KP, lane), b);
+            mma_pair2<PR, PR>(v[x], get_frag8(sA + x * AS, KP, lane), b, v[x + 1],
+                          get_frag8(sA + (x + 1) * AS, KP, lane), b);
         }
         float4 inva, invb;
         float *ia = &inva.x, *ib = &invb.x;
@@ -646,7 +661,7 @@ __global__ void __launch_bounds__(RefCfg<N>::TU, 1)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const int i = q / 2, j = 2 * h + q % 2;
-              float z = (v[x][i][j] + e[x][i][j]) * (pow2_field(254 - sf[x][h]) * iV) * wj[h][q];
+              float z = v[x][i][j] * (pow2_field(254 - sf[x][h]) * iV) * wj[h][q];
               if (x == 0) z *= wc[h][q];
               y[h][q] = z;
               mm[h] = fmaxf(mm[h], fabsf(z));
@@ -664,22 +679,21 @@ __global__ void __launch_bounds__(RefCfg<N>::TU, 1)
 #pragma unroll 1
       for (int c = c0; c < cend && mine; ++c) {
         const uint4 *W = sW + (c - c0) * 4 * 64;
-        const uint4 b[2] = {oP[(c * NB + 2 * w) * 32],
-                            pair ? oP[(c * NB + 2 * w + 1) * 32] : make_uint4(0, 0, 0, 0)};
+        const OpTile<uint4> b[2] = {oP[(c * NB + 2 * w) * 32], oP[(c * NB + 2 * w + (pair ? 1 : 0)) * 32]};
         const float4 va4 = sInv[(c - c0) * 16 + g], vb4 = sInv[(c - c0) * 16 + g + 8];
         const float ia[4] = {va4.x, va4.y, va4.z, va4.w}, ib[4] = {vb4.x, vb4.y, vb4.z, vb4.w};
-        float o[4][2][4] = {}, oe[4][2][4] = {};
+        float o[4][2][4] = {};
 #pragma unroll
         for (int x = 0; x < 4; x += 2)
-          mma_pair2<PR, 2>(o[x], oe[x], get_frag(W + x * 64, 0, lane), b, o[x + 1], oe[x + 1],
-                           get_frag(W + (x + 1) * 64, 0, lane), b);
+          mma_pair2<PR, PR>(o[x], get_frag(W + x * 64, 0, lane), b, o[x + 1],
+                        get_frag(W + (x + 1) * 64, 0, lane), b);
 #pragma unroll
         for (int x = 0; x < 4; ++x)
 #pragma unroll
           for (int i = 0; i < 2; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              r[x][i][j] = fmaf(o[x][i][j] + oe[x][i][j], j < 2 ? ia[x] : ib[x], r[x][i][j]);
+              r[x][i][j] = fmaf(o[x][i][j], j < 2 ? ia[x] : ib[x], r[x][i][j]);
       }
     }
     const float2 fa2 = both(fa), fd2 = both(fdt), fb2 = both(fb);
@@ -723,7 +737,7 @@ template <int N>
 static bbw_status ref_volume_n(int K, const float *vgeo, const float *Dr, const float *Ds,
                                const float *Dt, const float *Q, float *rhsQ, cudaStream_t st) {
   using C = RefCfg<N>;
-  const int sm = C::OPS_VOL * 4 + 16;
+  const int sm = C::OPS_VOL * 5 + 16;
   const bbw_status s = ensure_smem_limit(k_rk_volume_mma<N>, sm, "rk_volume attribute");
   if (s != BBW_OK) return s;
   k_rk_volume_mma<N><<<ref_grid(K), 256, sm, st>>>(K, vgeo, Dr, Ds, Dt, Q, rhsQ);
@@ -734,7 +748,7 @@ template <int N>
 static bbw_status ref_surface_n(int K, int bc, const float *fgeo, const int *Fmask, const int *vmapP,
                                 const float *LIFT, const float *Q, float *rhsQ, cudaStream_t st) {
   using C = RefCfg<N>;
-  const int sm = C::OPS_SURF * 4 + 16 + C::W * C::FLUX * 4;
+  const int sm = C::OPS_SURF * 5 + 16 + C::W * C::FLUX * 4;
   const bbw_status s = ensure_smem_limit(k_rk_surface_mma<N>, sm, "rk_surface attribute");
   if (s != BBW_OK) return s;
   k_rk_surface_mma<N><<<ref_grid(K), 256, sm, st>>>(K, bc, fgeo, Fmask, vmapP, LIFT, Q, rhsQ);
@@ -744,7 +758,7 @@ static bbw_status ref_surface_n(int K, int bc, const float *fgeo, const int *Fma
 template <int N>
 static size_t ref_update_smem(int Nq) {
   using C = RefCfg<N>;
-  return C::ops_upd(Nq) * 4 + 16 + (size_t)C::NG * C::UPD * 4;
+  return C::ops_upd(Nq) * 5 + 16 + (size_t)C::NG * C::UPD * 4;
 }
 
 template <int N>

@@ -10,9 +10,16 @@
 // the chain of dependent phases bounds them, not the tensor rate.
 //
 // FP32 values x are split into FP16 pairs x s = hi + lo with a power of two s
-// per element and operand, so each element keeps its own dynamic range; the
-// pair holds 23 bits.  With four products (hi hi, hi lo, lo hi, lo lo) the
-// contraction error is that of FP32 sums; the split-FP16 form uses three.
+// per element and operand, so each element keeps its own dynamic range.  A pair
+// holds 23 bits: one short of FP32.  For the operand that is a rounding that
+// changes from stage to stage; for an operator it would be the same error in
+// every stage, which a time loop adds up, so operators keep a third part (the
+// rest, a byte of three significant bits: 26 bits in all).  Likewise the matrix
+// unit's rounding toward zero, see mma_step.  Error after 100 stages over the
+// CUDA-core stage's, pairs alone and summed in one accumulator / this form
+// (relative L2 against 64 bits, mean of 14 smooth states): N = 2 1.13 / 0.97, N = 4
+// 1.12 / 1.02, N = 5 1.28 / 1.01, BB 1.32 / 0.97, N = 6 1.32 / 1.01, each to 2 %; of one
+// right-hand side 0.8 .. 1.1.  The split-FP16 form has no rest and takes three products.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -28,7 +35,7 @@ namespace bbw {
 struct WarpParams {
   int K, K0, Kc, Nq, Nq16, bc, pat_off, table_ints, bs, ws, nt32;
   int nit, ntile, step_shot, step_tile;  // items; tiles per shot; a group's stride in both
-  int oDt, oL, oLt, oV, oVt, oP, ops_n;  // operator offsets and size in uint4
+  int oDt, oL, oLt, oV, oVt, oP, oM, ops_n;  // operator offsets and size in uint4
   float fa, fb, fdt, cstage;
   float iD, iL, iV, iP, vnorm;      // inverse operator scales, max row sum of |Vq|
   const float *__restrict__ Qin;
@@ -64,6 +71,31 @@ __device__ __forceinline__ void mma8(float (&c)[4], uint32_t a0, uint32_t a1, ui
       : "r"(a0), "r"(a1), "r"(b0));
 }
 
+// the same with nothing to add to
+__device__ __forceinline__ void mma16_set(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
+                                          uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+      "{%8,%9}, {%10,%10,%10,%10};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+__device__ __forceinline__ void mma8_set(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%7,%7,%7,%7};\n"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(b0), "f"(0.f));
+}
+
+// c += s, rounded to nearest
+__device__ __forceinline__ void add4(float (&c)[4], const float (&s)[4]) {
+  const float2 a = __fadd2_rn(make_float2(c[0], c[1]), make_float2(s[0], s[1]));
+  const float2 b = __fadd2_rn(make_float2(c[2], c[3]), make_float2(s[2], s[3]));
+  c[0] = a.x, c[1] = a.y, c[2] = b.x, c[3] = b.y;
+}
+
 // A operand of one k16 step: FP16 pairs of 16 elements x 16 columns.  Lane
 // l holds elements l/4 (indices 0, 2) and l/4 + 8 (1, 3) at columns
 // 4 (l%4) + {0, 1} (indices 0, 1) and + {2, 3}: the operators are packed with
@@ -74,6 +106,76 @@ struct Frag {
 struct Frag8 {  // a k8 step: columns 2 (l%4) + {0, 1}
   uint32_t h[2], l[2];
 };
+
+// Operator tile of a k16 (W = uint4) or k8 step (uint2): the lane's hi and lo
+// words, and the bytes of the rest (four-product forms)
+template <class W>
+struct OpTile {
+  W w;
+  uint32_t m;
+};
+// Tiles in memory; the rests are a plane of their own, a byte per four of the
+// words.  GW, GM: words, rests in global memory (read-only path), else in shared.
+template <class W, int PR, bool GW, bool GM = GW>
+struct Ops {
+  using M = std::conditional_t<sizeof(W) == 16, uint32_t, uint16_t>;
+  const W *w;
+  const M *m;
+  // at: uint4 offset of the lane's first tile in the words at ops
+  __device__ __forceinline__ Ops(const uint4 *ops, const void *rests, int at, int lane)
+      : w(reinterpret_cast<const W *>(ops + at) + lane),
+        m(reinterpret_cast<const M *>(rests) + at * (int)(16 / sizeof(W)) + lane) {}
+  __device__ __forceinline__ Ops(const W *a, const M *b) : w(a), m(b) {}
+  __device__ __forceinline__ Ops operator+(int i) const { return Ops(w + i, m + i); }
+  __device__ __forceinline__ OpTile<W> operator[](int i) const {
+    OpTile<W> t;
+    if constexpr (GW) t.w = __ldg(w + i);
+    else t.w = w[i];
+    if constexpr (PR < 4) t.m = 0;
+    else if constexpr (GM) t.m = __ldg(m + i);
+    else t.m = m[i];
+    return t;
+  }
+};
+// two bytes of the rest as FP16 pairs
+__device__ __forceinline__ uint32_t rest_lo(uint32_t m) { return __byte_perm(m, 0, 0x1404); }
+__device__ __forceinline__ uint32_t rest_hi(uint32_t m) { return __byte_perm(m, 0, 0x3424); }
+
+// One k step of a contraction is summed from zero and added to the result on
+// the CUDA cores (add4).  The matrix unit rounds its sums toward zero: a chain of
+// steps in one accumulator loses half an ulp of the running sum at every step,
+// always the same way.  One such rounding per step is left, and the operators
+// are packed larger by its mean (kRoundingBias).  us per stage against one
+// accumulator, N = 5, K = 196608: 411 -> 429; N = 7, K = 24576: 177 -> 207.
+//
+// Product p of one step, from zero or onto s, smallest first: the operand's hi
+// with the operator's rest, lo with lo, hi with lo, lo with hi, hi with hi.  PR = 5:
+// all; 4: without lo with lo; 3: the last three.  A k8 step takes two of them in
+// one k16 product, which costs no more, so there 4 is 5.
+constexpr int kProducts = 5;
+template <int PR>
+__device__ __forceinline__ void mma_step(float (&s)[4], const Frag &x, const OpTile<uint4> &b, int p) {
+  if constexpr (PR >= 4) {
+    if (p == 0) mma16_set(s, x.h, rest_lo(b.m), rest_hi(b.m));
+    if (p == 1 && PR == 5) mma16(s, x.l, b.w.z, b.w.w);
+    if (p == 2) mma16(s, x.h, b.w.z, b.w.w);
+  } else if (p == 2) {
+    mma16_set(s, x.h, b.w.z, b.w.w);
+  }
+  if (p == 3) mma16(s, x.l, b.w.x, b.w.y);
+  if (p == 4) mma16(s, x.h, b.w.x, b.w.y);
+}
+template <int PR>
+__device__ __forceinline__ void mma_step(float (&s)[4], const Frag8 &x, const OpTile<uint2> &b, int p) {
+  const uint32_t hl[4] = {x.h[0], x.h[1], x.l[0], x.l[1]};
+  if constexpr (PR >= 4) {
+    if (p == 0) mma16_set(s, hl, rest_lo(b.m), b.w.y);
+    if (p == 2) mma16(s, hl, b.w.y, b.w.x);
+  } else if (p == 2) {
+    mma16_set(s, hl, b.w.y, b.w.x);
+  }
+  if (p == 4) mma8(s, x.h[0], x.h[1], b.w.x);
+}
 
 // x s = hi + lo for two values; s2 = (s, s)
 __device__ __forceinline__ void split2(float2 x, float2 s2, uint32_t &h, uint32_t &l) {
@@ -105,77 +207,43 @@ __device__ __forceinline__ void split_frag(Frag8 &f, const float2 a, const float
   split2(b, both(cb), f.h[1], f.l[1]);
 }
 
-// leading products into c, corrections into e (the same array, or its own so
-// that the small terms add up before they meet the large ones: the matrix
-// unit's sums round toward zero, so fewer large sums leave less bias)
-template <int PR>
-__device__ __forceinline__ void mma_tile(float (&c)[4], float (&e)[4], const Frag &x,
-                                         const uint4 b) {
-  mma16(c, x.h, b.x, b.y);
-  mma16(e, x.h, b.z, b.w);
-  mma16(e, x.l, b.x, b.y);
-  if constexpr (PR == 4) mma16(e, x.l, b.z, b.w);
-}
-template <int PR, int M>
-__device__ __forceinline__ void mma_tiles(float (&c)[M][4], float (&e)[M][4], const Frag &x,
-                                          const uint4 (&b)[M]) {
-#pragma unroll
-  for (int i = 0; i < M; ++i) mma16(c[i], x.h, b[i].x, b[i].y);
-#pragma unroll
-  for (int i = 0; i < M; ++i) mma16(e[i], x.h, b[i].z, b[i].w);
-#pragma unroll
-  for (int i = 0; i < M; ++i) mma16(e[i], x.l, b[i].x, b[i].y);
-  if constexpr (PR == 4) {
-#pragma unroll
-    for (int i = 0; i < M; ++i) mma16(e[i], x.l, b[i].z, b[i].w);
-  }
-}
-template <int PR, int M>
-__device__ __forceinline__ void mma_tiles(float (&c)[M][4], float (&e)[M][4], const Frag8 &x,
-                                          const uint2 (&b)[M]) {
-#pragma unroll
-  for (int i = 0; i < M; ++i) mma8(c[i], x.h[0], x.h[1], b[i].x);
-#pragma unroll
-  for (int i = 0; i < M; ++i) mma8(e[i], x.h[0], x.h[1], b[i].y);
-#pragma unroll
-  for (int i = 0; i < M; ++i) mma8(e[i], x.l[0], x.l[1], b[i].x);
-  if constexpr (PR == 4) {
-#pragma unroll
-    for (int i = 0; i < M; ++i) mma8(e[i], x.l[0], x.l[1], b[i].y);
-  }
-}
-
-__device__ __forceinline__ void mma_hl(float (&c)[4], const uint32_t (&a)[4], const uint4 b, bool lo) {
-  if (lo) mma16(c, a, b.z, b.w);
-  else mma16(c, a, b.x, b.y);
-}
-__device__ __forceinline__ void mma_hl(float (&c)[4], const uint32_t (&a)[2], const uint2 b, bool lo) {
-  mma8(c, a[0], a[1], lo ? b.y : b.x);
-}
-// two products x b and y bb, interleaved: an accumulator is used again only
-// after the 21 cycles that a product takes
+// c += x b for M operator tiles; an accumulator is used again only after the
+// other tiles' product (a product takes 21 cycles, 8 of them issuing)
 template <int PR, int M, class F, class T>
-__device__ __forceinline__ void mma_pair2(float (&c)[M][4], float (&e)[M][4], const F &x,
-                                          const T (&b)[M], float (&cc)[M][4], float (&ee)[M][4],
-                                          const F &y, const T (&bb)[M]) {
+__device__ __forceinline__ void mma_tiles(float (&c)[M][4], const F &x, const T (&b)[M]) {
+  float s[M][4];
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(c[i], x.h, b[i], false);
+  for (int p = 0; p < kProducts; ++p)
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(cc[i], y.h, bb[i], false);
+    for (int i = 0; i < M; ++i) mma_step<PR>(s[i], x, b[i], p);
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(e[i], x.h, b[i], true);
+  for (int i = 0; i < M; ++i) add4(c[i], s[i]);
+}
+// the first of two accumulators as an array of one
+__device__ __forceinline__ float (&one(float (&c)[2][4]))[1][4] {
+  return *reinterpret_cast<float(*)[1][4]>(&c[0]);
+}
+template <int PR, class F, class T>
+__device__ __forceinline__ void mma_tile(float (&c)[4], const F &x, const T b) {
+  const T b1[1] = {b};
+  mma_tiles<PR>(*reinterpret_cast<float(*)[1][4]>(&c), x, b1);
+}
+// two operands' products x b and y bb, interleaved
+template <int PX, int PY, int M, class F, class T>
+__device__ __forceinline__ void mma_pair2(float (&c)[M][4], const F &x, const T (&b)[M],
+                                          float (&cc)[M][4], const F &y, const T (&bb)[M]) {
+  float s[M][4], ss[M][4];
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.h, bb[i], true);
+  for (int p = 0; p < kProducts; ++p) {
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(e[i], x.l, b[i], false);
+    for (int i = 0; i < M; ++i) mma_step<PX>(s[i], x, b[i], p);
 #pragma unroll
-  for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, bb[i], false);
-  if constexpr (PR == 4) {
-#pragma unroll
-    for (int i = 0; i < M; ++i) mma_hl(e[i], x.l, b[i], true);
-#pragma unroll
-    for (int i = 0; i < M; ++i) mma_hl(ee[i], y.l, bb[i], true);
+    for (int i = 0; i < M; ++i) mma_step<PY>(ss[i], y, bb[i], p);
   }
+#pragma unroll
+  for (int i = 0; i < M; ++i) add4(c[i], s[i]);
+#pragma unroll
+  for (int i = 0; i < M; ++i) add4(cc[i], ss[i]);
 }
 
 // power of two that brings a maximum m below 2^15, as an exponent field; the
@@ -342,6 +410,7 @@ inline WarpParams warp_params(const WarpPlan &pl, const float *Qin, float *Qout,
   P.pat_off = pl.pat_off, P.table_ints = pl.table_ints, P.nt32 = (pl.K + 31) / 32;
   P.Nq16 = (pl.Nq + 15) / 16 * 16;
   P.oDt = pl.oDt, P.oL = pl.oL, P.oLt = pl.oLt, P.oV = pl.oV, P.oVt = pl.oVt, P.oP = pl.oP;
+  P.oM = pl.oM;
   P.ops_n = pl.ops_n;
   P.fa = fa, P.fb = fb, P.fdt = fdt, P.cstage = cstage;
   P.iD = pl.iD, P.iL = pl.iL, P.iV = pl.iV, P.iP = pl.iP, P.vnorm = pl.vnorm;

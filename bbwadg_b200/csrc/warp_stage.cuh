@@ -126,11 +126,13 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
   if constexpr (FB * 8 > Nfp)  // flux columns past Nfp meet zero operator columns
     for (int i = lane; i < C::FLUX; i += 32) sF[i] = 0.f;
   const uint4 *ops = OPS ? sOps : P.ops;
-  const uint4 *oD = ops + lane, *oL = ops + P.oL + lane, *oV = ops + P.oV + lane,
-              *oP = ops + P.oP + lane;
-  const uint2 *oDt = reinterpret_cast<const uint2 *>(ops + P.oDt) + lane,
-              *oLt = reinterpret_cast<const uint2 *>(ops + P.oLt) + lane,
-              *oVt = reinterpret_cast<const uint2 *>(ops + P.oVt) + lane;
+  constexpr int PD = PR == 4 ? 5 : PR;  // derivatives: large terms cancel
+  using O16 = Ops<uint4, PR, !OPS>;
+  using O8 = Ops<uint2, PR, !OPS>;
+  const void *rests = ops + P.oM;
+  const O16 oD(ops, rests, 0, lane), oL(ops, rests, P.oL, lane), oV(ops, rests, P.oV, lane),
+      oP(ops, rests, P.oP, lane);
+  const O8 oDt(ops, rests, P.oDt, lane), oLt(ops, rests, P.oLt, lane), oVt(ops, rests, P.oVt, lane);
   const int klast = P.Kc - 1;
   const size_t shot_stride = (size_t)P.K * EW;
   const int step = gridDim.x * C::W;
@@ -292,69 +294,46 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
       // one block of eight nodes: rhs of u, v, w and the lifted part of rhs_p
       auto block = [&](int j, float (&rv)[3][4], float (&rp)[4]) {
         {
-          float d[3][4] = {}, e[3][4] = {};
+          float d[3][4] = {};
 #pragma unroll
           for (int k = 0; k < KP; ++k) {
-            uint4 b[3];
+            OpTile<uint4> b[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) b[c] = oD[((c * KP + k) * NB + j) * 32];
-            mma_tiles<PR>(d, e, fp[k], b);
+            mma_tiles<PD>(d, fp[k], b);
           }
           if constexpr (KT) {
-            uint2 b[3];
+            OpTile<uint2> b[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) b[c] = oDt[(c * NB + j) * 32];
-            mma_tiles<PR>(d, e, fp8, b);
+            mma_tiles<PD>(d, fp8, b);
           }
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             const bool lo = v < 2;
             const float *G = lo ? Ha : Hb;
-            const float a = d[0][v] + e[0][v], b = d[1][v] + e[1][v], c = d[2][v] + e[2][v];
+            const float a = d[0][v], b = d[1][v], c = d[2][v];
 #pragma unroll
             for (int x = 0; x < 3; ++x) rv[x][v] = G[x] * a + G[3 + x] * b + G[6 + x] * c;
           }
         }
-        // corrections of all steps first, then the leading products
-        float L[4][4] = {};
+        // a face's nodes are one step, k16 or k8 (N <= 4)
+        static_assert(FP + FT == 1, "one step per face");
+        float L[4][4];
         {
-          uint4 b[FP > 0 ? FP : 1][4];
-          uint2 c[4];
+          OpTile<std::conditional_t<FT != 0, uint2, uint4>> b[4];
 #pragma unroll
-          for (int k = 0; k < FP; ++k)
-#pragma unroll
-            for (int f = 0; f < 4; ++f) b[k][f] = oL[((f * FP + k) * NB + j) * 32];
-          if constexpr (FT) {
-#pragma unroll
-            for (int f = 0; f < 4; ++f) c[f] = oLt[(f * NB + j) * 32];
+          for (int f = 0; f < 4; ++f) {
+            if constexpr (FT) b[f] = oLt[(f * NB + j) * 32];
+            else b[f] = oL[(f * NB + j) * 32];
           }
 #pragma unroll
-          for (int k = 0; k < FP; ++k) {
-            if constexpr (PR == 4) {
+          for (int p = 0; p < kProducts; ++p)
 #pragma unroll
-              for (int f = 0; f < 4; ++f) mma16(L[f], ff[f][k].l, b[k][f].z, b[k][f].w);
+            for (int f = 0; f < 4; ++f) {
+              if constexpr (FT) mma_step<PR>(L[f], f8[f], b[f], p);
+              else mma_step<PR>(L[f], ff[f][0], b[f], p);
             }
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mma16(L[f], ff[f][k].h, b[k][f].z, b[k][f].w);
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mma16(L[f], ff[f][k].l, b[k][f].x, b[k][f].y);
-          }
-          if constexpr (FT) {
-            if constexpr (PR == 4) {
-#pragma unroll
-              for (int f = 0; f < 4; ++f) mma8(L[f], f8[f].l[0], f8[f].l[1], c[f].y);
-            }
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mma8(L[f], f8[f].h[0], f8[f].h[1], c[f].y);
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mma8(L[f], f8[f].l[0], f8[f].l[1], c[f].x);
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mma8(L[f], f8[f].h[0], f8[f].h[1], c[f].x);
-          }
-#pragma unroll
-          for (int k = 0; k < FP; ++k)
-#pragma unroll
-            for (int f = 0; f < 4; ++f) mma16(L[f], ff[f][k].h, b[k][f].x, b[k][f].y);
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
@@ -440,7 +419,6 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
     // ---- 3. divergence of the contravariant velocities
     float r[NB][4];
     {
-      float e[NB][4];
       // twice the bound: its own rounding cannot bring a value to 2^16
       const int sa = scale_field(2.f * Ma), sb = scale_field(2.f * Mb);
       const float ca = pow2_field(sa), cb = pow2_field(sb);
@@ -448,28 +426,26 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
       for (int j = 0; j < NB; ++j)
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          r[j][v] = e[j][v] = 0.f;
+          r[j][v] = 0.f;
         }
       // products of one operand step with the tiles b of all node blocks
-      auto accumulate = [&](const auto &u, const auto *B) {
-        using T = std::remove_const_t<std::remove_reference_t<decltype(*B)>>;
+      auto accumulate = [&](const auto &u, const auto B) {
+        using T = decltype(B[0]);
 #pragma unroll
         for (int j0 = 0; j0 < NB; j0 += 4) {
           constexpr int full = NB / 4 * 4, rem = NB % 4 ? NB % 4 : 4;
           if (j0 < full) {
             T b[4];
             float(&rr)[4][4] = *reinterpret_cast<float(*)[4][4]>(&r[j0]);
-            float(&ee)[4][4] = *reinterpret_cast<float(*)[4][4]>(&e[j0]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) b[j] = B[(j0 + j) * 32];
-            mma_tiles<PR>(rr, ee, u, b);
+            mma_tiles<PD>(rr, u, b);
           } else {
             T b[rem];
             float(&rr)[rem][4] = *reinterpret_cast<float(*)[rem][4]>(&r[j0]);
-            float(&ee)[rem][4] = *reinterpret_cast<float(*)[rem][4]>(&e[j0]);
 #pragma unroll
             for (int j = 0; j < rem; ++j) b[j] = B[(j0 + j) * 32];
-            mma_tiles<PR>(rr, ee, u, b);
+            mma_tiles<PD>(rr, u, b);
           }
         }
       };
@@ -516,7 +492,7 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
       auto finish = [&](int j, const float (&l)[4]) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          r[j][v] = fmaf(r[j][v] + e[j][v], v < 2 ? ia : ib, l[v]);
+          r[j][v] = fmaf(r[j][v], v < 2 ? ia : ib, l[v]);
         }
       };
 #pragma unroll
@@ -547,7 +523,7 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
 
     // ---- 4. WADG projection of rhs_p: 16 cubature points at a time through
     //         Vq, c2 and Pq
-    float o[NB][4], oe[NB][4];
+    float o[NB][4];
     float oia, oib;
     {
       Frag fr[KP > 0 ? KP : 1];
@@ -559,7 +535,7 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
         mb = fmaxf(mb, fmaxf(fabsf(r[j][2]), fabsf(r[j][3])));
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-          o[j][v] = oe[j][v] = 0.f;
+          o[j][v] = 0.f;
         }
       }
       ma = quad_max(ma), mb = quad_max(mb);
@@ -584,36 +560,16 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
       float4 za = __ldg(Ca), zb = __ldg(Cb);  // c2 at this chunk's points
 #pragma unroll 1
       for (int c = 0; c < nch; ++c) {
-        float v[6][4] = {};
+        float v[2][4] = {};
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
-          const uint4 b0 = oV[((c * KP + k) * 2) * 32], b1 = oV[((c * KP + k) * 2 + 1) * 32];
-          mma16(v[0], fr[k].h, b0.x, b0.y);
-          mma16(v[1], fr[k].h, b1.x, b1.y);
-          mma16(v[2], fr[k].h, b0.z, b0.w);
-          mma16(v[3], fr[k].h, b1.z, b1.w);
-          mma16(v[4], fr[k].l, b0.x, b0.y);
-          mma16(v[5], fr[k].l, b1.x, b1.y);
-          if constexpr (PR == 4) {
-            mma16(v[2], fr[k].l, b0.z, b0.w);
-            mma16(v[3], fr[k].l, b1.z, b1.w);
-          }
+          const OpTile<uint4> b[2] = {oV[((c * KP + k) * 2) * 32], oV[((c * KP + k) * 2 + 1) * 32]};
+          mma_tiles<PR>(v, fr[k], b);
         }
         if constexpr (KT) {
-          const uint2 b0 = oVt[(c * 2) * 32], b1 = oVt[(c * 2 + 1) * 32];
-          mma8(v[0], fr8.h[0], fr8.h[1], b0.x);
-          mma8(v[1], fr8.h[0], fr8.h[1], b1.x);
-          mma8(v[2], fr8.h[0], fr8.h[1], b0.y);
-          mma8(v[3], fr8.h[0], fr8.h[1], b1.y);
-          mma8(v[4], fr8.l[0], fr8.l[1], b0.x);
-          mma8(v[5], fr8.l[0], fr8.l[1], b1.x);
-          if constexpr (PR == 4) {
-            mma8(v[2], fr8.l[0], fr8.l[1], b0.y);
-            mma8(v[3], fr8.l[0], fr8.l[1], b1.y);
-          }
+          const OpTile<uint2> b[2] = {oVt[(c * 2) * 32], oVt[(c * 2 + 1) * 32]};
+          mma_tiles<PR>(v, fr8, b);
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[0][i] += v[2][i] + v[4][i], v[1][i] += v[3][i] + v[5][i];
         // points 16 c + 4 t + 0 .. 3 of the two rows
         const float4 xa = make_float4(v[0][0] * via * za.x, v[0][1] * via * za.y,
                                       v[1][0] * via * za.z, v[1][1] * via * za.w);
@@ -622,24 +578,22 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
         Frag w;
         split_frag(w, xa, xb, da, db);
         if (c + 1 < nch) za = __ldg(Ca + (c + 1) * 4), zb = __ldg(Cb + (c + 1) * 4);
-        const uint4 *B = oP + c * NB * 32;
+        const O16 B = oP + c * NB * 32;
 #pragma unroll
         for (int j0 = 0; j0 < NB; j0 += 4) {
           constexpr int full = NB / 4 * 4, rem = NB % 4 ? NB % 4 : 4;
           if (j0 < full) {
-            uint4 b[4];
+            OpTile<uint4> b[4];
             float(&oo)[4][4] = *reinterpret_cast<float(*)[4][4]>(&o[j0]);
-            float(&ee)[4][4] = *reinterpret_cast<float(*)[4][4]>(&oe[j0]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) b[j] = B[(j0 + j) * 32];
-            mma_tiles<PR>(oo, ee, w, b);
+            mma_tiles<PR>(oo, w, b);
           } else {
-            uint4 b[rem];
+            OpTile<uint4> b[rem];
             float(&oo)[rem][4] = *reinterpret_cast<float(*)[rem][4]>(&o[j0]);
-            float(&ee)[rem][4] = *reinterpret_cast<float(*)[rem][4]>(&oe[j0]);
 #pragma unroll
             for (int j = 0; j < rem; ++j) b[j] = B[(j0 + j) * 32];
-            mma_tiles<PR>(oo, ee, w, b);
+            mma_tiles<PR>(oo, w, b);
           }
         }
       }
@@ -648,7 +602,7 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
     for (int j = 0; j < NB; ++j)
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
-        o[j][v] = (o[j][v] + oe[j][v]) * (v < 2 ? oia : oib);
+        o[j][v] *= v < 2 ? oia : oib;
       }
 
     // ---- 5. sources

@@ -10,18 +10,29 @@
 
 namespace bbw {
 
+// What the matrix unit's rounding toward zero takes off a sum of products on
+// average, relative to it (half an ulp: 3.65e-8 measured over 10^6 sums of 16).
+// Operators are packed larger by this, so contractions are free of a mean error.
+constexpr double kRoundingBias = 3.65e-8;
+// top byte of FP16 bits, rounded: sign, five bits of exponent, three significant bits
+__host__ __device__ inline uint8_t rest_byte(uint16_t bits) { return (uint8_t)((bits + 0x80u) >> 8); }
+
 // which form of the stage a context runs (auto: stage_form's rule)
 enum WarpForm { WARP_AUTO = 0, WARP_SINGLE = 1, WARP_GROUP = 2 };
+// where the group form's operators are: all in L2, all in shared memory, or the
+// rests in shared memory and the words in L2
+enum OpsPlace { OPS_L2 = 0, OPS_SHARED = 1, OPS_RESTS = 2 };
 
 struct WarpPlan {
   bool single = false, group = false;  // forms this context's sizes allow
   int pinned = WARP_AUTO;              // form chosen by the autotuner or the caller
-  bool warp_ops = false, group_ops = false;  // operators staged in shared memory
-  int products = 4;      // products per split pair (4: FP32 contexts, 3: split FP16)
+  bool warp_ops = false;               // operators staged in shared memory
+  int group_ops = OPS_L2;
+  int products = 4;      // 4: FP32 contexts (with the rest), 3: split FP16
   int N = 0, K = 0, K0 = 0, Kc = 0, Nq = 0, bc = 0, S = 1, nsm = 148, max_ctas = 0;
   bool chained = false;  // launched right behind another stage kernel
   int pat_off = 0, table_ints = 0;
-  int oDt = 0, oL = 0, oLt = 0, oV = 0, oVt = 0, oP = 0, ops_n = 0;
+  int oDt = 0, oL = 0, oLt = 0, oV = 0, oVt = 0, oP = 0, oM = 0, ops_n = 0;
   float iD = 1.f, iL = 1.f, iV = 1.f, iP = 1.f, vnorm = 1.f;
   const float *geo = nullptr, *c2p = nullptr, *c2max = nullptr;
   const int *nbr = nullptr, *tables = nullptr;
@@ -32,11 +43,14 @@ struct WarpPlan {
   const double *time = nullptr;
 };
 
-// Operators as FP16 pairs in the fragment order of the stage's B operands.
+// Operators as FP16 pairs and a rest in the fragment order of the stage's B
+// operands.
 // Indices run in blocks of eight; a pair of blocks (16 nodes) interleaves so
 // that one lane holds four consecutive nodes, an odd last block is in order
 // (warp_node).  A k16 tile gives lane l (hi, hi, lo, lo) of operator row l/4
-// and column pairs 2(l%4) of the pair's two blocks; a k8 tile (hi, lo).
+// and column pairs 2(l%4) of the pair's two blocks; a k8 tile (hi, lo).  The rests
+// follow as a plane of their own in the same order, a byte per entry (at oM;
+// four-product plans only).
 // Order: D [3][KP][NB] and its k8 tiles [3][NB], LIFT [4][FP][NB] and [4][NB],
 // Vq [chunk][KP][2] and [chunk][2], Pq [chunk][NB].  Sets the offsets, inverse
 // scales and vnorm of the plan.
@@ -45,9 +59,13 @@ float split_scale(const float *const *A, int n, size_t len);
 // Tiles of one column-major nr x nc operator, appended to out: split_rows
 // with its rows in chunks of 16 ([chunk][k16 step][2], then the k8 tails [chunk][2]),
 // split_columns with its columns in chunks of 16 ([chunk][row block]).
-void split_rows(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off,
-                int &off_tail);
-void split_columns(std::vector<uint32_t> &out, const float *A, int nr, int nc, float s, int &off);
+struct SplitOps {
+  std::vector<uint32_t> w;            // hi and lo
+  std::vector<uint8_t> m;             // rest, one byte per four of w
+  std::vector<uint32_t> words() const;  // w, then m
+};
+void split_rows(SplitOps &out, const float *A, int nr, int nc, float s, int &off, int &off_tail);
+void split_columns(SplitOps &out, const float *A, int nr, int nc, float s, int &off);
 void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
                const std::vector<float> &Vq, const std::vector<float> &Pq,
                std::vector<uint32_t> &out);
