@@ -32,7 +32,7 @@ struct CurvedCfg {
   static constexpr int ROWS = 16 * EW + 8 * ODD, TILE = ROWS > 16 * AS ? ROWS : 16 * AS;
   static constexpr int RC = N <= 3 ? 2 : 4;                 // cubature chunks per round
   static constexpr int WF = RC * 6 * 256;                   // split point values of a round
-  static constexpr int MISC = GW * 64 + 4 * 16;             // maxima, face scales
+  static constexpr int MISC = GW * 64 + 2 * 4 * 16;         // maxima, two scales a face
   static int scratch(int FC) { return TILE + WF + MISC + 4 * FC * 4 * 256; }
 };
 
@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
   uint4 *sA = reinterpret_cast<uint4 *>(scr);               // split p, u, v, w; then split rhs
   uint4 *sW = reinterpret_cast<uint4 *>(scr + C::TILE);     // split point values
   float4 *sMax = reinterpret_cast<float4 *>(scr + C::TILE + C::WF);  // [GW][16]
-  float *sInv = scr + C::TILE + C::WF + GW * 64;            // [4][16] face scales
-  uint4 *sFc = reinterpret_cast<uint4 *>(sInv + 64);        // [4][FC][4] split fluxes
+  float *sInv = scr + C::TILE + C::WF + GW * 64;            // [4][2][16] inverse flux scales
+  uint4 *sFc = reinterpret_cast<uint4 *>(sInv + 128);       // [4][FC][4] split fluxes
   using O16 = Ops<uint4, PR, true>;
   using O8 = Ops<uint2, PR, true>;
   using T16 = OpTile<uint4>;
@@ -84,7 +84,9 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
     for (int f = w; f < 4; f += GW) {
       constexpr int NV = FP * 4 + FT * 2;
       float x[7][2][NV];
-      float m = 0.f, mb = 0.f;
+      // pressure jumps, velocity jumps and averages may differ in size by any
+      // factor (p ~ c u in the caller's units): a scale each
+      float m[3] = {0.f, 0.f, 0.f}, mb[3] = {0.f, 0.f, 0.f};
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int k = A.k_off + (h ? rb_ : ra_);
@@ -105,19 +107,25 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll
           for (int c = 0; c < 7; ++c) {
             if (!on) x[c][h][j] = 0.f;
-            if (h) mb = fmaxf(mb, fabsf(x[c][h][j]));
-            else m = fmaxf(m, fabsf(x[c][h][j]));
+            float &y = (h ? mb : m)[(c + 2) / 3];
+            y = fmaxf(y, fabsf(x[c][h][j]));
           }
         }
       }
-      m = quad_max(m), mb = quad_max(mb);
-      const int sa = scale_field(m), sb = scale_field(mb);
-      const float2 ca = both(pow2_field(sa)), cb = both(pow2_field(sb));
-      const float ia = pow2_field(254 - sa) * A.iF, ib = pow2_field(254 - sb) * A.iF;
+      float2 ca3[3], cb3[3];
+      float ia[3], ib[3];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        m[q] = quad_max(m[q]), mb[q] = quad_max(mb[q]);
+        const int sa = scale_field(m[q]), sb = scale_field(mb[q]);
+        ca3[q] = both(pow2_field(sa)), cb3[q] = both(pow2_field(sb));
+        ia[q] = pow2_field(254 - sa) * A.iF, ib[q] = pow2_field(254 - sb) * A.iF;
+      }
       Frag fx[7][FP > 0 ? FP : 1];
       Frag8 f8[7];
 #pragma unroll
       for (int c = 0; c < 7; ++c) {
+        const float2 ca = ca3[(c + 2) / 3], cb = cb3[(c + 2) / 3];
 #pragma unroll
         for (int s = 0; s < FP; ++s) {
           split2(make_float2(x[c][0][4 * s], x[c][0][4 * s + 1]), ca, fx[c][s].h[0], fx[c][s].l[0]);
@@ -130,13 +138,22 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
           split2(make_float2(x[c][1][4 * FP], x[c][1][4 * FP + 1]), cb, f8[c].h[1], f8[c].l[1]);
         }
       }
-      // |flux| <= 4 fnorm max|jump| sJ (|n| = 1); twice that against rounding
-      const int ga = scale_field(8.f * A.fnorm * m * __ldg(A.bound + (size_t)ra_ * 8 + 4 + f)),
-                gb = scale_field(8.f * A.fnorm * mb * __ldg(A.bound + (size_t)rb_ * 8 + 4 + f));
-      const float da = pow2_field(ga), db = pow2_field(gb);
-      if (t == 0) {
-        sInv[f * 16 + g] = pow2_field(254 - ga) * A.iP;
-        sInv[f * 16 + g + 8] = pow2_field(254 - gb) * A.iP;
+      // flux of p: |av - dp / 2| sJ <= fnorm (2 m[2] + m[0] / 2) sJ, of the velocities: |dp -
+      // du| / 2 sJ <= fnorm (m[0] / 2 + m[1]) sJ (|n| = 1); twice that against rounding
+      float da[2], db[2];
+      {
+        const float ka = 2.f * A.fnorm * __ldg(A.bound + (size_t)ra_ * 8 + 4 + f),
+                    kb = 2.f * A.fnorm * __ldg(A.bound + (size_t)rb_ * 8 + 4 + f);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int ga = scale_field(ka * (q ? m[0] + m[1] : 2.f * m[2] + m[0])),
+                    gb = scale_field(kb * (q ? mb[0] + mb[1] : 2.f * mb[2] + mb[0]));
+          da[q] = pow2_field(ga), db[q] = pow2_field(gb);
+          if (t == 0) {
+            sInv[(f * 2 + q) * 16 + g] = pow2_field(254 - ga) * A.iP;
+            sInv[(f * 2 + q) * 16 + g + 8] = pow2_field(254 - gb) * A.iP;
+          }
+        }
       }
 #pragma unroll 1
       for (int ch = 0; ch < A.FC; ++ch) {
@@ -181,13 +198,13 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
           const float4 n0 = __ldg(gp), n1 = __ldg(gp + 64), n2 = __ldg(gp + 128), n3 = __ldg(gp + 192);
           const float nx[4] = {n0.x, n0.y, n0.z, n0.w}, ny[4] = {n1.x, n1.y, n1.z, n1.w};
           const float nz[4] = {n2.x, n2.y, n2.z, n2.w}, sJ[4] = {n3.x, n3.y, n3.z, n3.w};
-          const float inv = h ? ib : ia;
+          const float *inv = h ? ib : ia;
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int i = q / 2, j = 2 * h + q % 2;
-            const float dp = v[0][i][j] * inv;
-            const float uj = (v[1][i][j] * nx[q] + v[2][i][j] * ny[q] + v[3][i][j] * nz[q]) * inv;
-            const float ua = (v[4][i][j] * nx[q] + v[5][i][j] * ny[q] + v[6][i][j] * nz[q]) * inv;
+            const float dp = v[0][i][j] * inv[0];
+            const float uj = (v[1][i][j] * nx[q] + v[2][i][j] * ny[q] + v[3][i][j] * nz[q]) * inv[1];
+            const float ua = (v[4][i][j] * nx[q] + v[5][i][j] * ny[q] + v[6][i][j] * nz[q]) * inv[2];
             const float U = -.5f * (dp - uj) * sJ[q];
             fl[0][h][q] = -(ua - .5f * dp) * sJ[q];
             fl[1][h][q] = U * nx[q], fl[2][h][q] = U * ny[q], fl[3][h][q] = U * nz[q];
@@ -197,7 +214,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
         for (int c = 0; c < 4; ++c) {
           Frag o;
           split_frag(o, make_float4(fl[c][0][0], fl[c][0][1], fl[c][0][2], fl[c][0][3]),
-                     make_float4(fl[c][1][0], fl[c][1][1], fl[c][1][2], fl[c][1][3]), da, db);
+                     make_float4(fl[c][1][0], fl[c][1][1], fl[c][1][2], fl[c][1][3]), da[c > 0], db[c > 0]);
           put_frag(sFc + ((f * A.FC + ch) * 4 + c) * 64, 0, lane, o);
         }
       }
@@ -267,9 +284,11 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
     {
       const float um = fmaxf(fmaxf(ma.y, ma.z), ma.w), un = fmaxf(fmaxf(mb.y, mb.z), mb.w);
       const float *Ba = A.bound + (size_t)ra_ * 8, *Bb = A.bound + (size_t)rb_ * 8;
-      const int ta = scale_field(2.f * fmaxf(__ldg(Ba) * A.dnorm * ma.x, __ldg(Ba + 1) * A.vnorm * um)),
-                tb = scale_field(2.f * fmaxf(__ldg(Bb) * A.dnorm * mb.x, __ldg(Bb + 1) * A.vnorm * un));
-      const float da = pow2_field(ta), db = pow2_field(tb);
+      // gradient of p (for u, v, w) and contravariant velocities (for p): a scale each
+      const int ta[2] = {scale_field(2.f * __ldg(Ba) * A.dnorm * ma.x),
+                         scale_field(2.f * __ldg(Ba + 1) * A.vnorm * um)};
+      const int tb[2] = {scale_field(2.f * __ldg(Bb) * A.dnorm * mb.x),
+                         scale_field(2.f * __ldg(Bb + 1) * A.vnorm * un)};
       float isc[4][2];
 #pragma unroll
       for (int c = 0; c < 4; ++c)
@@ -339,7 +358,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll
           for (int x = 0; x < 6; ++x) {
             Frag f;
-            split_frag(f, tv[x][0], tv[x][1], da, db);
+            split_frag(f, tv[x][0], tv[x][1], pow2_field(ta[x / 3]), pow2_field(tb[x / 3]));
             put_frag(sW + ((c - c0) * 6 + x) * 64, 0, lane, f);
           }
         }
@@ -363,13 +382,14 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
           }
         }
       }
-      const float ia = -pow2_field(254 - ta) * A.iP, ib = -pow2_field(254 - tb) * A.iP;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+      for (int c = 0; c < 4; ++c) {
+        const float ia = -pow2_field(254 - ta[c == 0]) * A.iP, ib = -pow2_field(254 - tb[c == 0]) * A.iP;
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) r[c][i][j] = o[c][i][j] * (j < 2 ? ia : ib);
+      }
     }
 
     // ---- 4. lifted fluxes
@@ -392,14 +412,13 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
           }
         }
       }
-      const float ia = sInv[f * 16 + g], ib = sInv[f * 16 + g + 8];
 #pragma unroll
       for (int c = 0; c < 4; ++c)
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            r[c][i][j] = fmaf(o[c][i][j], j < 2 ? ia : ib, r[c][i][j]);
+            r[c][i][j] = fmaf(o[c][i][j], sInv[(f * 2 + (c > 0)) * 16 + g + (j < 2 ? 0 : 8)], r[c][i][j]);
     }
 
     // ---- 5. rk_update_WADG: interpolate, weight with 1/J (c2/J on p), project

@@ -53,3 +53,32 @@ def test_state_round_trip_between_stages(cuda):
         a.get_data(), a.get_residual()
     assert np.array_equal(a.get_data(), b.get_data())
     assert np.array_equal(a.get_residual(), b.get_residual())
+
+
+@pytest.mark.parametrize("N,n", [(3, 8), (5, 6)])
+def test_pressure_and_velocity_of_different_size(cuda, N, n):
+    """Pressure 2^24 times the velocity (p ~ c u in the caller's units) and the
+    other way round, both continuous, the pressure zero on the wall: each field's
+    right-hand side on the curved elements is as far from 64 bits as with equal
+    sizes, since every field has its own power-of-two scale (half as much again
+    is left for the sums of both in the fluxes)."""
+    from curved import CurvedOracle
+    p = problem(N, n, "default")
+    a = p.desc_arrays()
+    kc = np.asarray(a["KlistCurved"])
+    x, y, z = (np.asarray(p.mesh[c], np.float64).reshape(p.K, p.Np) for c in "xyz")
+    Q0 = np.stack([(1 - x * x - y * y - z * z) * np.cos(x + 2 * y - z), np.sin(2 * x + y),
+                   np.cos(y - z), np.sin(z + x * y)], 1)
+    err = []
+    for kp, ku in ((0, 0), (24, 0), (0, 24)):
+        Q = Q0 * np.array([2.0 ** kp] + 3 * [2.0 ** ku])[:, None]
+        Q = np.ascontiguousarray(Q, np.float32).ravel()
+        s = CurvedSolver(p)
+        s.set_data(Q)
+        s.rk_stage(0.0, 0.0, p.dt)
+        res = s.get_residual().reshape(p.K, 4, p.Np)
+        s.close()
+        _, ref = CurvedOracle(N, p.K, p.Nq, p.Nfq, a).run(Q, p.dt, 1)
+        ref = np.asarray(ref).reshape(p.K, 4, p.Np)
+        err.append([rel_l2(res[kc, c], ref[kc, c]) for c in range(4)])
+    assert (np.array(err[1:]) <= 1.5 * np.array(err[0])).all(), err
