@@ -518,22 +518,28 @@ static bool vectors(const void *a, const void *b, const void *c = nullptr) {
   return (((size_t)a | (size_t)b | (size_t)c) & 15) == 0;
 }
 // and split the operators in every CTA, which few elements do not repay.  us,
-// thread per node / matrix:
-//   volume   N = 2 K = 24576: 8.6 / 10.5   N = 3 K = 3072: 7.6 / 8.5, K = 10368: 9.4 / 8.4
-//            N = 4 K = 384: 16.7 / 10.6    N = 5 K = 384: 16.6 / 12.6, K = 24576: 76 / 29
-//            N = 6 K = 384: 16.7 / 20.8, K = 3072: 26.8 / 21.2   N = 7 K = 384: 41 / 35
-//   surface  N = 2 K = 24576: 12.4 / 14.4  N = 3 K = 384: 10.4 / 7.3, K = 24576: 22.7 / 16.6
-//            N = 5 K = 24576: 139 / 29     N = 6 K = 384: 14.5 / 16.3, K = 3072: 24.7 / 16.5
-//   update   N = 2 K = 10368: 12.4 / 16.4, K = 24576: 20.6 / 18.2
-//            N = 3 K = 3072: 12.4 / 12.4, K = 10368: 16.6 / 14.5
-//            N = 4 K = 3072: 17.8 / 16.5   N = 5 K = 384: 16.5 / 17.6, K = 24576: 154 / 83
-//            N = 6 K = 384: 24.7 / 32.9, K = 3072: 56 / 51   (N = 7: 214 points do not fit)
+// thread per node / matrix, each launch alone, one tile to 48000 elements:
+//   volume   N = 2: never (K = 48000 12.4)  N = 3 K = 10368: 8.7 / 9.0, K = 16464: 12.4 / 10.3
+//            N = 4 K = 6: 12.9 / 10.3, K = 24576: 43 / 31
+//            N = 5 K = 6: 14.6 / 12.4, K = 24576: 76 / 31
+//            N = 6 K = 2058: 22.6 / 24.7, K = 3072: 26.1 / 24.7
+//            N = 7 K = 2058: 43.9 / 45.2, K = 3072: 58 / 45
+//   surface  N = 2: 12.4 / 14.4 at K = 24576  N = 3 K = 6: 9.3 / 7.1, K = 24576: 22.7 / 16.5
+//            N = 4 K = 6: 12.4 / 8.8, K = 24576: 52 / 31
+//            N = 5 K = 6: 16.5 / 12.4, K = 24576: 139 / 29
+//            N = 6 K = 1296: 15.4 / 17.8, K = 2058: 18.6 / 18.5, K = 3072: 24.7 / 18.5
+//            N = 7 K = 1296: 18.5 / 22.7, K = 2058: 27.8 / 22.7
+//   update   N = 2 K = 24576: 20.6 / 18.5, but K = 34992: 24.7 / 30.8
+//            N = 3 K = 4374: 12.4 / 12.4, K = 13182: 22.6 / 14.5
+//            N = 4 K = 1296: 16.5 / 14.6, K = 24576: 74 / 62
+//            N = 5 K = 1296: 18.5 / 19.3, K = 2058: 20.6 / 20.6, K = 24576: 155 / 88
+//            N = 6 K = 3072: 57 / 54, K = 6000: 88 / 72   (N = 7: the operators do not fit)
 enum { REF_VOLUME, REF_SURFACE, REF_UPDATE };
 static bool matrix_form(int kernel, int N, int K) {
   constexpr int never = 1 << 30;
-  constexpr int from[3][8] = {{never, never, never, 8000, 0, 0, 1500, 0},
-                              {never, never, never, 0, 0, 0, 1000, 1000},
-                              {never, never, 20000, 4000, 1000, 1000, 2500, 2500}};
+  constexpr int from[3][8] = {{never, never, never, 13000, 0, 0, 2500, 2500},
+                              {never, never, never, 0, 0, 0, 2000, 2000},
+                              {never, never, never, 4000, 1000, 2000, 2500, never}};
   return N >= 1 && N <= 7 && K >= from[kernel][N];
 }
 
@@ -543,11 +549,9 @@ static bool matrix_form(int kernel, int N, int K) {
     case 4: return CALL(4);  \
     case 5: return CALL(5);  \
     case 6: return CALL(6);  \
-    case 7: return CALL(7);  \
   }
 static bool update_fits(int N, int Nq) {
 #define CALL(n) ref_update_fits_##n(Nq)
-  if (N == 2) return CALL(2);
   BBW_MMA_SWITCH(CALL)
 #undef CALL
   return false;
@@ -567,6 +571,7 @@ extern "C" bbw_status bbw_rk_volume(int N, int K, const float *vgeo, const float
   cudaStream_t st = (cudaStream_t)stream;
   if (matrix_form(REF_VOLUME, N, K) && vectors(Q, rhsQ)) {
 #define CALL(n) ref_volume_##n(K, vgeo, Dr, Ds, Dt, Q, rhsQ, st)
+    if (N == 7) return CALL(7);
     BBW_MMA_SWITCH(CALL)
 #undef CALL
   }
@@ -597,6 +602,7 @@ extern "C" bbw_status bbw_rk_surface(int N, int K, int bc, const float *fgeo, co
   cudaStream_t st = (cudaStream_t)stream;
   if (matrix_form(REF_SURFACE, N, K) && vectors(Q, rhsQ)) {
 #define CALL(n) ref_surface_##n(K, bc, fgeo, Fmask, vmapP, LIFT, Q, rhsQ, st)
+    if (N == 7) return CALL(7);
     BBW_MMA_SWITCH(CALL)
 #undef CALL
   }
@@ -642,7 +648,6 @@ extern "C" bbw_status bbw_rk_update_wadg(int N, int K, int Nq, const float *Vq, 
   cudaStream_t st = (cudaStream_t)stream;
   if (matrix_form(REF_UPDATE, N, K) && vectors(Q, rhsQ, resQ) && update_fits(N, Nq)) {
 #define CALL(n) ref_update_##n(K, Nq, Vq, Pq, Jq, c2q, fa, fb, fdt, rhsQ, resQ, Q, st)
-    if (N == 2) return CALL(2);
     BBW_MMA_SWITCH(CALL)
 #undef CALL
   }

@@ -1,5 +1,4 @@
 #include "ref_mma.cuh"
 namespace bbw {
 BBW_REF_RHS_INSTANCE(7)
-BBW_REF_UPDATE_INSTANCE(7)
 }

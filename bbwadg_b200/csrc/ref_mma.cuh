@@ -6,7 +6,8 @@
 // as warp_pack does), then its warps
 // walk 16-element tiles.  The kernels with a thread per node (kernels_ref.cu)
 // spend one operator load and one or more shared loads per FMA; they stay for
-// small meshes, N = 8, and pointers that are not 16-byte aligned.
+// small meshes (matrix_form, kernels_ref.cu), N = 1, 2 and 8, and pointers that are
+// not 16-byte aligned.
 #pragma once
 #include <vector>
 

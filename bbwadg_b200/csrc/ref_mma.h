@@ -16,8 +16,7 @@ namespace bbw {
   bbw_status ref_update_##n(int, int, const float *, const float *, const float *, const float *, \
                             float, float, float, const float *, float *, float *, cudaStream_t);
 BBW_REF_RHS_DECL(3) BBW_REF_RHS_DECL(4) BBW_REF_RHS_DECL(5) BBW_REF_RHS_DECL(6) BBW_REF_RHS_DECL(7)
-BBW_REF_UPDATE_DECL(2) BBW_REF_UPDATE_DECL(3) BBW_REF_UPDATE_DECL(4) BBW_REF_UPDATE_DECL(5)
-BBW_REF_UPDATE_DECL(6) BBW_REF_UPDATE_DECL(7)
+BBW_REF_UPDATE_DECL(3) BBW_REF_UPDATE_DECL(4) BBW_REF_UPDATE_DECL(5) BBW_REF_UPDATE_DECL(6)
 #undef BBW_REF_RHS_DECL
 #undef BBW_REF_UPDATE_DECL
 
