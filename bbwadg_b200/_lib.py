@@ -90,6 +90,7 @@ SIGNATURES = {
     "bbw_stage_ex": (c_int, [c_void_p, c_float, c_float, c_float, c_float]),
     "bbw_set_shots": (c_int, [c_void_p, c_int]),
     "bbw_set_compute_range": (c_int, [c_void_p, c_int]),
+    "bbw_set_whole_mesh": (c_int, [c_void_p, c_int]),
     "bbw_gather_elements": (c_int, [c_void_p, c_int, P, P]),
     "bbw_scatter_elements": (c_int, [c_void_p, c_int, P, P]),
     "bbw_stage_part": (c_int, [c_void_p, c_float, c_float, c_float, c_int, c_int]),

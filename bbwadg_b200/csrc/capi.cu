@@ -384,6 +384,7 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
 
   bbw_ctx *c = new bbw_ctx;
   c->N = N, c->K = K, c->Nq = Nq, c->Np = Np, c->Nfp = Nfp, c->variant = variant, c->bc = bc;
+  c->whole_K = K;
   dense_operators(N, Nq, o, bb, c);
   c->hFmask.assign(m->Fmask, m->Fmask + NF);
   c->hvmapP.assign(m->vmapP, m->vmapP + (size_t)K * NF);
@@ -584,7 +585,7 @@ static bool narrow_tiles(const bbw_ctx *c) {
 
 bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
                         float fdt, float cstage, cudaStream_t st, int K0, int Kc, bool chained) {
-  const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, (long long)c->S * c->K);
+  const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, (long long)c->S * c->K, (long long)c->S * c->whole_K);
   if (form != WARP_AUTO) {
     WarpPlan p = c->wp;
     p.S = c->S, p.K0 = K0, p.Kc = Kc > 0 ? Kc : c->plan.Kc, p.max_ctas = c->plan.max_ctas;
@@ -848,6 +849,16 @@ extern "C" bbw_status bbw_set_compute_range(bbw_ctx *c, int Kc) {
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_compute_range");
   c->plan.Kc = Kc;
+  drop_graphs(c);
+  return BBW_OK;
+}
+
+extern "C" bbw_status bbw_set_whole_mesh(bbw_ctx *c, int K_whole) {
+  DeviceGuard dg(c ? c->device : -1);
+  if (!c || K_whole < 1) return set_error(BBW_ERR_ARG, "bbw_set_whole_mesh: bad argument");
+  cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_whole_mesh");
+  c->whole_K = K_whole;
   drop_graphs(c);
   return BBW_OK;
 }

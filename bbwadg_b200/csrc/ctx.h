@@ -76,6 +76,7 @@ struct bbw_ctx {
   float *ops_narrow = nullptr;
   int precision = BBW_PREC_FP32;
   int S = 1;  // shots
+  int whole_K = 0;  // elements of the whole mesh (K unless the context holds a part)
   double *d_time = nullptr;
   int *d_step = nullptr;
   int *src_off = nullptr, *src_elem = nullptr;

@@ -71,24 +71,30 @@ void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<floa
                std::vector<uint32_t> &out);
 // Sets the forms that fit (pl.single, pl.group).
 bbw_status warp_prepare(WarpPlan &pl);
-// The form for `elements` (mesh elements times shots) when none is pinned;
-// WARP_AUTO: the CTA-wide stages.  One warp and group give the same results
-// bit for bit, the CTA-wide stages the same to FP32 rounding.  us per stage,
-// CTA-wide FP32 / one warp / group:
-//   N = 2  K = 1296: 5.4 / 9.4 / -      K = 6000: 12.0 / 9.4 / -
-//   N = 3  K = 3072: 9.4 / 10.7 / -     K = 6000: 17.2 / 10.7 / -
-//   N = 4  K = 3072: 16.8 / 17.6 / 12.7 K = 10368: 43.4 / 22.3 / 34.1
-//   N = 5  K = 384: 23.3 / 24.4 / 10.6  K = 196608: 879 / 422 / 411
-//   N = 6  K = 384: 73 / 45 / 17        K = 24576: 454 / 154 / 123
-//   N = 7  K = 384: 112 / 80 / 17       K = 24576: 706 / 327 / 178
+// The form for `elements` (elements of this context times shots) when none is
+// pinned; WARP_AUTO: the CTA-wide stages.  One warp and group give the same
+// results bit for bit, the CTA-wide stages the same to FP32 rounding: whether the
+// arithmetic is the matrix units' depends on N and `whole` only, the elements of
+// the whole mesh times shots, of which the context may be a part
+// (bbw_set_whole_mesh), so the parts of a cut mesh give the uncut one's bits.  It
+// does not depend on the grid limit either.  us per stage, CTA-wide FP32 / one
+// warp / group:
+//   N = 1  K = 6000: 8.2 / 6.5 / -      K = 93750: 57 / 29 / -
+//   N = 2  K = 1296: 5.7 / 9.4 / -      K = 6000: 11.9 / 9.5 / -
+//   N = 3  K = 3072: 9.4 / 11.2 / -     K = 6000: 17.6 / 11.5 / -
+//   N = 4  K = 6: 15.6 / - / 9.9        K = 3072: 16.8 / 18.2 / 13.2  K = 10368: 43.8 / 22.6 / 34
+//   N = 5  K = 6: 21.0 / - / 10.3       K = 3072: 23.8 / - / 14.7     K = 196608: 878 / - / 429
+//   N = 6  K = 6: 73 / - / 17.7         K = 24576: 475 / - / 140
+//   N = 7  K = 6: 112 / - / 19.3        K = 24576: 736 / - / 206
+// and with the package's own rules N = 5, 216 points K = 6: 53.9 / - / 15.2, K = 24576:
+// 335 / - / 97; N = 6, 343 points, K = 10368: 289 / - / 72 (before the rests).
 // One warp per tile pays once there are about two tiles per SM; the group
-// form, three tiles or more per SM at a time, up to the 592 tiles of its first
-// wave at N = 4, and at every size above.
-inline int stage_form(const WarpPlan &pl, long long elements) {
-  const long long tiles = elements / 16;
+// form, three tiles or more per SM at a time, up to the tiles of its first wave
+// at N = 4 (four per SM), and at every size above.
+inline int stage_form(const WarpPlan &pl, long long elements, long long whole) {
   if (pl.pinned != WARP_AUTO) return pl.pinned;
-  if (pl.group && (pl.N >= 5 || tiles <= 4 * 148)) return WARP_GROUP;
-  return pl.single && tiles > 2 * 148 ? WARP_SINGLE : WARP_AUTO;
+  if (pl.group && (pl.N >= 5 || elements / 16 <= 4LL * pl.nsm)) return WARP_GROUP;
+  return pl.single && (pl.N >= 4 || whole / 16 > 2LL * pl.nsm) ? WARP_SINGLE : WARP_AUTO;
 }
 bbw_status warp_launch(const WarpPlan &pl, int form, const float *Qin, float *Qout, float *res,
                        float fa, float fb, float fdt, float cstage, cudaStream_t st);

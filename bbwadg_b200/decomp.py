@@ -12,7 +12,8 @@ bbw_scatter_elements), so the next stage sees current neighbour traces.
 One exchange per stage carries 4 Np floats per halo element and shot.  The
 reference runs on one device (cpp/src/WaveOKL3d.cpp:1415); the per-element
 arithmetic is unchanged by the cut, so the decomposed run reproduces the
-single-device run.
+single-device run bit for bit (local_solver names the whole mesh's size, by
+which the stage's arithmetic is chosen).
 
 Overlap (``slab_partition(..., interface_first=True)`` and
 ``run_decomposed(..., overlap=True)``): each part's owned elements are
@@ -116,6 +117,7 @@ def local_solver(prob, part, **kw):
     s = WaveSolver(N=prob.N, K=part.K, Nq=prob.Nq, variant=prob.variant, ops=prob.ops_dict(),
                    vgeo=part.vgeo, fgeo=part.fgeo, vmapP=part.vmapP, c2q=part.c2q, **kw)
     s.set_compute_range(part.Kc)
+    s.set_whole_mesh(prob.K)
     return s
 
 

@@ -174,6 +174,11 @@ class WaveSolver:
         """Advance elements [0, Kc) only; [Kc, K) are halo copies."""
         _lib.call("bbw_set_compute_range", self._h, int(Kc))
 
+    def set_whole_mesh(self, K_whole):
+        """This solver holds a part of a mesh of K_whole elements: its stage is
+        chosen as for the whole one (same bits)."""
+        _lib.call("bbw_set_whole_mesh", self._h, int(K_whole))
+
     def gather_elements(self, idx, buf):
         """buf[s][j] = state of element idx[j] in shot s (device int32 idx,
         device float32 buf of S * len(idx) * 4 * Np floats)."""

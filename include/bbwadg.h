@@ -330,6 +330,11 @@ bbw_status bbw_set_grid_limit(bbw_ctx *ctx, int max_ctas);
  * buffer back.  No reference counterpart (the reference runs one device,
  * cpp/src/WaveOKL3d.cpp:1415).  FP32 stage only. */
 bbw_status bbw_set_compute_range(bbw_ctx *ctx, int Kc);
+/* The context holds a part of a mesh of K_whole elements (default: all of it):
+ * the stage's arithmetic (CUDA cores or matrix units, BBW_PREC_FP32 above) is
+ * chosen as for the whole mesh, so that the parts give the bits of one context
+ * with the same number of shots.  No reference counterpart. */
+bbw_status bbw_set_whole_mesh(bbw_ctx *ctx, int K_whole);
 bbw_status bbw_gather_elements(bbw_ctx *ctx, int n, const int *idx, float *buf);
 bbw_status bbw_scatter_elements(bbw_ctx *ctx, int n, const int *idx, const float *buf);
 
@@ -351,7 +356,10 @@ bbw_status bbw_move_elements(bbw_ctx *ctx, int which, int dir, int n, const int 
 /* ---- batched shots, sources, receivers (every precision)
  * S independent shots share mesh, medium and operators; the state, residual
  * and traces hold S consecutive blocks and every stage launch advances all
- * of them.  Resizing drops state (zeroed) and the source table. */
+ * of them.  Resizing drops state (zeroed) and the source table.  At N <= 3
+ * the stage's arithmetic is chosen by elements times shots (BBW_PREC_FP32 above), so
+ * there a shot's last bits can depend on the number of shots beside it; a pinned
+ * configuration (bbw_set_config) rules that out. */
 bbw_status bbw_set_shots(bbw_ctx *ctx, int S);
 
 /* Source entries (acous_elas_cpp/src/WaveOKL3d.cpp:765-781 and
