@@ -724,14 +724,21 @@ extern "C" bbw_status bbw_set_config(bbw_ctx *c, int config) {
   const int W = config & 255;
   if ((W != 8 && W != 16) || ((config >> 11) != 0 && config != kWarpConfig && config != kGroupConfig))
     return set_error(BBW_ERR_ARG, "bbw_set_config: W must be 8 or 16, flags bits 8-10");
-  if (c->precision != BBW_PREC_FP32) return BBW_OK;
+  const bool split = c->precision == BBW_PREC_F16X3 && !c->gs;
+  if (c->precision != BBW_PREC_FP32 && !split) return BBW_OK;
   cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_config");
   if (config == kWarpConfig || config == kGroupConfig) {
     const bool group = config == kGroupConfig;
     if (!(group ? c->wp.group : c->wp.single))
-      return set_error(BBW_ERR_UNSUPPORTED, "bbw_set_config: no such form at this size");
+      return split ? BBW_OK
+                   : set_error(BBW_ERR_UNSUPPORTED, "bbw_set_config: no such form at this size");
     c->wp.pinned = group ? WARP_GROUP : WARP_SINGLE, c->cta_form = false;
+    drop_graphs(c);
+    return BBW_OK;
+  }
+  if (split) {  // one CTA-wide form: the tcgen05 stage
+    c->cta_form = true;
     drop_graphs(c);
     return BBW_OK;
   }

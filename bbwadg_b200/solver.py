@@ -211,7 +211,9 @@ class WaveSolver:
 
     def set_config(self, warps, ops_in_smem, pipelined, tile=32):
         """Pin a fused-stage variant (as returned by autotune); tile is the
-        elements per tile, 32 or 16."""
+        elements per tile, 32 or 16.  A CTA-wide variant (pipelined a flag) gives
+        steps() the bits of forward(); in split-FP16 solvers it is the tcgen05
+        stage."""
         _lib.call("bbw_set_config", self._h, encode_config(warps, ops_in_smem, pipelined, tile))
 
     def set_grid_limit(self, max_ctas):
@@ -274,7 +276,8 @@ class WaveSolver:
         _lib.call("bbw_set_c2q", self._h, c2q.ctypes.data)
 
     def forward(self, dt, nsteps, checkpoint_every=50, keep="cubature"):
-        """nsteps steps as steps() does; returns a Tape.  keep="cubature"
+        """nsteps steps as steps() does (the same bits while a CTA-wide variant is
+        pinned, see set_config; else to rounding); returns a Tape.  keep="cubature"
         stores every stage's cubature values when the device has room (the
         backward pass then recomputes nothing), else checkpoints every
         checkpoint_every steps; keep="checkpoints" always checkpoints."""

@@ -310,7 +310,10 @@ bbw_status bbw_run(bbw_ctx *ctx, double final_time, float dt);
  * (cpp/src/WaveOKL3d.cpp:1618-1650, cpp/profileKernels). */
 bbw_status bbw_autotune(bbw_ctx *ctx, float dt, int stages, int *config);
 /* Applies a configuration code as returned by bbw_autotune (for instance one
- * cached from an earlier run); BBW_ERR_UNSUPPORTED if it does not fit. */
+ * cached from an earlier run); BBW_ERR_UNSUPPORTED if it does not fit.  F16X3
+ * contexts: a code of the CTA-wide variants takes the tcgen05 stage, those of the
+ * warp-matrix stages these where they exist; other precisions ignore it.  While a
+ * CTA-wide variant is set, bbw_steps gives the bits of bbw_forward. */
 bbw_status bbw_set_config(bbw_ctx *ctx, int config);
 /* Caps the persistent stage kernels (FP32 fused and tensor-core forms) at
  * max_ctas CTAs, each then looping over more element tiles; 0 restores one
@@ -492,10 +495,12 @@ typedef struct bbw_tape bbw_tape;
 bbw_status bbw_set_c2q(bbw_ctx *ctx, const float *c2q);
 
 /* Advances nsteps steps of dt as bbw_steps does, on the CUDA-core or tcgen05
- * stage whose rounding the FP64 gradient is pinned to (the time loop's stage
- * agrees with it to FP32 rounding; receivers must be set; traces land at the current step count onwards) and returns a tape
- * for bbw_backward: bbw_forward_ex with BBW_TAPE_CUBATURE (every stage's
- * cubature values when they fit, else the state at every
+ * stage whose rounding the FP64 gradient follows: the time loop's stage agrees
+ * with it to FP32 rounding, and bit for bit while a CTA-wide variant is set
+ * (bbw_set_config; a misfit at the medium that made the data is then exactly
+ * zero).  Receivers must be set; traces land at the current step count onwards.
+ * Returns a tape for bbw_backward: bbw_forward_ex with BBW_TAPE_CUBATURE (every
+ * stage's cubature values when they fit, else the state at every
  * checkpoint_every-th step start).  No counterpart in the reference. */
 bbw_status bbw_forward(bbw_ctx *ctx, float dt, int nsteps, int checkpoint_every,
                        bbw_tape **tape);
