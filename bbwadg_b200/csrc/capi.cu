@@ -242,7 +242,9 @@ bbw_status compress_connectivity(int N, int K, const int *Fmask, const int *vmap
 
 }  // namespace
 
-// the fused stage's plan and packed operators with W warps and E-element tiles
+// plan of the fused stage with W warps, E-element tiles and the requested
+// placement; the packed operators are uploaded to *ops_buf (owned by the
+// caller)
 static bbw_status make_variant(bbw_ctx *c, int W, int E, int want_ops, int want_pipe,
                                FusedPlan &p, float **ops_buf) {
   FusedOps fo;
@@ -711,9 +713,6 @@ extern "C" bbw_status bbw_steps(bbw_ctx *c, float dt, int nsteps) {
   return run_steps(c, dt, nsteps, false);
 }
 
-// plan of the fused stage with W warps, E-element tiles and the requested
-// placement; the packed operators are uploaded to *ops_buf (owned by the
-// caller)
 static int config_code(const FusedPlan &p) {
   return p.W | (p.ops_smem > 0 ? 1 << 8 : 0) | (p.pipe ? 1 << 9 : 0) | (p.E == 16 ? 1 << 10 : 0);
 }
@@ -788,27 +787,30 @@ extern "C" bbw_status bbw_autotune(bbw_ctx *c, float dt, int stages, int *config
   const int Ws[2] = {8, 16}, Es[2] = {32, 16};
   float best_ms = 0.f;
   int best = -1;
-  // times one form over `stages` launches; launch(in, out, a, b) is one stage
+  // times one form over `stages` launches; launch(in, out, a, b, chained) is one
+  // stage, chained as in a step of the time loop.  A form that is refused is out.
   auto time_form = [&](int code, auto &&launch) {
     int cur = 0;
-    for (int i = 0; i < 2; ++i, cur ^= 1)  // warm-up
-      launch(q[cur], q[cur ^ 1], 0.f, (float)kRK4B[0]);
+    bbw_status ok = BBW_OK;
+    for (int i = 0; i < 2 && ok == BBW_OK; ++i, cur ^= 1)  // warm-up
+      ok = launch(q[cur], q[cur ^ 1], 0.f, (float)kRK4B[0], false);
     cudaEventRecord(e0, c->stream);
-    for (int i = 0; i < stages; ++i, cur ^= 1)
-      launch(q[cur], q[cur ^ 1], (float)kRK4A[i % 5], (float)kRK4B[i % 5]);
+    for (int i = 0; i < stages && ok == BBW_OK; ++i, cur ^= 1)
+      ok = launch(q[cur], q[cur ^ 1], (float)kRK4A[i % 5], (float)kRK4B[i % 5], i % 5 > 0);
     cudaEventRecord(e1, c->stream);
     e = cudaEventSynchronize(e1);
     float ms = 0.f;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-    if (e == cudaSuccess && (best < 0 || ms < best_ms)) best = code, best_ms = ms;
+    if (e == cudaSuccess && ok == BBW_OK && (best < 0 || ms < best_ms)) best = code, best_ms = ms;
   };
   for (int form = WARP_SINGLE; form <= WARP_GROUP; ++form) {
     if (!(form == WARP_GROUP ? c->wp.group : c->wp.single)) continue;
     WarpPlan p = c->wp;
     p.S = c->S, p.Kc = c->plan.Kc, p.max_ctas = c->plan.max_ctas;
     time_form(form == WARP_GROUP ? kGroupConfig : kWarpConfig,
-              [&](const float *in, float *out, float fa, float fb) {
-                warp_launch(p, form, in, out, r, fa, fb, dt, 0.f, c->stream);
+              [&](const float *in, float *out, float fa, float fb, bool chained) {
+                p.chained = chained;
+                return warp_launch(p, form, in, out, r, fa, fb, dt, 0.f, c->stream);
               });
   }
   for (int ei = 0; ei < 2 && e == cudaSuccess; ++ei)
@@ -820,8 +822,9 @@ extern "C" bbw_status bbw_autotune(bbw_ctx *c, float dt, int stages, int *config
         cudaFree(buf);  // does not fit
         continue;
       }
-      time_form(config_code(p), [&](const float *in, float *out, float fa, float fb) {
-        fused_launch(p, in, out, r, fa, fb, dt, 0.f, c->stream);
+      time_form(config_code(p), [&](const float *in, float *out, float fa, float fb, bool chained) {
+        p.chained = chained;
+        return fused_launch(p, in, out, r, fa, fb, dt, 0.f, c->stream);
       });
       cudaFree(buf);
     }
