@@ -155,7 +155,9 @@ extern "C" bbw_status bbw_set_c2q(bbw_ctx *c, const float *c2q) {
   if (e == cudaSuccess)
     e = cudaMemcpy(c->c2q, c2q, (size_t)c->K * c->Nq * sizeof(float), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return set_cuda_error(e, "bbw_set_c2q");
-  return c->c2p ? warp_medium(c->K, c->Nq, c->c2q, c->c2max, c->c2p) : BBW_OK;
+  if (!c->c2p) return BBW_OK;
+  const bbw_status s = warp_medium(c->K, c->Nq, c->c2q, c->c2max, c->c2p);
+  return s != BBW_OK ? s : setup_done("bbw_set_c2q");
 }
 
 extern "C" bbw_status bbw_tape_free(bbw_tape *t) {

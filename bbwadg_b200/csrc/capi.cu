@@ -78,7 +78,6 @@ void release(bbw_ctx *c) {
   cudaFree(c->geo_tc);
   cudaFree(c->ops_tc);
   cudaFree(c->ops_wp);
-  cudaFree(c->c2max);
   cudaFree(c->c2p);
   cudaFree(c->err);
   adj_release(c);
@@ -440,27 +439,30 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
       return s;
     }
   }
-  if (!gemm && (tcp || N <= 7) &&
-      ((s = upload<float>(&c->geo_tc, nullptr, (size_t)(K + 16) * TC_GEO, "bbw_create: geometry")) !=
-           BBW_OK ||
-       (s = geometry_records(K, c->vgeo, c->fgeo, c->geo_tc)) != BBW_OK)) {
-    release(c);
-    return s;
+  const bool matrix = !gemm && precision != BBW_PREC_BF16X3 && N <= 7;
+  if (!gemm && (tcp || N <= 7)) {
+    // written in full by kernels: no fill
+    const size_t rec = (size_t)(K + 16) * TC_GEO, med = (size_t)K * ((Nq + 15) / 16 * 16);
+    e = cudaMalloc((void **)&c->geo_tc, rec * sizeof(float));
+    if (e == cudaSuccess && matrix) e = cudaMalloc((void **)&c->c2p, (med + K) * sizeof(float));
+    s = set_cuda_error(e, "bbw_create: geometry and medium");
+    if (s == BBW_OK) s = geometry_records(K, c->vgeo, c->fgeo, c->geo_tc);
+    if (s == BBW_OK && matrix) {
+      c->c2max = c->c2p + med;
+      s = warp_medium(K, Nq, c->c2q, c->c2max, c->c2p);
+    }
+    if (s != BBW_OK) {
+      release(c);
+      return s;
+    }
   }
-  if (!gemm && precision != BBW_PREC_BF16X3 && N <= 7) {
+  if (matrix) {
     // FP32 contexts take four products per split pair, split FP16 three; BB
     // contexts the dense equivalents of their sparse operators
     WarpPlan &wp = c->wp;
     wp.N = N, wp.K = K, wp.Nq = Nq, wp.bc = bc, wp.products = precision == BBW_PREC_FP32 ? 4 : 3;
     wp.pat_off = pat_off, wp.table_ints = bb_off;  // Fmask and the face permutations
-    std::vector<uint32_t> wops;
-    warp_pack(wp, c->hD, c->hLIFT, c->hVq, c->hPq, wops);
-    if ((s = upload(&c->ops_wp, reinterpret_cast<const uint4 *>(wops.data()), wops.size() / 4,
-                    "bbw_create: split operators")) != BBW_OK ||
-        (s = upload<float>(&c->c2max, nullptr, K, "bbw_create: medium bound")) != BBW_OK ||
-        (s = upload<float>(&c->c2p, nullptr, (size_t)K * ((Nq + 15) / 16 * 16),
-                           "bbw_create: medium")) != BBW_OK ||
-        (s = warp_medium(K, Nq, c->c2q, c->c2max, c->c2p)) != BBW_OK) {
+    if ((s = warp_pack(wp, c->hD, c->hLIFT, c->hVq, c->hPq, &c->ops_wp)) != BBW_OK) {
       release(c);
       return s;
     }
@@ -513,6 +515,10 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
       release(c);
       return s;
     }
+  }
+  if ((s = setup_done("bbw_create")) != BBW_OK) {
+    release(c);
+    return s;
   }
   *out = c;
   return BBW_OK;

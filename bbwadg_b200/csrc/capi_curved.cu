@@ -109,40 +109,41 @@ bbw_status setup_mma(bbw_curved *h, const bbw_curved_desc *d) {
   bbw_status s = curved_mma_prepare(h->N, M);
   if (s == BBW_ERR_UNSUPPORTED) return BBW_OK;
   if (s != BBW_OK) return s;
-  SplitOps ops;
   const size_t mq = (size_t)Nq * Np, mr = (size_t)Nr * Np;
-  const float *V[4] = {d->Vq, d->Vrq, d->Vsq, d->Vtq}, *P[4] = {d->Pq, d->Prq, d->Psq, d->Ptq};
-  const float sV = split_scale(V, 1, mq), sD = split_scale(V + 1, 3, mq);
+  const float *hV[4] = {d->Vq, d->Vrq, d->Vsq, d->Vtq}, *hP[4] = {d->Pq, d->Prq, d->Psq, d->Ptq};
+  const float sV = split_scale(hV, 1, mq), sD = split_scale(hV + 1, 3, mq);
   const float *pf[1] = {d->Pfq};
-  const float sP = std::min(split_scale(P, 4, mq), split_scale(pf, 1, (size_t)Np * 4 * Nfq));
+  const float sP = std::min(split_scale(hP, 4, mq), split_scale(pf, 1, (size_t)Np * 4 * Nfq));
+  const float sF = split_scale(&d->VfqFace, 1, (size_t)Nfq * Nfp);
+  const float sVr = split_scale(&d->Vq_reduced, 1, mr), sPr = split_scale(&d->Pq_reduced, 1, mr);
+  std::vector<PackRegion> ops;  // of the operators on the device
+  const float *V[4] = {S.Vq, S.Vrq, S.Vsq, S.Vtq}, *P[4] = {S.Pq, S.Prq, S.Psq, S.Ptq};
   for (int i = 0; i < 4; ++i) {
     split_rows(ops, V[i], Nq, Np, i == 0 ? sV : sD, M.oV[i], M.oVt[i]);
     split_columns(ops, P[i], Np, Nq, sP, M.oP[i]);
   }
-  const float sF = split_scale(&d->VfqFace, 1, (size_t)Nfq * Nfp);
-  split_rows(ops, d->VfqFace, Nfq, Nfp, sF, M.oF, M.oFt);
+  split_rows(ops, S.VfqFace, Nfq, Nfp, sF, M.oF, M.oFt);
   for (int f = 0; f < 4; ++f) {
     int off = 0;
-    split_columns(ops, d->Pfq + (size_t)f * Nfq * Np, Np, Nfq, sP, off);
+    split_columns(ops, S.Pfq + (size_t)f * Nfq * Np, Np, Nfq, sP, off);
     if (f == 0) M.oL = off;
   }
-  const float sVr = split_scale(&d->Vq_reduced, 1, mr), sPr = split_scale(&d->Pq_reduced, 1, mr);
-  split_rows(ops, d->Vq_reduced, Nr, Np, sVr, M.oVr, M.oVrt);
-  split_columns(ops, d->Pq_reduced, Np, Nr, sPr, M.oPr);
+  split_rows(ops, S.Vqr, Nr, Np, sVr, M.oVr, M.oVrt);
+  split_columns(ops, S.Pqr, Np, Nr, sPr, M.oPr);
+  M.oM = ops.back().end();
   M.iV = 1.f / sV, M.iD = 1.f / sD, M.iP = 1.f / sP, M.iF = 1.f / sF, M.iVr = 1.f / sVr,
   M.iPr = 1.f / sPr;
   M.vnorm = max_row_sum(d->Vq, Nq, Np), M.rnorm = max_row_sum(d->Vq_reduced, Nr, Np);
   M.fnorm = max_row_sum(d->VfqFace, Nfq, Nfp);
   M.dnorm = std::max(max_row_sum(d->Vrq, Nq, Np),
                      std::max(max_row_sum(d->Vsq, Nq, Np), max_row_sum(d->Vtq, Nq, Np)));
-  M.oM = (int)(ops.w.size() / 4);
-  const std::vector<uint32_t> words = ops.words();
   uint4 *dops = nullptr;
   float *gq = nullptr, *fq = nullptr, *jq = nullptr, *bound = nullptr;
   const size_t nt = M.nt;
   const float *none = nullptr;
-  if ((s = own_upload(h, &dops, reinterpret_cast<const uint4 *>(words.data()), words.size() / 4,
-                      "bbw_curved_create: split operators")) != BBW_OK ||
+  if ((s = own_upload(h, &dops, (const uint4 *)nullptr, (size_t)M.oM / 4 * 5, "bbw_curved_create")) !=
+          BBW_OK ||
+      (s = pack_operators(ops, dops, dops + M.oM)) != BBW_OK ||
       (s = own_upload(h, &gq, none, nt * M.nch * 10 * 256, "bbw_curved_create")) != BBW_OK ||
       (s = own_upload(h, &fq, none, nt * 4 * M.FC * 4 * 256, "bbw_curved_create")) != BBW_OK ||
       (s = own_upload(h, &jq, none, nt * M.nchr * 2 * 256, "bbw_curved_create")) != BBW_OK ||

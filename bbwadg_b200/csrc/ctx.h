@@ -90,7 +90,7 @@ struct bbw_ctx {
   bbw::WarpPlan wp;         // warp-matrix stages
   bool cta_form = false;    // the caller or the autotuner chose a CTA-wide variant
   uint4 *ops_wp = nullptr;
-  float *c2max = nullptr;   // [K] largest |c2q| of each element
+  float *c2max = nullptr;   // [K] largest |c2q| of each element (behind c2p)
   float *c2p = nullptr;     // [K][Nq rounded up to 16] c2q padded with zeros
   bbw::GemmStage *gs = nullptr;  // precision-study GEMM form (null: fused or tensor-core stage)
   float *geo_tc = nullptr;

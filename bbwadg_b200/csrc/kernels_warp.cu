@@ -1,16 +1,12 @@
 // Host side of the warp-matrix stage (warp_stage.cuh): operator packing,
 // dispatch over N, per-element medium bounds.
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
-#include <utility>
 
-#include "device_common.cuh"
 #include "internal.h"
-#include "warp_stage.h"
+#include "warp_mma.cuh"
 
 namespace bbw {
 
@@ -72,64 +68,30 @@ static float operator_scale(const float *a, size_t n) {
   return std::ldexp(1.f, std::min(std::max(15 - e, -100), 100));
 }
 
-// operator entry times its scale (1 + kRoundingBias) as FP16 hi and lo and the
-// top byte of an FP16 rest
-struct Parts {
-  std::vector<uint32_t> w;  // hi | lo << 16
-  std::vector<uint8_t> m;
-  int nr = 0;
-};
-static void split_entry(double a, uint32_t &w, uint8_t &m) {
-  const __half h = __double2half(a), l = __double2half(a - __half2float(h));
-  w = (uint32_t)__half_as_ushort(h) | (uint32_t)__half_as_ushort(l) << 16;
-  m = rest_byte(__half_as_ushort(__double2half(a - __half2float(h) - __half2float(l))));
-}
-// the column-major nr x nc matrix A times s
-static void split_matrix(Parts &p, const float *A, int nr, int nc, float s) {
-  const size_t n = (size_t)nr * nc;
-  p.nr = nr, p.w.resize(n), p.m.resize(n);
-  for (size_t i = 0; i < n; ++i) split_entry((double)A[i] * s * (1.0 + kRoundingBias), p.w[i], p.m[i]);
+// one thread per lane of a tile of the region r
+template <bool K16>
+__global__ void k_pack(const PackRegion r, uint4 *ops, uint4 *rests) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, tile = i >> 5, lane = i & 31;
+  if (tile >= r.tiles()) return;
+  const int j = tile % r.nj, k = tile / r.nj % r.nk, o = tile / (r.nj * r.nk);
+  const float *A = r.A + (size_t)o * r.stride;
+  const int row = slot_index(r.nrp, j + o * r.row_step, lane >> 2);
+  uint32_t *w = reinterpret_cast<uint32_t *>(ops + r.at);
+  uint32_t *m = rests ? reinterpret_cast<uint32_t *>(rests) + r.at : nullptr;
+  split_tile<K16>(w, m, i, r.k0 + k, 2 * (lane & 3), r.s, [&](int b, int slot) {
+    const int col = slot_index(r.ncp, b, slot);
+    return row < r.nr && col < r.nc ? __ldg(A + row + (size_t)col * r.nr) : 0.f;
+  });
 }
 
-// index of slot c of block b when n indices are stored in blocks of eight
-static int warp_node(int n, int b, int c) {
-  const int nb = (n + 7) / 8;
-  if (b == nb - 1 && nb % 2) return 8 * b + c;
-  return 16 * (b / 2) + 4 * (c / 2) + 2 * (b % 2) + c % 2;
-}
-
-// tile of row block j and columns of pair (k16) or block (k8) k of the matrix
-// at p.w + at (nr x nc), zero outside; nrp, ncp: extents whose blocks the
-// indices run over
-struct PackTile {
-  const Parts *p;
-  size_t at;
-  int nr, nc, nrp, ncp, j, k;
-  bool k16;
-};
-
-static void pack_tile(const PackTile &q, uint32_t *out, uint8_t *rest) {
-  for (int lane = 0; lane < 32; ++lane) {
-    const int r = warp_node(q.nrp, q.j, lane / 4), c = 2 * (lane % 4);
-    // entries c and c + 1 of block b: words of hi, lo; bytes of the rest
-    auto words = [&](int b, uint32_t &hi, uint32_t &lo, uint8_t *m) {
-      uint32_t x[2];
-      for (int i = 0; i < 2; ++i) {
-        const int col = warp_node(q.ncp, b, c + i);
-        const bool in = r < q.nr && col < q.nc;
-        const size_t e = q.at + r + (size_t)col * q.nr;
-        x[i] = in ? q.p->w[e] : 0u, m[i] = in ? q.p->m[e] : 0;
-      }
-      hi = (x[0] & 0xffffu) | x[1] << 16, lo = x[0] >> 16 | (x[1] & 0xffff0000u);
-    };
-    if (q.k16) {
-      uint32_t *o = out + 4 * lane;
-      words(2 * q.k, o[0], o[2], rest + 4 * lane);
-      words(2 * q.k + 1, o[1], o[3], rest + 4 * lane + 2);
-    } else {
-      words(q.k, out[2 * lane], out[2 * lane + 1], rest + 2 * lane);
-    }
+bbw_status pack_operators(const std::vector<PackRegion> &regions, uint4 *ops, uint4 *rests) {
+  for (const PackRegion &r : regions) {
+    const int n = r.tiles() * 32;
+    if (n == 0) continue;
+    if (r.k16) k_pack<true><<<(n + 127) / 128, 128>>>(r, ops, rests);
+    else k_pack<false><<<(n + 127) / 128, 128>>>(r, ops, rests);
   }
+  return check_launch("split operators");
 }
 
 float split_scale(const float *const *A, int n, size_t len) {
@@ -138,99 +100,68 @@ float split_scale(const float *const *A, int n, size_t len) {
   return s;
 }
 
-static void append(SplitOps &out, const PackTile &q) {
-  const size_t n = q.k16 ? 128 : 64, at = out.w.size();
-  out.w.resize(at + n), out.m.resize(at + n);
-  pack_tile(q, &out.w[at], &out.m[at]);
+// appends a region behind the ones before it; returns its offset
+static int append(std::vector<PackRegion> &out, PackRegion r) {
+  r.at = out.empty() ? 0 : out.back().end();
+  out.push_back(r);
+  return r.at;
 }
 
-void split_rows(SplitOps &out, const float *A, int nr, int nc, float s, int &off, int &off_tail) {
+void split_rows(std::vector<PackRegion> &out, const float *A, int nr, int nc, float s, int &off,
+                int &off_tail) {
   const int nch = (nr + 15) / 16, NB = (nc + 7) / 8, KP = NB / 2, KT = NB % 2;
-  Parts p;
-  split_matrix(p, A, nr, nc, s);
-  off = (int)(out.w.size() / 4);
-  for (int c = 0; c < nch; ++c)
-    for (int k = 0; k < KP; ++k)
-      for (int h = 0; h < 2; ++h) append(out, {&p, 0, nr, nc, 16 * nch, nc, 2 * c + h, k, true});
-  off_tail = (int)(out.w.size() / 4);
-  for (int c = 0; c < nch && KT; ++c)
-    for (int h = 0; h < 2; ++h) append(out, {&p, 0, nr, nc, 16 * nch, nc, 2 * c + h, 2 * KP, false});
+  PackRegion r{A, 0, nr, nc, 16 * nch, nc, nch, KP, 2, 0, 2, 0, true, s};
+  off = append(out, r);
+  r.k0 = 2 * KP, r.nk = KT, r.k16 = false;
+  off_tail = append(out, r);
 }
 
-void split_columns(SplitOps &out, const float *A, int nr, int nc, float s, int &off) {
+void split_columns(std::vector<PackRegion> &out, const float *A, int nr, int nc, float s, int &off) {
   const int nch = (nc + 15) / 16, NB = (nr + 7) / 8;
-  Parts p;
-  split_matrix(p, A, nr, nc, s);
-  off = (int)(out.w.size() / 4);
-  for (int c = 0; c < nch; ++c)
-    for (int j = 0; j < NB; ++j) append(out, {&p, 0, nr, nc, nr, 16 * nch, j, c, true});
+  off = append(out, {A, 0, nr, nc, nr, 16 * nch, 1, nch, NB, 0, 0, 0, true, s});
 }
 
-std::vector<uint32_t> SplitOps::words() const {
-  std::vector<uint32_t> all(w);
-  all.resize(w.size() + m.size() / 4);
-  std::memcpy(all.data() + w.size(), m.data(), m.size());
-  return all;
+// blocks of the columns of n matrices A + i * stride, [i][k][block], then the odd last ones
+static void split_blocks(std::vector<PackRegion> &out, const float *A, size_t stride, int n, int nr,
+                         int nc, float s, int &off, int &off_tail) {
+  const int RB = (nr + 7) / 8, NB = (nc + 7) / 8, KP = NB / 2, KT = NB % 2;
+  PackRegion r{A, stride, nr, nc, nr, nc, n, KP, RB, 0, 0, 0, true, s};
+  off = append(out, r);
+  r.k0 = 2 * KP, r.nk = KT, r.k16 = false;
+  off_tail = append(out, r);
 }
 
-void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
-               const std::vector<float> &Vq, const std::vector<float> &Pq,
-               std::vector<uint32_t> &out) {
+bbw_status warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
+                     const std::vector<float> &Vq, const std::vector<float> &Pq, uint4 **ops) {
   const int N = pl.N, Np = np_of(N), Nfp = nfp_of(N), Nq = pl.Nq;
-  const int NB = (Np + 7) / 8, KP = NB / 2, KT = NB % 2, FB = (Nfp + 7) / 8, FP = FB / 2, FT = FB % 2;
-  const int nch = (Nq + 15) / 16, Nq16 = 16 * nch;
-  float sD = operator_scale(D[0].data(), D[0].size());
-  for (int d = 1; d < 3; ++d) sD = std::min(sD, operator_scale(D[d].data(), D[d].size()));
-  const float sL = operator_scale(LIFT.data(), LIFT.size());
+  const float *Dp[3] = {D[0].data(), D[1].data(), D[2].data()};
+  const float sD = split_scale(Dp, 3, D[0].size()), sL = operator_scale(LIFT.data(), LIFT.size());
   const float sV = operator_scale(Vq.data(), Vq.size()), sP = operator_scale(Pq.data(), Pq.size());
-  Parts D3[3], L, V, P;
-#pragma omp parallel for schedule(dynamic) num_threads(6) if (Np > 30)
-  for (int i = 0; i < 6; ++i) {
-    if (i < 3) split_matrix(D3[i], D[i].data(), Np, Np, sD);
-    else if (i == 3) split_matrix(L, LIFT.data(), Np, 4 * Nfp, sL);
-    else if (i == 4) split_matrix(V, Vq.data(), Nq, Np, sV);
-    else split_matrix(P, Pq.data(), Np, Nq, sP);
-  }
-  std::vector<PackTile> tiles;
-  std::vector<size_t> offset;
-  size_t words = 0;
-  auto add = [&](const PackTile &q) {
-    tiles.push_back(q), offset.push_back(words);
-    words += q.k16 ? 128 : 64;
+  // the operators themselves sit behind the tiles in the same buffer: the device
+  // packs them (on eight host threads creation took up to 7 ms longer where other
+  // work held these up)
+  std::vector<float> all;
+  for (const std::vector<float> *v : {&D[0], &D[1], &D[2], &LIFT, &Vq, &Pq}) all.insert(all.end(), v->begin(), v->end());
+  auto regions = [&](const float *A) {
+    std::vector<PackRegion> r;
+    const size_t n = (size_t)Np * Np;
+    int none = 0;
+    split_blocks(r, A, n, 3, Np, Np, sD, none, pl.oDt);
+    split_blocks(r, A + 3 * n, (size_t)Nfp * Np, 4, Np, Nfp, sL, pl.oL, pl.oLt);
+    const float *V = A + 3 * n + (size_t)4 * Nfp * Np;
+    split_rows(r, V, Nq, Np, sV, pl.oV, pl.oVt);
+    split_columns(r, V + (size_t)Nq * Np, Np, Nq, sP, pl.oP);
+    return r;
   };
-  auto at = [&]() { return (int)(words / 4); };
-  for (int d = 0; d < 3; ++d)
-    for (int k = 0; k < KP; ++k)
-      for (int j = 0; j < NB; ++j) add({&D3[d], 0, Np, Np, Np, Np, j, k, true});
-  pl.oDt = at();
-  for (int d = 0; d < 3 && KT; ++d)
-    for (int j = 0; j < NB; ++j) add({&D3[d], 0, Np, Np, Np, Np, j, 2 * KP, false});
-  pl.oL = at();
-  auto face = [&](int f) { return (size_t)f * Nfp * Np; };
-  for (int f = 0; f < 4; ++f)
-    for (int k = 0; k < FP; ++k)
-      for (int j = 0; j < NB; ++j) add({&L, face(f), Np, Nfp, Np, Nfp, j, k, true});
-  pl.oLt = at();
-  for (int f = 0; f < 4 && FT; ++f)
-    for (int j = 0; j < NB; ++j) add({&L, face(f), Np, Nfp, Np, Nfp, j, 2 * FP, false});
-  pl.oV = at();
-  for (int c = 0; c < nch; ++c)
-    for (int k = 0; k < KP; ++k)
-      for (int h = 0; h < 2; ++h) add({&V, 0, Nq, Np, Nq16, Np, 2 * c + h, k, true});
-  pl.oVt = at();
-  for (int c = 0; c < nch && KT; ++c)
-    for (int h = 0; h < 2; ++h) add({&V, 0, Nq, Np, Nq16, Np, 2 * c + h, 2 * KP, false});
-  pl.oP = at();
-  for (int c = 0; c < nch; ++c)
-    for (int j = 0; j < NB; ++j) add({&P, 0, Np, Nq, Np, Nq16, j, c, true});
-  pl.oM = at();
-  SplitOps all;
-  all.w.resize(words), all.m.resize(words);
-  const long long nt = (long long)tiles.size();
-#pragma omp parallel for schedule(static) num_threads(8) if (nt > 128)
-  for (long long i = 0; i < nt; ++i) pack_tile(tiles[i], &all.w[offset[i]], &all.m[offset[i]]);
-  out = pl.products == 4 ? all.words() : std::move(all.w);
-  pl.ops_n = (int)(out.size() / 4);
+  pl.oM = regions(nullptr).back().end();
+  pl.ops_n = pl.oM + (pl.products == 4 ? pl.oM / 4 : 0);
+  cudaError_t e = cudaMalloc((void **)ops, (size_t)pl.ops_n * 16 + all.size() * sizeof(float));
+  if (e != cudaSuccess) return set_cuda_error(e, "split operators");
+  float *dense = reinterpret_cast<float *>(*ops + pl.ops_n);
+  e = cudaMemcpy(dense, all.data(), all.size() * sizeof(float), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) return set_cuda_error(e, "split operators");
+  const bbw_status st = pack_operators(regions(dense), *ops, pl.products == 4 ? *ops + pl.oM : nullptr);
+  if (st != BBW_OK) return st;
   pl.iD = 1.f / sD, pl.iL = 1.f / sL, pl.iV = 1.f / sV, pl.iP = 1.f / sP;
   double vn = 0.0;
   for (int q = 0; q < Nq; ++q) {
@@ -240,6 +171,7 @@ void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<floa
   }
   // twice the bound, as for the divergence: rounding cannot reach 2^16
   pl.vnorm = (float)(2.0 * vn);
+  return BBW_OK;
 }
 
 // one warp per element
@@ -268,17 +200,19 @@ __global__ void k_records(int K, const float *__restrict__ vgeo, const float *__
   geo[i] = k >= K || c >= 25 ? 0.f : c < 16 ? fgeo[k * 16 + c] : vgeo[k * 9 + c - 16];
 }
 
+bbw_status setup_done(const char *what) {
+  return set_cuda_error(cudaStreamSynchronize(nullptr), what);
+}
+
 bbw_status geometry_records(int K, const float *vgeo, const float *fgeo, float *geo) {
   const long long n = (long long)(K + 16) * 28;
   k_records<<<(int)((n + 255) / 256), 256>>>(K, vgeo, fgeo, geo);
-  const bbw_status s = check_launch("geometry records");
-  return s != BBW_OK ? s : set_cuda_error(cudaStreamSynchronize(nullptr), "geometry records");
+  return check_launch("geometry records");
 }
 
 bbw_status warp_medium(int K, int Nq, const float *c2q, float *c2max, float *c2p) {
   k_medium<<<(K + 7) / 8, 256>>>(K, Nq, (Nq + 15) / 16 * 16, c2q, c2max, c2p);
-  const bbw_status s = check_launch("medium bound");
-  return s != BBW_OK ? s : set_cuda_error(cudaStreamSynchronize(nullptr), "medium bound");
+  return check_launch("medium bound");
 }
 
 }  // namespace bbw

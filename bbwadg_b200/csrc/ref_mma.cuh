@@ -16,14 +16,6 @@
 
 namespace bbw {
 
-// index of slot c of block b when n indices are stored in blocks of eight (the
-// order of warp_pack's tiles, kernels_warp.cu)
-__device__ __forceinline__ int slot_index(int n, int b, int c) {
-  const int nb = (n + 7) / 8;
-  if (b == nb - 1 && nb % 2) return 8 * b + c;
-  return 16 * (b / 2) + 4 * (c / 2) + 2 * (b % 2) + c % 2;
-}
-
 // power of two that brings the CTA-wide maximum of |A| (n values) into [2^14,
 // 2^15), as an exponent field; sRed: one int of shared memory, zero on entry
 __device__ __forceinline__ void block_max(int *sRed, const float *__restrict__ A, int n) {
@@ -43,38 +35,6 @@ __device__ __forceinline__ void block_max(int *sRed, const float *__restrict__ A
   if ((threadIdx.x & 31) == 0) atomicMax(sRed, __float_as_int(m));
 }
 __device__ __forceinline__ int operator_field(int red) { return scale_field(__int_as_float(red)); }
-
-// two operator values as hi, lo and the bytes of the rest, larger by
-// kRoundingBias (split_entry, kernels_warp.cu)
-__device__ __forceinline__ void split_operator(float2 x, float s, uint32_t &h, uint32_t &l, uint32_t &m) {
-  const float2 y = __fmul2_rn(x, both(s));
-  const __half2 hh = __float22half2_rn(y);
-  const float2 f = __half22float2(hh);
-  const float2 r = __ffma2_rn(y, both((float)kRoundingBias), __fadd2_rn(y, make_float2(-f.x, -f.y)));
-  const __half2 ll = __float22half2_rn(r);
-  const float2 g = __half22float2(ll);
-  const __half2 mm = __float22half2_rn(__fadd2_rn(r, make_float2(-g.x, -g.y)));
-  h = *reinterpret_cast<const uint32_t *>(&hh);
-  l = *reinterpret_cast<const uint32_t *>(&ll);
-  m = rest_byte(__half_as_ushort(__low2half(mm))) | rest_byte(__half_as_ushort(__high2half(mm))) << 8;
-}
-// lane's words of a k16 (uint4) or k8 (uint2) tile: at(block, slot) gives the entries
-template <bool K16, class At>
-__device__ __forceinline__ void split_tile(uint32_t *out, uint32_t *rest, int i, int k, int c, float s,
-                                           At &&at) {
-  uint32_t h0, l0, m0;
-  if constexpr (K16) {
-    uint32_t h1, l1, m1;
-    split_operator(make_float2(at(2 * k, c), at(2 * k, c + 1)), s, h0, l0, m0);
-    split_operator(make_float2(at(2 * k + 1, c), at(2 * k + 1, c + 1)), s, h1, l1, m1);
-    reinterpret_cast<uint4 *>(out)[i] = make_uint4(h0, h1, l0, l1);
-    rest[i] = m0 | m1 << 16;
-  } else {
-    split_operator(make_float2(at(k, c), at(k, c + 1)), s, h0, l0, m0);
-    reinterpret_cast<uint2 *>(out)[i] = make_uint2(h0, l0);
-    reinterpret_cast<uint16_t *>(rest)[i] = (uint16_t)m0;
-  }
-}
 
 // split tiles of the column-major nr x nc operator A times s into word `off` of
 // the words at `out` (the rests in the plane at `rest`): row blocks rb, column

@@ -246,6 +246,47 @@ __device__ __forceinline__ void mma_pair2(float (&c)[M][4], const F &x, const T 
   for (int i = 0; i < M; ++i) add4(cc[i], ss[i]);
 }
 
+// index of slot c of block b when n indices are stored in blocks of eight
+// (warp_stage.h)
+__device__ __forceinline__ int slot_index(int n, int b, int c) {
+  const int nb = (n + 7) / 8;
+  if (b == nb - 1 && nb % 2) return 8 * b + c;
+  return 16 * (b / 2) + 4 * (c / 2) + 2 * (b % 2) + c % 2;
+}
+
+// two operator values as hi, lo and the bytes of the rest, larger by
+// kRoundingBias
+__device__ __forceinline__ void split_operator(float2 x, float s, uint32_t &h, uint32_t &l, uint32_t &m) {
+  const float2 y = __fmul2_rn(x, both(s));
+  const __half2 hh = __float22half2_rn(y);
+  const float2 f = __half22float2(hh);
+  const float2 r = __ffma2_rn(y, both((float)kRoundingBias), __fadd2_rn(y, make_float2(-f.x, -f.y)));
+  const __half2 ll = __float22half2_rn(r);
+  const float2 g = __half22float2(ll);
+  const __half2 mm = __float22half2_rn(__fadd2_rn(r, make_float2(-g.x, -g.y)));
+  h = *reinterpret_cast<const uint32_t *>(&hh);
+  l = *reinterpret_cast<const uint32_t *>(&ll);
+  m = rest_byte(__half_as_ushort(__low2half(mm))) | rest_byte(__half_as_ushort(__high2half(mm))) << 8;
+}
+// lane's words of a k16 (uint4) or k8 (uint2) tile and its rest (null: none): at(block,
+// slot) gives the entries
+template <bool K16, class At>
+__device__ __forceinline__ void split_tile(uint32_t *out, uint32_t *rest, int i, int k, int c, float s,
+                                           At &&at) {
+  uint32_t h0, l0, m0;
+  if constexpr (K16) {
+    uint32_t h1, l1, m1;
+    split_operator(make_float2(at(2 * k, c), at(2 * k, c + 1)), s, h0, l0, m0);
+    split_operator(make_float2(at(2 * k + 1, c), at(2 * k + 1, c + 1)), s, h1, l1, m1);
+    reinterpret_cast<uint4 *>(out)[i] = make_uint4(h0, h1, l0, l1);
+    if (rest) rest[i] = m0 | m1 << 16;
+  } else {
+    split_operator(make_float2(at(k, c), at(k, c + 1)), s, h0, l0, m0);
+    reinterpret_cast<uint2 *>(out)[i] = make_uint2(h0, l0);
+    if (rest) reinterpret_cast<uint16_t *>(rest)[i] = (uint16_t)m0;
+  }
+}
+
 // power of two that brings a maximum m below 2^15, as an exponent field; the
 // inverse is the field 254 - f.  Clamped so that both stay normal numbers
 // (m below 2^-99, zero included, takes 2^113).

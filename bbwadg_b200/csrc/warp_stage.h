@@ -54,21 +54,34 @@ struct WarpPlan {
 // Order: D [3][KP][NB] and its k8 tiles [3][NB], LIFT [4][FP][NB] and [4][NB],
 // Vq [chunk][KP][2] and [chunk][2], Pq [chunk][NB].  Sets the offsets, inverse
 // scales and vnorm of the plan.
-// common power-of-two scale of n operators of `len` values
+// Device kernels pack them.
+//
+// A run of tiles: outer matrices A + o * stride (column-major nr x nc, device), nk
+// column pairs (k16) or the odd last block (k8) from k0 on, nj row blocks shifted
+// by o * row_step, order [outer][k][row block]; nrp, ncp: extents whose blocks the
+// indices run over, at: uint4 offset of the first tile, s: scale.
+struct PackRegion {
+  const float *A;
+  size_t stride;
+  int nr, nc, nrp, ncp, outer, nk, nj, k0, row_step, at;
+  bool k16;
+  float s;
+  __host__ __device__ int tiles() const { return outer * nk * nj; }
+  int end() const { return at + tiles() * (k16 ? 32 : 16); }
+};
+// common power-of-two scale of n operators of `len` values (host)
 float split_scale(const float *const *A, int n, size_t len);
 // Tiles of one column-major nr x nc operator, appended to out: split_rows
 // with its rows in chunks of 16 ([chunk][k16 step][2], then the k8 tails [chunk][2]),
 // split_columns with its columns in chunks of 16 ([chunk][row block]).
-struct SplitOps {
-  std::vector<uint32_t> w;            // hi and lo
-  std::vector<uint8_t> m;             // rest, one byte per four of w
-  std::vector<uint32_t> words() const;  // w, then m
-};
-void split_rows(SplitOps &out, const float *A, int nr, int nc, float s, int &off, int &off_tail);
-void split_columns(SplitOps &out, const float *A, int nr, int nc, float s, int &off);
-void warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
-               const std::vector<float> &Vq, const std::vector<float> &Pq,
-               std::vector<uint32_t> &out);
+void split_rows(std::vector<PackRegion> &out, const float *A, int nr, int nc, float s, int &off,
+                int &off_tail);
+void split_columns(std::vector<PackRegion> &out, const float *A, int nr, int nc, float s, int &off);
+// words to ops and rests to rests (null: none)
+bbw_status pack_operators(const std::vector<PackRegion> &regions, uint4 *ops, uint4 *rests);
+// *ops is the context's to free, also on failure
+bbw_status warp_pack(WarpPlan &pl, const std::vector<float> *D, const std::vector<float> &LIFT,
+                     const std::vector<float> &Vq, const std::vector<float> &Pq, uint4 **ops);
 // Sets the forms that fit (pl.single, pl.group).
 bbw_status warp_prepare(WarpPlan &pl);
 // The form for `elements` (elements of this context times shots) when none is
@@ -100,9 +113,11 @@ bbw_status warp_launch(const WarpPlan &pl, int form, const float *Qin, float *Qo
                        float fa, float fb, float fdt, float cstage, cudaStream_t st);
 // geometry records [K + 16][28] of the tensor-core and warp-matrix stages (device
 // pointers): fgeo 16 | vgeo 9 | pad, a tile's worth of zero records at the end
-// Both setup kernels run on the legacy stream, behind the copies and fills that
-// made their arguments, and have ended on return: the contexts' streams do
-// not wait for that stream.
+// The setup kernels (pack_operators, geometry_records, warp_medium) run on the
+// legacy stream, behind the copies and fills that made their arguments; the
+// contexts' streams do not wait for that stream, so setup_done comes before
+// the first launch on them.
+bbw_status setup_done(const char *what);
 bbw_status geometry_records(int K, const float *vgeo, const float *fgeo, float *geo);
 // c2max[k] = max_q |c2q[k][q]|; c2p[k]: c2q[k] padded with zeros to a multiple of 16
 bbw_status warp_medium(int K, int Nq, const float *c2q, float *c2max, float *c2p);
