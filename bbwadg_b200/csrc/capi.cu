@@ -260,6 +260,26 @@ static bbw_status make_variant(bbw_ctx *c, int W, int E, int want_ops, int want_
   return fused_prepare(p);
 }
 
+// medium, split operators and plan of the warp-matrix stages; FP32 contexts take
+// four products per split pair, split FP16 three; BB contexts the dense
+// equivalents of their sparse operators
+static bbw_status matrix_setup(bbw_ctx *c, int pat_off, int table_ints) {
+  const size_t med = (size_t)c->K * ((c->Nq + 15) / 16 * 16);
+  bbw_status s = set_cuda_error(cudaMalloc((void **)&c->c2p, (med + c->K) * sizeof(float)),
+                                "bbw_create: medium");
+  if (s != BBW_OK) return s;
+  c->c2max = c->c2p + med;
+  if ((s = warp_medium(c->K, c->Nq, c->c2q, c->c2max, c->c2p)) != BBW_OK) return s;
+  WarpPlan &wp = c->wp;
+  wp.N = c->N, wp.K = c->K, wp.Nq = c->Nq, wp.bc = c->bc;
+  wp.products = c->precision == BBW_PREC_FP32 ? 4 : 3;
+  wp.pat_off = pat_off, wp.table_ints = table_ints;  // Fmask and the face permutations
+  if ((s = warp_pack(wp, c->hD, c->hLIFT, c->hVq, c->hPq, &c->ops_wp)) != BBW_OK) return s;
+  wp.geo = c->geo_tc, wp.c2p = c->c2p, wp.c2max = c->c2max;
+  wp.nbr = c->nbr, wp.tables = c->tables, wp.ops = c->ops_wp, wp.time = c->d_time;
+  return warp_prepare(wp);
+}
+
 extern "C" bbw_status bbw_create(const bbw_mesh_desc *m, const bbw_ops_desc *o, int variant,
                                  int bc, bbw_ctx **out) {
   return bbw_create_ex(m, o, variant, bc, BBW_PREC_FP32, out);
@@ -425,10 +445,11 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
   c->precision = precision;
   if (precision == BBW_PREC_FP32 && N <= 3 &&
       (s = make_variant(c, bb && N == 3 ? 16 : 8, 16, 1, 0, c->narrow, &c->ops_narrow)) != BBW_OK) {
-    if (s != BBW_ERR_UNSUPPORTED) {
+    if (s != BBW_ERR_UNSUPPORTED && s != BBW_ERR_NOMEM) {
       release(c);
       return s;
     }
+    if (s == BBW_ERR_NOMEM) cudaGetLastError();
     c->narrow.W = 0;  // does not fit with a large cubature
   }
   if (gemm) {
@@ -440,35 +461,21 @@ extern "C" bbw_status bbw_create_ex(const bbw_mesh_desc *m, const bbw_ops_desc *
     }
   }
   const bool matrix = !gemm && precision != BBW_PREC_BF16X3 && N <= 7;
-  if (!gemm && (tcp || N <= 7)) {
-    // written in full by kernels: no fill
-    const size_t rec = (size_t)(K + 16) * TC_GEO, med = (size_t)K * ((Nq + 15) / 16 * 16);
-    e = cudaMalloc((void **)&c->geo_tc, rec * sizeof(float));
-    if (e == cudaSuccess && matrix) e = cudaMalloc((void **)&c->c2p, (med + K) * sizeof(float));
-    s = set_cuda_error(e, "bbw_create: geometry and medium");
+  if (matrix || tcp) {  // written in full by kernels: no fill
+    s = set_cuda_error(cudaMalloc((void **)&c->geo_tc, (size_t)(K + 16) * TC_GEO * sizeof(float)),
+                       "bbw_create: geometry");
     if (s == BBW_OK) s = geometry_records(K, c->vgeo, c->fgeo, c->geo_tc);
-    if (s == BBW_OK && matrix) {
-      c->c2max = c->c2p + med;
-      s = warp_medium(K, Nq, c->c2q, c->c2max, c->c2p);
+    if (s == BBW_OK && matrix) s = matrix_setup(c, pat_off, bb_off);
+    if (s == BBW_ERR_NOMEM && matrix && (c->geo_tc || !tcp)) {
+      // no room for the matrix stages' data (500 bytes an element at N = 5): the
+      // CTA-wide stages do without
+      cudaGetLastError();
+      cudaFree(c->c2p), cudaFree(c->ops_wp);
+      c->c2p = c->c2max = nullptr, c->ops_wp = nullptr, c->wp = WarpPlan();
+      if (!tcp) cudaFree(c->geo_tc), c->geo_tc = nullptr;
+      s = BBW_OK;
     }
     if (s != BBW_OK) {
-      release(c);
-      return s;
-    }
-  }
-  if (matrix) {
-    // FP32 contexts take four products per split pair, split FP16 three; BB
-    // contexts the dense equivalents of their sparse operators
-    WarpPlan &wp = c->wp;
-    wp.N = N, wp.K = K, wp.Nq = Nq, wp.bc = bc, wp.products = precision == BBW_PREC_FP32 ? 4 : 3;
-    wp.pat_off = pat_off, wp.table_ints = bb_off;  // Fmask and the face permutations
-    if ((s = warp_pack(wp, c->hD, c->hLIFT, c->hVq, c->hPq, &c->ops_wp)) != BBW_OK) {
-      release(c);
-      return s;
-    }
-    wp.geo = c->geo_tc, wp.c2p = c->c2p, wp.c2max = c->c2max;
-    wp.nbr = c->nbr, wp.tables = c->tables, wp.ops = c->ops_wp, wp.time = c->d_time;
-    if ((s = warp_prepare(wp)) != BBW_OK) {
       release(c);
       return s;
     }
