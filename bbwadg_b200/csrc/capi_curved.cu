@@ -67,6 +67,18 @@ const T *own_upload_c(bbw_curved *h, const T *src, size_t n, bbw_status &s) {
   return d;
 }
 
+// frees one of the handle's buffers
+template <class T>
+void drop(bbw_curved *h, T *&p) {
+  for (size_t i = 0; i < h->owned.size(); ++i)
+    if (h->owned[i] == (const void *)p) {
+      cudaFree(h->owned[i]);
+      h->owned.erase(h->owned.begin() + i);
+      break;
+    }
+  p = nullptr;
+}
+
 void release(bbw_curved *h) {
   for (auto &g : h->graph)
     if (g) cudaGraphExecDestroy(g);
@@ -298,7 +310,20 @@ extern "C" bbw_status bbw_curved_create(const bbw_curved_desc *d, int device, bb
     A.Vqr = own_upload_c(h, d->Vq_reduced, mr, s), A.Pqr = own_upload_c(h, d->Pq_reduced, mr, s);
     A.Fmask = own_upload_c(h, d->Fmask, (size_t)NF, s);
     A.vmapP = own_upload_c(h, vmapP.data(), vmapP.size(), s);
-    if (s == BBW_OK && curved_mma_preferred(N, d->KCurved)) s = setup_mma(h, d);
+    if (s == BBW_OK && curved_mma_preferred(N, d->KCurved)) {
+      const size_t kept = h->owned.size();
+      s = setup_mma(h, d);
+      if (s == BBW_ERR_NOMEM) {  // no room beside the compact rows: the thread-per-output kernel
+        cudaGetLastError();
+        for (; h->owned.size() > kept; h->owned.pop_back()) cudaFree(h->owned.back());
+        h->mma = CurvedMma();
+        s = BBW_OK;
+      }
+      if (h->mma.on)  // its tiles hold the same point data, its operators are split
+        for (const float **p : {&A.vgeoq, &A.Jq, &A.fgeoq, &A.Jr, &A.c2q, &A.Vq, &A.Vrq, &A.Vsq, &A.Vtq,
+                                &A.Pq, &A.Prq, &A.Psq, &A.Ptq, &A.VfqFace, &A.Pfq, &A.Vqr, &A.Pqr})
+          drop(h, *p);
+    }
   }
   if (s == BBW_OK) s = own_upload(h, &h->d_perm, perm.data(), perm.size(), "bbw_curved_create");
   // one stage on the zero state (it stays zero) sets the kernels' launch

@@ -1,10 +1,12 @@
 """Device memory of the solvers: contexts are still created where there is no
-room for the matrix stages' own data."""
+room for the matrix stages' own data, and the curved solver keeps its point data
+once."""
 import numpy as np
 import pytest
 from conftest import golden
 
 from bbwadg_b200 import WaveSolver, make_problem
+from bbwadg_b200.curved import CurvedSolver, make_curved_problem
 
 pytestmark = pytest.mark.gpu
 
@@ -54,3 +56,20 @@ def test_context_without_room_for_the_matrix_stages(cuda, precision):
         torch.cuda.empty_cache()
     # which CTA-wide variant is the default does not change its bits
     assert np.array_equal(got, ref)
+
+
+def test_curved_point_data_is_kept_once(cuda):
+    """N = 5, ball 10: 2160 of 6000 elements curved.  State, next state and residual,
+    the planar context's arrays and one copy of the point data, with a
+    quarter for padding to 16 points and 16 elements and the allocator's blocks."""
+    p = make_curved_problem(5, 10, **rule(5))
+    a = p.desc_arrays()
+    kc, Nfp = len(a["KlistCurved"]), 21
+    point = 4 * kc * (10 * p.Nq + 16 * p.Nfq + 2 * p.Nq)
+    whole = 4 * p.K * (3 * 4 * p.Np + 25 + 28 + 4 + 4 * Nfp + 2 * p.Nq + 16)
+    before = free()
+    s = CurvedSolver(p)
+    used = before - free()
+    s.steps(p.dt, 1)
+    s.close()
+    assert used < 1.25 * (point + whole) + (4 << 20), (used, point, whole)
