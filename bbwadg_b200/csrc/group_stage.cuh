@@ -9,11 +9,11 @@
 // barrier between phases.  Against one warp per tile (warp_stage.cuh) a tile's
 // chain is three to eight times shorter, which counts where a mesh has few tiles
 // or an element much work.  The results are the same bit for bit.  us per
-// stage, CTA-wide FP32 stage / one warp / group: N = 5, K = 3072: 23.8 / 24.6 /
-// 13.6, K = 196608: 879 / 422 / 411; N = 7, K = 24576: 706 / 327 / 178; N = 4, K =
-// 3072: 16.8 / 18.2 / 12.7.  Bound by instruction and L1 wavefront rate together
-// (issue 34 %, L1 data pipe 58 %, tensor 28 %); without the products 261 us,
-// without global loads 399, without stores 325 (N = 5, K = 196608).
+// stage, CTA-wide FP32 stage / group: N = 5, K = 3072: 23.8 / 14.4, K = 196608: 878 /
+// 432; N = 6, K = 24576: 475 / 132; N = 7: 736 / 212; N = 4, K = 3072: 16.8 / 12.8 (one
+// warp per tile 18.2).  Bound by instruction and L1 wavefront rate together
+// (before the rests: issue 34 %, L1 data pipe 58 %, tensor 28 %; without the products
+// 261 of 411 us, without global loads 399, without stores 325, N = 5, K = 196608).
 #pragma once
 #include <vector>
 
@@ -28,15 +28,15 @@ struct GroupCfg {
   // is a k8 step (same for the face nodes)
   static constexpr int NB = (Np + 7) / 8, KP = NB / 2, KT = NB % 2;
   static constexpr int FB = (Nfp + 7) / 8, FP = FB / 2, FT = FB % 2;
-  // a unit of work is a pair of blocks (or the odd last one); GW warps per
-  // group, NG groups per CTA.  us per stage at K = 24576 with three or four
-  // warps and two units each, 168 registers / one unit per warp: N = 6 145 / 123,
-  // N = 7 254 / 178 (one group of 255 registers; two of 128: 205).
+  // a unit of work is a pair of blocks (or the odd last one): one for each of the
+  // group's GW warps, whose old state stays in registers; NG groups per CTA.  us per
+  // stage at K = 24576 with three or four warps and two units each, 168 registers /
+  // one unit per warp: N = 6 145 / 123, N = 7 254 / 178 (one group of 255 registers;
+  // two of 128: 205).
   static constexpr int U = KP + KT;
   static constexpr int GW = U;  // 3, 4, 6, 8 at N = 4 .. 7
   static constexpr int NG = N <= 6 ? 12 / GW : 1;
   static constexpr int W = GW * NG, T = 32 * W;
-  static constexpr bool KEEP = U <= GW;  // a warp's old state stays in registers
   // operators in shared memory when they fit; else their rests (a fifth of them;
   // rests from L2 as well / from shared memory: N = 7, K = 24576 219 / 207 us per stage)
   static constexpr bool OPS = N <= 5;
@@ -354,27 +354,24 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
     if (it + step < P.nit) codes(kn, code0, code1);
 
     const float *Qa = sQ + C::row(ka - k0), *Qb = sQ + C::row(kb - k0);
-    // old state of the warp's units, rows a and b; reread when a warp has
-    // several units
+    // old state of the warp's unit, rows a and b
     float4 qa[4], qb[4];
     {
       float m[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int u = w; u < C::U; u += GW) {
-        if (KT == 0 || u < KP) {
+      if (KT == 0 || w < KP) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            qa[c] = load4<Np, V>(Qa + c * Np, 16 * u + 4 * t);
-            qb[c] = load4<Np, V>(Qb + c * Np, 16 * u + 4 * t);
-            m[c] = max4(m[c], qa[c]), m[4 + c] = max4(m[4 + c], qb[c]);
-          }
-        } else {
+        for (int c = 0; c < 4; ++c) {
+          qa[c] = load4<Np, V>(Qa + c * Np, 16 * w + 4 * t);
+          qb[c] = load4<Np, V>(Qb + c * Np, 16 * w + 4 * t);
+          m[c] = max4(m[c], qa[c]), m[4 + c] = max4(m[4 + c], qb[c]);
+        }
+      } else {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const float2 x = load2<Np, V>(Qa + c * Np, 16 * KP + 2 * t);
-            const float2 y = load2<Np, V>(Qb + c * Np, 16 * KP + 2 * t);
-            qa[c] = make_float4(x.x, x.y, 0.f, 0.f), qb[c] = make_float4(y.x, y.y, 0.f, 0.f);
-            m[c] = max2(m[c], x), m[4 + c] = max2(m[4 + c], y);
-          }
+        for (int c = 0; c < 4; ++c) {
+          const float2 x = load2<Np, V>(Qa + c * Np, 16 * KP + 2 * t);
+          const float2 y = load2<Np, V>(Qb + c * Np, 16 * KP + 2 * t);
+          qa[c] = make_float4(x.x, x.y, 0.f, 0.f), qb[c] = make_float4(y.x, y.y, 0.f, 0.f);
+          m[c] = max2(m[c], x), m[4 + c] = max2(m[4 + c], y);
         }
       }
 #pragma unroll
@@ -432,47 +429,14 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
                       cua, cub);
         }
       };
-      if constexpr (C::KEEP) {
-        if (KT == 0 || w < KP) {
-          if (w < KP) split_unit(std::integral_constant<int, 2>(), w, qa, qb);
-        } else if (w < C::U) {
-          split_unit(std::integral_constant<int, 1>(), w, qa, qb);
-        }
-      } else {
-        // the fragments overwrite the rows: read all units before the first write
-        constexpr int UW = (C::U + GW - 1) / GW;
-        float4 xa[UW][4], xb[UW][4];
-#pragma unroll
-        for (int i = 0; i < UW; ++i) {
-          const int u = w + i * GW;
-          if (u >= C::U) break;
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            if (KT == 0 || u < KP) {
-              xa[i][c] = load4<Np, V>(Qa + c * Np, 16 * u + 4 * t);
-              xb[i][c] = load4<Np, V>(Qb + c * Np, 16 * u + 4 * t);
-            } else {
-              const float2 x = load2<Np, V>(Qa + c * Np, 16 * KP + 2 * t);
-              const float2 y = load2<Np, V>(Qb + c * Np, 16 * KP + 2 * t);
-              xa[i][c] = make_float4(x.x, x.y, 0.f, 0.f), xb[i][c] = make_float4(y.x, y.y, 0.f, 0.f);
-            }
-          }
-        }
-        group_sync<GW>(grp);
-#pragma unroll
-        for (int i = 0; i < UW; ++i) {
-          const int u = w + i * GW;
-          if (u < KP) split_unit(std::integral_constant<int, 2>(), u, xa[i], xb[i]);
-          else if (u < C::U) split_unit(std::integral_constant<int, 1>(), u, xa[i], xb[i]);
-        }
-      }
+      if (KT == 0 || w < KP) split_unit(std::integral_constant<int, 2>(), w, qa, qb);
+      else split_unit(std::integral_constant<int, 1>(), w, qa, qb);
     }
     group_sync<GW>(grp);  // operands ready
 
-    // ---- 3. gradient, divergence and lift of the warp's units: update of u, v,
+    // ---- 3. gradient, divergence and lift of the warp's unit: update of u, v,
     //         w; rhs_p stays in registers
-    constexpr int UW = (C::U + GW - 1) / GW;
-    float rp[UW][2][4];
+    float rp[2][4];
     float ma = 0.f, mb = 0.f;  // maxima of rhs_p
     auto rhs_unit = [&](auto M, int u, float (&r)[2][4]) {
       constexpr int m = decltype(M)::value;
@@ -543,18 +507,16 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
       for (int c = 0; c < 3; ++c) {
         ra[c] = Un::template load<Np, V>(Ra + (c + 1) * Np, n);
         rb[c] = Un::template load<Np, V>(Rb + (c + 1) * Np, n);
-        if constexpr (!C::KEEP) {
-          xa[c] = Un::template load<Np, V>(Qs + ea + (c + 1) * Np, n);
-          xb[c] = Un::template load<Np, V>(Qs + eb + (c + 1) * Np, n);
-        } else if constexpr (m == 2) {
+        if constexpr (m == 2) {
           xa[c] = qa[c + 1], xb[c] = qb[c + 1];
         } else {
           xa[c] = lo2(qa[c + 1]), xb[c] = lo2(qb[c + 1]);
         }
       }
-      // rolled up or not by registers; us per stage unrolled / rolled: N = 5 (K =
-      // 196608) 448 / 429, split FP16 (K = 82944) 167 / 171; N = 4 (K = 3072) 13.3 / 14.0
-      constexpr int LU = OPS && (N == 4 || PR == 3) ? 2 : 1;
+      // rolled up but for N = 5 in FP32, by registers; us per stage unrolled / rolled:
+      // N = 5 432 / 437 (K = 196608), split FP16 172 / 169 (K = 82944, with the loop over Pq's
+      // chunks), N = 4 13.1 / 12.8 (K = 3072), N = 6 137 / 132, N = 7 221 / 212 (K = 24576)
+      constexpr int LU = OPS && N == 5 && PR == 4 ? 2 : 1;
 #pragma unroll LU
       for (int f0 = 0; f0 < 4; f0 += 2) {
         float L[2][m][4] = {};
@@ -626,14 +588,10 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
         }
       }
     };
-#pragma unroll
-    for (int i = 0; i < UW; ++i) {
-      const int u = w + i * GW;
-      if (u < KP) {
-        if constexpr (KP > 0) rhs_unit(std::integral_constant<int, 2>(), u, rp[i]);
-      } else if (u < C::U) {
-        if constexpr (KT > 0) rhs_unit(std::integral_constant<int, 1>(), u, rp[i]);
-      }
+    if (w < KP) {
+      if constexpr (KP > 0) rhs_unit(std::integral_constant<int, 2>(), w, rp);
+    } else {
+      if constexpr (KT > 0) rhs_unit(std::integral_constant<int, 1>(), w, rp);
     }
     const float cma = __ldg(P.c2max + ka), cmb = __ldg(P.c2max + kb);
     ma = quad_max(ma), mb = quad_max(mb);
@@ -655,14 +613,10 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
                 wb = scale_field(P.vnorm * mb * cmb);
       da = pow2_field(wa), db = pow2_field(wb);
       oia = pow2_field(254 - wa) * P.iP, oib = pow2_field(254 - wb) * P.iP;
-#pragma unroll
-      for (int i = 0; i < UW; ++i) {
-        const int u = w + i * GW;
-        if (u < KP) Unit<2>::split(sR, u, lane, Unit<2>::row(rp[i], 0), Unit<2>::row(rp[i], 1), ca, cb);
-        else if (u < C::U)
-          Unit<1>::split(sR, u, lane, make_float2(rp[i][0][0], rp[i][0][1]),
-                         make_float2(rp[i][0][2], rp[i][0][3]), ca, cb);
-      }
+      if (w < KP) Unit<2>::split(sR, w, lane, Unit<2>::row(rp, 0), Unit<2>::row(rp, 1), ca, cb);
+      else
+        Unit<1>::split(sR, w, lane, make_float2(rp[0][0], rp[0][1]), make_float2(rp[0][2], rp[0][3]), ca,
+                       cb);
     }
     const float4 *Ca = reinterpret_cast<const float4 *>(P.c2p + (size_t)ka * P.Nq16) + t,
                  *Cb = reinterpret_cast<const float4 *>(P.c2p + (size_t)kb * P.Nq16) + t;
@@ -671,30 +625,20 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 
     // residual of p: loaded here it is in flight during the projection, where
     // the registers allow (N = 7 187 -> 173 us per stage, N = 4 19.3 -> 19.7)
-    float4 ra[UW], rb[UW];
+    float4 ra, rb;
     auto load_rp = [&]() {
-#pragma unroll
-      for (int i = 0; i < UW; ++i) {
-        const int u = w + i * GW;
-        if (u < KP) {
-          ra[i] = load4<Np, V>(Ra, 16 * u + 4 * t), rb[i] = load4<Np, V>(Rb, 16 * u + 4 * t);
-        } else if (u < C::U) {
-          const float2 x = load2<Np, V>(Ra, 16 * u + 2 * t), y = load2<Np, V>(Rb, 16 * u + 2 * t);
-          ra[i] = make_float4(x.x, x.y, 0.f, 0.f), rb[i] = make_float4(y.x, y.y, 0.f, 0.f);
-        }
+      if (w < KP) {
+        ra = load4<Np, V>(Ra, 16 * w + 4 * t), rb = load4<Np, V>(Rb, 16 * w + 4 * t);
+      } else {
+        const float2 x = load2<Np, V>(Ra, 16 * w + 2 * t), y = load2<Np, V>(Rb, 16 * w + 2 * t);
+        ra = make_float4(x.x, x.y, 0.f, 0.f), rb = make_float4(y.x, y.y, 0.f, 0.f);
       }
     };
     if constexpr (C::EARLY) load_rp();
 
     // ---- 5. WADG projection of rhs_p, RC chunks of 16 cubature points at a
-    //         time: Vq and c2 of the warp's chunks, then Pq of its units
-    float o[UW][2][4];
-#pragma unroll
-    for (int i = 0; i < UW; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) o[i][j][v] = 0.f;
+    //         time: Vq and c2 of the warp's chunks, then Pq of its unit
+    float o[2][4] = {};
 #pragma unroll 1
     for (int c0 = 0; c0 < nch; c0 += C::RC) {
       const int cend = min(nch, c0 + C::RC);
@@ -728,7 +672,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
                                       v[1][2] * vib * zb.z, v[1][3] * vib * zb.w);
         Unit<2>::split(sW, c - c0, lane, xa, xb, da, db);
       }
-      if constexpr (!OPS && UW == 1) {
+      if constexpr (!OPS) {
         // operators from L2: the next four chunks' loads in flight
         OpTile<uint4> b[4][2];
         auto load_p = [&](int c) {
@@ -750,53 +694,44 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           for (int j = 0; j < 4; ++j) {
             if (c + j >= cend) break;
             const Frag x = get_frag(sW, c + j - c0, lane);
-            if (w < KP) mma_tiles<PR>(o[0], x, bb[j]);
-            else if (w < C::U) mma_tile<PR>(o[0][0], x, bb[j][0]);
+            if (w < KP) mma_tiles<PR>(o, x, bb[j]);
+            else mma_tile<PR>(o[0], x, bb[j][0]);
           }
         }
         continue;
       }
       group_sync<GW>(grp);  // the round's values ready
-#pragma unroll 2
+      constexpr int PU = PR == 4 ? 2 : 1;
+#pragma unroll PU
       for (int c = c0; c < cend; ++c) {
         const Frag x = get_frag(sW, c - c0, lane);
-#pragma unroll
-        for (int i = 0; i < UW; ++i) {
-          const int u = w + i * GW;
-          if (u < KP) {
-            const OpTile<uint4> b[2] = {oP[(c * NB + 2 * u) * 32], oP[(c * NB + 2 * u + 1) * 32]};
-            mma_tiles<PR>(o[i], x, b);
-          } else if (u < C::U) {
-            mma_tile<PR>(o[i][0], x, oP[(c * NB + 2 * u) * 32]);
-          }
+        if (w < KP) {
+          const OpTile<uint4> b[2] = {oP[(c * NB + 2 * w) * 32], oP[(c * NB + 2 * w + 1) * 32]};
+          mma_tiles<PR>(o, x, b);
+        } else {
+          mma_tile<PR>(o[0], x, oP[(c * NB + 2 * w) * 32]);
         }
       }
     }
 
     // ---- 6. sources and the LSRK update of p
 #pragma unroll
-    for (int i = 0; i < UW; ++i)
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) o[i][j][v] *= v < 2 ? oia : oib;
+      for (int v = 0; v < 4; ++v) o[j][v] *= v < 2 ? oia : oib;
     if (P.src_tile)
       tile_sources(P, Np, shot, k0, [&](int e, float amp, const float *vec) {
 #pragma unroll
-        for (int i = 0; i < UW; ++i) {
-          const int u = w + i * GW;
-#pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            if (u >= C::U || (u >= KP && j > 0)) continue;
-            const int n = u < KP ? 16 * u + 4 * t + 2 * j : 16 * KP + 2 * t;
-            const float s0 = n < Np ? amp * __ldg(vec + n) : 0.f;
-            const float s1 = n + 1 < Np ? amp * __ldg(vec + n + 1) : 0.f;
-            if (e == g) o[i][j][0] += s0, o[i][j][1] += s1;
-            if (e == g + 8) o[i][j][2] += s0, o[i][j][3] += s1;
-          }
+        for (int j = 0; j < 2; ++j) {
+          if (w >= KP && j > 0) continue;
+          const int n = w < KP ? 16 * w + 4 * t + 2 * j : 16 * KP + 2 * t;
+          const float s0 = n < Np ? amp * __ldg(vec + n) : 0.f;
+          const float s1 = n + 1 < Np ? amp * __ldg(vec + n + 1) : 0.f;
+          if (e == g) o[j][0] += s0, o[j][1] += s1;
+          if (e == g + 8) o[j][2] += s0, o[j][3] += s1;
         }
       });
-    auto update_p = [&](auto M, int u, int i, const float (&x)[2][4]) {
+    auto update_p = [&](auto M, int u, const float (&x)[2][4]) {
       using Un = Unit<decltype(M)::value>;
       using T = typename Un::T;
       const int n = Un::node(u, t);
@@ -804,13 +739,11 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
       if constexpr (!C::EARLY) {
         sa = Un::template load<Np, V>(Ra, n), sb = Un::template load<Np, V>(Rb, n);
       } else if constexpr (decltype(M)::value == 2) {
-        sa = ra[i], sb = rb[i];
+        sa = ra, sb = rb;
       } else {
-        sa = lo2(ra[i]), sb = lo2(rb[i]);
+        sa = lo2(ra), sb = lo2(rb);
       }
-      if constexpr (!C::KEEP) {
-        pa = Un::template load<Np, V>(Qs + ea, n), pb = Un::template load<Np, V>(Qs + eb, n);
-      } else if constexpr (decltype(M)::value == 2) {
+      if constexpr (decltype(M)::value == 2) {
         pa = qa[0], pb = qb[0];
       } else {
         pa = lo2(qa[0]), pb = lo2(qb[0]);
@@ -832,14 +765,10 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
         Un::template store<Np, V>(Ob, n, q);
       }
     };
-#pragma unroll
-    for (int i = 0; i < UW; ++i) {
-      const int u = w + i * GW;
-      if (u < KP) {
-        if constexpr (KP > 0) update_p(std::integral_constant<int, 2>(), u, i, o[i]);
-      } else if (u < C::U) {
-        if constexpr (KT > 0) update_p(std::integral_constant<int, 1>(), u, i, o[i]);
-      }
+    if (w < KP) {
+      if constexpr (KP > 0) update_p(std::integral_constant<int, 2>(), w, o);
+    } else {
+      if constexpr (KT > 0) update_p(std::integral_constant<int, 1>(), w, o);
     }
   }
 }

@@ -10,6 +10,8 @@
 // (issue 27 %, HBM 34 %); us per stage, CTA-wide FP32 stage -> this form: N = 2,
 // K = 93750: 94 -> 46; N = 3, K = 196608: 310 -> 137; N = 4, K = 82944: 249 -> 129.
 #pragma once
+#include <vector>
+
 #include "warp_mma.cuh"
 
 namespace bbw {
@@ -668,12 +670,16 @@ static bbw_status warp_launch_n(const WarpPlan &pl, const float *Qin, float *Qou
   WarpParams P = warp_params(pl, Qin, Qout, res, fa, fb, fdt, cstage);
   const int grid = warp_grid(pl, C::W, P);
   const size_t sm = warp_smem<N>(pl, pl.warp_ops);
-  if (pl.warp_ops) {
-    if (pl.products == 4) k_warp_stage<N, 4, true><<<grid, C::T, sm, st>>>(P);
-    else k_warp_stage<N, 3, true><<<grid, C::T, sm, st>>>(P);
+  // split FP16 contexts (three products) exist from N = 2
+  auto launch = [&](auto PR) {
+    if (pl.warp_ops) k_warp_stage<N, decltype(PR)::value, true><<<grid, C::T, sm, st>>>(P);
+    else k_warp_stage<N, decltype(PR)::value, false><<<grid, C::T, sm, st>>>(P);
+  };
+  if constexpr (N >= 2) {
+    if (pl.products == 3) launch(std::integral_constant<int, 3>());
+    else launch(std::integral_constant<int, 4>());
   } else {
-    if (pl.products == 4) k_warp_stage<N, 4, false><<<grid, C::T, sm, st>>>(P);
-    else k_warp_stage<N, 3, false><<<grid, C::T, sm, st>>>(P);
+    launch(std::integral_constant<int, 4>());
   }
   return check_launch("warp-matrix stage");
 }
@@ -684,8 +690,14 @@ static bbw_status warp_prepare_n(WarpPlan &pl) {
   pl.warp_ops = warp_smem<N>(pl, true) <= (size_t)maxsm;
   if (warp_smem<N>(pl, pl.warp_ops) > (size_t)maxsm)
     return set_error(BBW_ERR_UNSUPPORTED, "warp-matrix stage: does not fit in shared memory");
-  const void *fn[4] = {(const void *)k_warp_stage<N, 3, false>, (const void *)k_warp_stage<N, 4, false>,
-                       (const void *)k_warp_stage<N, 3, true>, (const void *)k_warp_stage<N, 4, true>};
+  if (N < 2 && pl.products == 3)
+    return set_error(BBW_ERR_UNSUPPORTED, "warp-matrix stage: three products from N = 2");
+  std::vector<const void *> fn = {(const void *)k_warp_stage<N, 4, false>,
+                                  (const void *)k_warp_stage<N, 4, true>};
+  if constexpr (N >= 2) {
+    fn.push_back((const void *)k_warp_stage<N, 3, false>);
+    fn.push_back((const void *)k_warp_stage<N, 3, true>);
+  }
   for (const void *f : fn) {
     const bbw_status s = ensure_smem_limit(f, maxsm, "warp-matrix stage attribute");
     if (s != BBW_OK) return s;
