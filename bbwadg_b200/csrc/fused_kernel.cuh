@@ -89,7 +89,7 @@ struct FusedParams {
   int Kc;  // elements [K0, Kc) are advanced; the others supply neighbour traces only
   int pat_off, bb_off;              // int offsets of the tables (multiples of 4)
   float fa, fb, fdt;
-  const float *__restrict__ Qin;
+  const float *Qin;                 // written by the stage before (stage_wait): not read-only
   float *__restrict__ Qout;
   float *__restrict__ res;
   const float *__restrict__ vgeo;   // [K][9]
@@ -109,7 +109,7 @@ struct FusedParams {
   const int *__restrict__ src_elem;
   const float *__restrict__ src_vec;
   float f0, tR, samp, cstage;
-  const double *__restrict__ time;  // simulation time at the start of the step
+  const double *time;               // simulation time at the start of the step
   // optional: Vq (raw rhs_p) at the cubature points, before c2/J, stored as
   // [shot][Nq][K] (the c^2 gradient of the discrete adjoint needs it)
   float *__restrict__ vq_out;

@@ -51,7 +51,7 @@ struct WarpParams {
   const int *__restrict__ src_elem;
   const float *__restrict__ src_vec;
   float f0, tR, samp;
-  const double *__restrict__ time;
+  const double *time;
 };
 
 __device__ __forceinline__ void mma16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0,
