@@ -600,7 +600,8 @@ static bool narrow_tiles(const bbw_ctx *c) {
 
 bbw_status launch_stage(bbw_ctx *c, const float *Qin, float *Qout, float *res, float fa, float fb,
                         float fdt, float cstage, cudaStream_t st, int K0, int Kc, bool chained) {
-  const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, (long long)c->S * c->K, (long long)c->S * c->whole_K);
+  const long long advanced = (long long)c->S * (c->plan.Kc > 0 ? c->plan.Kc : c->K);
+  const int form = c->cta_form ? WARP_AUTO : stage_form(c->wp, advanced, (long long)c->S * c->whole_K);
   if (form != WARP_AUTO) {
     WarpPlan p = c->wp;
     p.S = c->S, p.K0 = K0, p.Kc = Kc > 0 ? Kc : c->plan.Kc, p.max_ctas = c->plan.max_ctas;

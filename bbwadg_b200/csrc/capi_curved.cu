@@ -283,7 +283,12 @@ extern "C" bbw_status bbw_curved_create(const bbw_curved_desc *d, int device, bb
     od.Dr = d->Dr, od.Ds = d->Ds, od.Dt = d->Dt, od.LIFT = d->LIFT;
     od.Vq = d->Vq_reduced, od.Pq = d->Pq_reduced;
     s = bbw_create(&md, &od, BBW_NODAL, BBW_BC_PRESSURE_RELEASE, &h->aff);
+    // its form by the planar elements alone.  At N = 4 the group form holds the SMs
+    // that the thread-per-output kernel runs on beside it (KC = 720: 34.9 us per
+    // stage, 29.9 with the CTA-wide stage)
     if (s == BBW_OK && KP < K) s = bbw_set_compute_range(h->aff, KP);
+    if (s == BBW_OK) s = bbw_set_whole_mesh(h->aff, KP);
+    if (s == BBW_OK && N == 4 && !curved_mma_preferred(N, d->KCurved)) h->aff->cta_form = true;
     if (s == BBW_OK) h->Q[0] = h->aff->Q[0], h->Q[1] = h->aff->Q[1], h->res = h->aff->res;
   } else {
     if (s == BBW_OK) s = own_upload(h, &h->Q[0], (const float *)nullptr, ns, "bbw_curved_create");

@@ -46,16 +46,16 @@ struct CurvedMma {
 };
 // Whether the matrix form is the faster one for KC curved elements: its tile
 // is a longer chain than the thread-per-output kernel's block, so it wants
-// enough tiles.  us per stage with the planar elements, thread per output /
-// matrix:  N = 1  KC = 1344: 8.8 / 15.6   KC = 5760: 24.7 / 22.1
-//          N = 2  KC = 2160: 20.3 / 24.2  KC = 3168: 27.8 / 26.4
-//          N = 3  KC = 720: 17.9 / 21.1   KC = 1344: 22.8 / 21.2  KC = 13248: 207 / 99
-//          N = 4  KC = 288: 23.1 / 29.5   KC = 720: 29.9 / 29.3   KC = 3168: 117 / 47
-//          N = 5  KC = 288: 36.5 / 39.6   KC = 720: 49.2 / 39.3   KC = 2160: 134 / 50
-// (planar part of the first column: the CTA-wide stage).
+// enough tiles.  us per stage with the planar elements beside them, thread per
+// output / matrix (the former with the better planar stage):
+//   N = 1  never: KC = 4368: 18.4 / 20.9, KC = 37440: 122 / 139
+//   N = 2  KC = 2160: 20.3 / 23.6  KC = 3168: 27.7 / 26.9  KC = 4368: 32.7 / 28.5
+//   N = 3  KC = 720: 18.1 / 21.8   KC = 1344: 22.8 / 22.3  KC = 13248: 207 / 106
+//   N = 4  KC = 720: 29.9 / 31.1   KC = 1344: 50.3 / 31.8  KC = 3168: 117 / 51
+//   N = 5  KC = 288: 34.0 / 41.4   KC = 720: 50.9 / 42.0   KC = 2160: 134 / 55
 inline bool curved_mma_preferred(int N, int KC) {
-  constexpr int from[6] = {0, 5000, 3000, 1100, 700, 400};
-  return N >= 1 && N <= 5 && KC >= from[N];
+  constexpr int from[6] = {0, 0, 3000, 1100, 1000, 400};
+  return N >= 2 && N <= 5 && KC >= from[N];
 }
 bbw_status curved_mma_prepare(int N, CurvedMma &A);
 bbw_status curved_mma_stage(int N, const CurvedMma &A, const float *Qold, float *Qnew, float *res,

@@ -10,12 +10,11 @@ namespace bbw {
 #define BBW_DECL(n)                                                                             \
   bbw_status curved_mma_launch_##n(const CurvedMma &, const float *, float *, float *, cudaStream_t); \
   bbw_status curved_mma_prepare_##n(const CurvedMma &);
-BBW_DECL(1) BBW_DECL(2) BBW_DECL(3) BBW_DECL(4) BBW_DECL(5)
+BBW_DECL(2) BBW_DECL(3) BBW_DECL(4) BBW_DECL(5)
 #undef BBW_DECL
 
 #define BBW_SWITCH(CALL) \
   switch (N) {           \
-    case 1: CALL(1);     \
     case 2: CALL(2);     \
     case 3: CALL(3);     \
     case 4: CALL(4);     \

@@ -82,3 +82,21 @@ def test_pressure_and_velocity_of_different_size(cuda, N, n):
         ref = np.asarray(ref).reshape(p.K, 4, p.Np)
         err.append([rel_l2(res[kc, c], ref[kc, c]) for c in range(4)])
     assert (np.array(err[1:]) <= 1.5 * np.array(err[0])).all(), err
+
+
+@pytest.mark.parametrize("N,n", [(2, 10), (4, 6), (4, 8)])
+def test_planar_and_curved_forms_beside_each_other(cuda, N, n):
+    """Thread-per-output curved kernel beside the CTA-wide planar stage (N = 2, ball 10:
+    3840 planar elements of 6000; N = 4, ball 6) and matrix form beside the group
+    form (N = 4, ball 8)."""
+    from curved import CurvedOracle
+    p = problem(N, n, "table" if N >= 3 else "default")
+    rng = np.random.default_rng(N + n)
+    Q = (p.Q0 + 0.05 * rng.standard_normal(p.Q0.size)).astype(np.float32)
+    s = CurvedSolver(p)
+    s.set_data(Q)
+    s.steps(p.dt, 1)
+    got = s.get_data()
+    s.close()
+    ref, _ = CurvedOracle(N, p.K, p.Nq, p.Nfq, p.desc_arrays()).run(Q, p.dt, 5)
+    assert rel_l2(got, ref) < TOL
