@@ -43,6 +43,9 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
   using C = CurvedCfg<N, GWP>;
   constexpr int Np = C::Np, Nfp = C::Nfp, NB = C::NB, KP = C::KP, KT = C::KT, EW = C::EW;
   constexpr int FP = C::FP, FT = C::FT, V = C::V, GW = C::GW, AS = C::AS, PR = 4, PD = 5;
+  // a sum's first step sets it instead of adding to zero; by the registers (us per
+  // stage added / set: N = 3, ball 24 107 / 105, N = 4, ball 12 50.7 / 46.1, N = 5, ball 10 54.7 / 56.0)
+  constexpr bool SET = N == 3 || N == 4;
   extern __shared__ __align__(16) float smem_f[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int grp = warp / GW, w = warp - grp * GW, g = lane >> 2, t = lane & 3;
@@ -171,22 +174,12 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
           for (int s = 0; s < FP; ++s) {
             each(s7, [&](int c) { return fx[c][s]; }, op(A.oF)[((ch * FP + s) * 2 + i) * 32]);
 #pragma unroll
-            for (int c = 0; c < 7; ++c) {
-              if (s > 0) add4(v[c][i], s7[c]);
-              else
-#pragma unroll
-                for (int q = 0; q < 4; ++q) v[c][i][q] = s7[c][q];
-            }
+            for (int c = 0; c < 7; ++c) add4(v[c][i], s7[c], s == 0);
           }
           if constexpr (FT) {
             each(s7, [&](int c) { return f8[c]; }, tail(A.oFt)[(ch * 2 + i) * 32]);
 #pragma unroll
-            for (int c = 0; c < 7; ++c) {
-              if (FP > 0) add4(v[c][i], s7[c]);
-              else
-#pragma unroll
-                for (int q = 0; q < 4; ++q) v[c][i][q] = s7[c][q];
-            }
+            for (int c = 0; c < 7; ++c) add4(v[c][i], s7[c], FP == 0);
           }
         }
         // points 16 ch + 4 t + 0 .. 3: row h, point 2 i + j of the four
@@ -312,7 +305,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
               const O16 Q = op(A.oV[0]) + ((c * KP + k) * 2) * 32;
               const T16 bd[2] = {D[0], D[32]}, bq[2] = {Q[0], Q[32]};
               const Frag u = get_frag(sA + (1 + d) * AS, k, lane);
-              mma_pair2<PD, PR>(v[3 + d], p, bd, v[d], u, bq);
+              mma_pair2<PD, PR>(v[3 + d], p, bd, v[d], u, bq, SET && k == 0, SET && k == 0);
             }
           }
           if constexpr (KT) {
@@ -470,7 +463,7 @@ __global__ void __launch_bounds__(CurvedCfg<N, GWP>::T, 1)
 #pragma unroll
             for (int x = 0; x < 4; x += 2)
               mma_pair2<PR, PR>(v[x], get_frag(sA + x * AS, k, lane), b2, v[x + 1],
-                            get_frag(sA + (x + 1) * AS, k, lane), b2);
+                            get_frag(sA + (x + 1) * AS, k, lane), b2, SET && k == 0, SET && k == 0);
           }
           if constexpr (KT) {
             const O8 B = tail(A.oVrt) + (c * 2) * 32;

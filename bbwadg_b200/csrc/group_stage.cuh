@@ -53,6 +53,10 @@ struct GroupCfg {
   static_assert(NB <= 4 * FB, "rhs_p fits over the fluxes");
   static constexpr int RC = GW == 6 ? 12 : 8;  // cubature chunks per round
   static constexpr bool EARLY = !OPS;    // residual of p loaded before the projection
+  // a sum's first step sets it instead of adding to zero: fewer instructions, but by
+  // the registers it pays at N = 6 only (us per stage added / set: N = 5, K = 196608 432 /
+  // 437, N = 6, K = 24576 132 / 125, N = 7 212 / 215)
+  static constexpr bool SET = N == 6;
   static constexpr int SCR1 = 8 * FB * 8;      // one warp's face fluxes of eight elements
   static constexpr int WF = RC * 256 > GW * SCR1 ? RC * 256 : GW * SCR1;  // split cubature values
   static constexpr int GEO = 16 * 28;
@@ -237,6 +241,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
   float *sMaxR = sGeo + C::GEO + GW * 64, *sInv = sMaxR + GW * 16;  // [GW][16], [4][16]
   const uint4 *ops = OPS ? sOps : P.ops;
   constexpr int PD = PR == 4 ? 5 : PR;  // derivatives: large terms cancel
+  constexpr bool SET = C::SET;
   using O16 = Ops<uint4, PR, !OPS, PLACE == OPS_L2>;
   using O8 = Ops<uint2, PR, !OPS, PLACE == OPS_L2>;
   const void *rests = PLACE == OPS_RESTS ? sOps : ops + P.oM;
@@ -466,7 +471,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             const Frag y = get_frag(sA + (c + 1) * AS, k, lane);
-            mma_pair2<PD, PD>(d[c], x, b[c], dv, y, b[c]);
+            mma_pair2<PD, PD>(d[c], x, b[c], dv, y, b[c], SET && k == 0, SET && k == 0 && c == 0);
           }
         }
         if constexpr (KT) {
@@ -540,7 +545,8 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           }
         }
 #pragma unroll
-        for (int k = 0; k < FP; ++k) mma_pair2<PR, PR>(L[0], x[0][k], b[0][k], L[1], x[1][k], b[1][k]);
+        for (int k = 0; k < FP; ++k)
+          mma_pair2<PR, PR>(L[0], x[0][k], b[0][k], L[1], x[1][k], b[1][k], SET && k == 0, SET && k == 0);
         if constexpr (FT) mma_pair2<PR, PR>(L[0], x8[0], b8[0], L[1], x8[1], b8[1]);
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -658,7 +664,7 @@ __global__ void __launch_bounds__(GroupCfg<N>::T, 1) k_group_stage(const WarpPar
           const Frag x = get_frag(sR, k, lane);
           const OpTile<uint4> b[2] = {OPS ? oV[((c * KP + k) * 2) * 32] : bv[OPS ? 0 : k][0],
                                       OPS ? oV[((c * KP + k) * 2 + 1) * 32] : bv[OPS ? 0 : k][1]};
-          mma_tiles<PR>(v, x, b);
+          mma_tiles<PR>(v, x, b, SET && k == 0);
         }
         if constexpr (KT) {
           const Frag8 x = get_frag8(sR, KP, lane);

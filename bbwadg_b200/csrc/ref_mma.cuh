@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256, 1)
           OpTile<uint4> b[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) b[c] = oD[((c * KP + k) * NB + j) * 32];
-          mma_tiles<PD>(d, fp[k], b);
+          mma_tiles<PD>(d, fp[k], b, N == 3 && k == 0);
         }
         if constexpr (KT) {
           OpTile<uint2> b[3];

@@ -89,8 +89,13 @@ __device__ __forceinline__ void mma8_set(float (&c)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(b0), "f"(0.f));
 }
 
-// c += s, rounded to nearest
-__device__ __forceinline__ void add4(float (&c)[4], const float (&s)[4]) {
+// c = s (the first step), or c += s, rounded to nearest
+__device__ __forceinline__ void add4(float (&c)[4], const float (&s)[4], bool first = false) {
+  if (first) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = s[i];
+    return;
+  }
   const float2 a = __fadd2_rn(make_float2(c[0], c[1]), make_float2(s[0], s[1]));
   const float2 b = __fadd2_rn(make_float2(c[2], c[3]), make_float2(s[2], s[3]));
   c[0] = a.x, c[1] = a.y, c[2] = b.x, c[3] = b.y;
@@ -207,17 +212,17 @@ __device__ __forceinline__ void split_frag(Frag8 &f, const float2 a, const float
   split2(b, both(cb), f.h[1], f.l[1]);
 }
 
-// c += x b for M operator tiles; an accumulator is used again only after the
+// c += x b (first: c = x b) for M operator tiles; an accumulator is used again only after the
 // other tiles' product (a product takes 21 cycles, 8 of them issuing)
 template <int PR, int M, class F, class T>
-__device__ __forceinline__ void mma_tiles(float (&c)[M][4], const F &x, const T (&b)[M]) {
+__device__ __forceinline__ void mma_tiles(float (&c)[M][4], const F &x, const T (&b)[M], bool first = false) {
   float s[M][4];
 #pragma unroll
   for (int p = 0; p < kProducts; ++p)
 #pragma unroll
     for (int i = 0; i < M; ++i) mma_step<PR>(s[i], x, b[i], p);
 #pragma unroll
-  for (int i = 0; i < M; ++i) add4(c[i], s[i]);
+  for (int i = 0; i < M; ++i) add4(c[i], s[i], first);
 }
 // the first of two accumulators as an array of one
 __device__ __forceinline__ float (&one(float (&c)[2][4]))[1][4] {
@@ -231,7 +236,8 @@ __device__ __forceinline__ void mma_tile(float (&c)[4], const F &x, const T b) {
 // two operands' products x b and y bb, interleaved
 template <int PX, int PY, int M, class F, class T>
 __device__ __forceinline__ void mma_pair2(float (&c)[M][4], const F &x, const T (&b)[M],
-                                          float (&cc)[M][4], const F &y, const T (&bb)[M]) {
+                                          float (&cc)[M][4], const F &y, const T (&bb)[M],
+                                          bool first = false, bool first2 = false) {
   float s[M][4], ss[M][4];
 #pragma unroll
   for (int p = 0; p < kProducts; ++p) {
@@ -241,9 +247,9 @@ __device__ __forceinline__ void mma_pair2(float (&c)[M][4], const F &x, const T 
     for (int i = 0; i < M; ++i) mma_step<PY>(ss[i], y, bb[i], p);
   }
 #pragma unroll
-  for (int i = 0; i < M; ++i) add4(c[i], s[i]);
+  for (int i = 0; i < M; ++i) add4(c[i], s[i], first);
 #pragma unroll
-  for (int i = 0; i < M; ++i) add4(cc[i], ss[i]);
+  for (int i = 0; i < M; ++i) add4(cc[i], ss[i], first2);
 }
 
 // index of slot c of block b when n indices are stored in blocks of eight

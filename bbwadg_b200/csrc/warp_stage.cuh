@@ -129,6 +129,10 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
     for (int i = lane; i < C::FLUX; i += 32) sF[i] = 0.f;
   const uint4 *ops = OPS ? sOps : P.ops;
   constexpr int PD = PR == 4 ? 5 : PR;  // derivatives: large terms cancel
+  // a sum's first step sets it instead of adding to zero; by the registers it pays at
+  // N = 3 only (us per stage added / set: N = 2, K = 93750 45.3 / 45.7, N = 3, K = 82944
+  // 63.9 / 61.6, N = 4, K = 24576 48.5 / 49.1)
+  constexpr bool SET = N == 3;
   using O16 = Ops<uint4, PR, !OPS>;
   using O8 = Ops<uint2, PR, !OPS>;
   const void *rests = ops + P.oM;
@@ -302,7 +306,7 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
             OpTile<uint4> b[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) b[c] = oD[((c * KP + k) * NB + j) * 32];
-            mma_tiles<PD>(d, fp[k], b);
+            mma_tiles<PD>(d, fp[k], b, SET && k == 0);
           }
           if constexpr (KT) {
             OpTile<uint2> b[3];
@@ -566,7 +570,7 @@ __global__ void __launch_bounds__(WarpCfg<N>::T, 1) k_warp_stage(const WarpParam
 #pragma unroll
         for (int k = 0; k < KP; ++k) {
           const OpTile<uint4> b[2] = {oV[((c * KP + k) * 2) * 32], oV[((c * KP + k) * 2 + 1) * 32]};
-          mma_tiles<PR>(v, fr[k], b);
+          mma_tiles<PR>(v, fr[k], b, SET && k == 0);
         }
         if constexpr (KT) {
           const OpTile<uint2> b[2] = {oVt[(c * 2) * 32], oVt[(c * 2 + 1) * 32]};
