@@ -50,8 +50,8 @@ struct CurvedMma {
 // output / matrix (the former with the better planar stage):
 //   N = 1  never: KC = 4368: 18.4 / 20.9, KC = 37440: 122 / 139
 //   N = 2  KC = 2160: 20.3 / 23.6  KC = 3168: 27.7 / 26.9  KC = 4368: 32.7 / 28.5
-//   N = 3  KC = 720: 18.1 / 21.8   KC = 1344: 22.8 / 22.3  KC = 13248: 207 / 106
-//   N = 4  KC = 720: 29.9 / 31.1   KC = 1344: 50.3 / 31.8  KC = 3168: 117 / 51
+//   N = 3  KC = 720: 18.1 / 21.8   KC = 1344: 22.8 / 22.3  KC = 13248: 207 / 105
+//   N = 4  KC = 720: 29.9 / 31.1   KC = 1344: 50.3 / 31.8  KC = 3168: 117 / 46
 //   N = 5  KC = 288: 34.0 / 41.4   KC = 720: 50.9 / 42.0   KC = 2160: 134 / 55
 inline bool curved_mma_preferred(int N, int KC) {
   constexpr int from[6] = {0, 0, 3000, 1100, 1000, 400};

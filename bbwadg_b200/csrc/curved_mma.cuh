@@ -569,9 +569,8 @@ static bbw_status curved_mma_prepare_g(const CurvedMma &A) {
 
 // Warps per tile: four (a face each) while the tiles fit one wave of two
 // groups per SM, else as many as there are units of nodes (the results are the
-// same).  us per stage with the planar elements, N = 3: K = 3072 (84 tiles) 21.2
-// with four, 24.9 with two; K = 82944 (828 tiles) 114 and 99.  The kernel with a
-// thread per output: 23.2 and 154 on the same planar stage.
+// same).  us per stage with the planar elements, N = 3, before the rests: K = 3072
+// (84 tiles) 21.2 with four, 24.9 with two; K = 82944 (828 tiles) 114 and 99.
 template <int N>
 static bool curved_wide(const CurvedMma &A) { return A.nt <= 2 * A.nsm; }
 

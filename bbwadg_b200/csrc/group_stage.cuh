@@ -10,9 +10,9 @@
 // chain is three to eight times shorter, which counts where a mesh has few tiles
 // or an element much work.  The results are the same bit for bit.  us per
 // stage, CTA-wide FP32 stage / group: N = 5, K = 3072: 23.8 / 14.4, K = 196608: 878 /
-// 432; N = 6, K = 24576: 475 / 132; N = 7: 736 / 212; N = 4, K = 3072: 16.8 / 12.8 (one
+// 432; N = 6, K = 24576: 475 / 125; N = 7: 736 / 212; N = 4, K = 3072: 16.8 / 12.7 (one
 // warp per tile 18.2).  Bound by instruction and L1 wavefront rate together
-// (before the rests: issue 34 %, L1 data pipe 58 %, tensor 28 %; without the products
+// (issue 36 %, L1 data pipe 57 %, tensor 28 %; before the rests, without the products
 // 261 of 411 us, without global loads 399, without stores 325, N = 5, K = 196608).
 #pragma once
 #include <vector>

@@ -151,7 +151,7 @@ __device__ __forceinline__ uint32_t rest_hi(uint32_t m) { return __byte_perm(m, 
 // steps in one accumulator loses half an ulp of the running sum at every step,
 // always the same way.  One such rounding per step is left, and the operators
 // are packed larger by its mean (kRoundingBias).  us per stage against one
-// accumulator, N = 5, K = 196608: 411 -> 429; N = 7, K = 24576: 177 -> 207.
+// accumulator, N = 5, K = 196608: 411 -> 432; N = 7, K = 24576: 177 -> 212.
 //
 // Product p of one step, from zero or onto s, smallest first: the operand's hi
 // with the operator's rest, lo with lo, hi with lo, lo with hi, hi with hi.  PR = 5:

@@ -8,7 +8,7 @@
 // c2 -> Pq chains in registers, without shared memory or any barrier between
 // warps.  Bound by instruction latency at two or three warps per scheduler
 // (issue 27 %, HBM 34 %); us per stage, CTA-wide FP32 stage -> this form: N = 2,
-// K = 93750: 94 -> 46; N = 3, K = 196608: 310 -> 137; N = 4, K = 82944: 249 -> 129.
+// K = 93750: 94 -> 46; N = 3, K = 196608: 310 -> 137; N = 4, K = 82944: 249 -> 128.
 #pragma once
 #include <vector>
 

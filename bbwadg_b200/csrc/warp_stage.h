@@ -94,13 +94,13 @@ bbw_status warp_prepare(WarpPlan &pl);
 // warp / group:
 //   N = 1  K = 6000: 8.2 / 6.5 / -      K = 93750: 57 / 29 / -
 //   N = 2  K = 1296: 5.7 / 9.4 / -      K = 6000: 11.9 / 9.5 / -
-//   N = 3  K = 3072: 9.4 / 11.2 / -     K = 6000: 17.6 / 11.5 / -
-//   N = 4  K = 6: 15.6 / - / 9.9        K = 3072: 16.8 / 18.2 / 13.2  K = 10368: 43.8 / 22.6 / 34
-//   N = 5  K = 6: 21.0 / - / 10.3       K = 3072: 23.8 / - / 14.7     K = 196608: 878 / - / 429
-//   N = 6  K = 6: 73 / - / 17.7         K = 24576: 475 / - / 140
-//   N = 7  K = 6: 112 / - / 19.3        K = 24576: 736 / - / 206
+//   N = 3  K = 3072: 9.4 / 11.2 / -     K = 6000: 17.6 / 11.1 / -
+//   N = 4  K = 6: 15.6 / - / 9.9        K = 3072: 16.8 / 18.2 / 12.7  K = 10368: 43.8 / 22.6 / 34
+//   N = 5  K = 6: 21.0 / - / 10.3       K = 3072: 23.8 / - / 14.4     K = 196608: 878 / - / 432
+//   N = 6  K = 6: 73 / - / 17.7         K = 24576: 475 / - / 125
+//   N = 7  K = 6: 112 / - / 19.3        K = 24576: 736 / - / 212
 // and with the package's own rules N = 5, 216 points K = 6: 53.9 / - / 15.2, K = 24576:
-// 335 / - / 97; N = 6, 343 points, K = 10368: 289 / - / 72 (before the rests).
+// 335 / - / 96; N = 6, 343 points, K = 10368: 289 / - / 72 (before the rests).
 // One warp per tile pays once there are about two tiles per SM; the group
 // form, three tiles or more per SM at a time, up to the tiles of its first wave
 // at N = 4 (four per SM), and at every size above.
